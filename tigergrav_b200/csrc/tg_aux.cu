@@ -130,6 +130,7 @@ int ewald_tables(Solver &S, cudaStream_t st) {
     k_periodic_parts<<<(NFOUR_HALF + 63) / 64, 64, 0, st>>>(S.ew_four.p, NFOUR_HALF, 2.0, S.ew_Hd.p, S.ew_Hf.p, S.ew_Pf.p,
                                                             S.ew_Pd.p);
     TG_TRY(launched(S));
+    if (S.ew_use_tab && !S.ew_tab) TG_TRY(ewald_table_acquire(S.dev, S.ew_real.p, S.ew_four.p, &S.ew_tab, st));
     TG_CUDA(cudaStreamSynchronize(st)); /* host vectors go out of scope */
     S.have_tables = true;
     return TG_OK;

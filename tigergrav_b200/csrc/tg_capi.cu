@@ -287,6 +287,7 @@ int tg_create(const tg_params *params, tg_solver **out) {
     Solver &S = h->S;
     S.prm = *params;
     S.dev = params->device;
+    S.ew_use_tab = params->ewald && params->precision == TG_PREC_F32;
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, S.dev) == cudaSuccess) S.num_sms = prop.multiProcessorCount;
     int rc = ensure(S.dev_err, 4);
@@ -346,6 +347,7 @@ int tg_destroy(tg_solver *s) {
     release(S.fof_gmin); release(S.fof_group); release(S.fof_has); release(S.fof_pairs); release(S.fof_radii);
     release(S.fof_stats);
     release(S.rung_flag); release(S.rung_scan); release(S.rung_nact); release(S.rung_out);
+    if (S.ew_tab) ewald_table_release(S.dev);
     if (S.h_err) cudaFreeHost(S.h_err);
     if (S.h_cnt) cudaFreeHost(S.h_cnt);
     if (S.h_small) cudaFreeHost(S.h_small);
@@ -739,6 +741,7 @@ int tg_memory_report(tg_solver *s, char *buf, int64_t cap) {
     TG_MEM(tid_u); TG_MEM(tid_o); TG_MEM(tid_U); TG_MEM(tid_V); TG_MEM(fof_P); TG_MEM(fof_key); TG_MEM(fof_mem);
     TG_MEM(fof_pairs); TG_MEM(rung_flag); TG_MEM(rung_scan); TG_MEM(rung_nact);
 #undef TG_MEM
+    if (S.ew_tab) add("ewald_table(shared)", ewald_table_bytes());
     out += "total " + std::to_string(total) + "\n";
     if ((int64_t)out.size() + 1 > cap) return TG_ERR_SIZE;
     std::memcpy(buf, out.c_str(), out.size() + 1);

@@ -252,6 +252,7 @@ struct EwaldTables {
     const double *Hd;   /* NFOUR_HALF rows of HS, double */
     const float4 *Pf;   /* NFOUR_HALF x (H0, Hx, Hy, Hz): the potential and force terms, float */
     const double2 *Pd;  /* NFOUR_HALF x 2, double */
+    const float *tab;   /* local expansions of green_ewald (tg_ewald_table.cuh); solvers of the FP32 path only */
 };
 
 /* Real-space cut of the Ewald sum.  The reference masks images at r >= 3.6

@@ -21,6 +21,8 @@
  * sums folded into Kahan-compensated accumulators) or T = double (the plain
  * FP64 port).  Expansions L are FP64 in both.
  */
+#include <mutex>
+
 #include "tg_solver.cuh"
 
 namespace tg {
@@ -332,6 +334,7 @@ __global__ void __launch_bounds__(128) k_node(GParams P, int64_t nn, const int32
     }
 }
 
+#include "tg_ewald_table.cuh"
 #include "tg_ewald_node.cuh"
 
 /* ---- L2L, one level ---- */
@@ -629,7 +632,7 @@ __global__ void k_seam_node(GParams P, int kind_ewald, int is_cc, int64_t ngroup
 }
 
 static EwaldTables tables(Solver &S) {
-    return EwaldTables{S.ew_real.p, S.ew_four.p, S.ew_Hf.p, S.ew_Hd.p, S.ew_Pf.p, S.ew_Pd.p};
+    return EwaldTables{S.ew_real.p, S.ew_four.p, S.ew_Hf.p, S.ew_Hd.p, S.ew_Pf.p, S.ew_Pd.p, S.ew_tab};
 }
 
 static ListView listview(Solver &S) {

@@ -139,6 +139,8 @@ struct Solver {
     DevBuf<double2> ew_Pd;
     DevBuf<float2> ew_nt, ew_sf; /* per node and h: (cos, sin) at the centre of mass; per leaf: sums over particles */
     DevBuf<float> ew_tpart;      /* per leaf Ewald chunk and h: 8 reciprocal-space source sums */
+    bool ew_use_tab = false;       /* a periodic solver of the FP32 path */
+    const float *ew_tab = nullptr; /* the device's table of local expansions (FP32 path), shared by its solvers */
     bool have_tables = false;
 
     /* rung (individual) time steps: the rung lives in vel[i].w */
@@ -214,6 +216,10 @@ void release(DevBuf<T> &b) {
 
 int init_constants();
 int ewald_tables(Solver &S, cudaStream_t st);
+/* the device's shared Ewald expansion table: made by the first solver that needs it, freed with the last */
+int ewald_table_acquire(int dev, const float4 *real, const float4 *four, const float **tab, cudaStream_t st);
+void ewald_table_release(int dev);
+size_t ewald_table_bytes();
 int tree_build(Solver &S, cudaStream_t st);
 int tree_multipoles(Solver &S, cudaStream_t st);
 int tree_walk(Solver &S, cudaStream_t st);
