@@ -130,6 +130,30 @@ int ewald_tables(Solver &S, cudaStream_t st) {
     k_periodic_parts<<<(NFOUR_HALF + 63) / 64, 64, 0, st>>>(S.ew_four.p, NFOUR_HALF, 2.0, S.ew_Hd.p, S.ew_Hf.p, S.ew_Pf.p,
                                                             S.ew_Pd.p);
     TG_TRY(launched(S));
+    /* the PP Ewald split: vectors in increasing |h|^2 */
+    std::vector<int4> sh;
+    std::vector<double> sw;
+    double r0 = 0.0, r2 = 0.0;
+    const auto rec = lattice(30);
+    for (auto v = rec.rbegin(); v != rec.rend(); ++v) {
+        const int lead = (*v)[0] != 0 ? (*v)[0] : ((*v)[1] != 0 ? (*v)[1] : (*v)[2]);
+        if (lead <= 0) continue;
+        const double pi = 3.141592653589793;
+        const double h2 = (double)((*v)[0] * (*v)[0] + (*v)[1] * (*v)[1] + (*v)[2] * (*v)[2]);
+        const double w = 2.0 * std::exp(-pi * pi * h2 / (SEP_ALPHA_D * SEP_ALPHA_D)) / h2;
+        sh.push_back(make_int4((*v)[0], (*v)[1], (*v)[2], 0));
+        sw.push_back(w);
+        r0 -= w / pi;
+        r2 += 4.0 * pi / 3.0 * w * h2;
+    }
+    if ((int)sh.size() != NSEP) return TG_ERR_STATE;
+    S.ew_sep_k = (float)(3.141592653589793 / (SEP_ALPHA_D * SEP_ALPHA_D));
+    S.ew_sep_r0 = (float)r0;
+    S.ew_sep_r2 = (float)r2;
+    TG_TRY(ensure(S.ew_sep_h, NSEP));
+    TG_TRY(ensure(S.ew_sep_w, NSEP));
+    TG_CUDA(cudaMemcpyAsync(S.ew_sep_h.p, sh.data(), sizeof(int4) * NSEP, cudaMemcpyHostToDevice, st));
+    TG_CUDA(cudaMemcpyAsync(S.ew_sep_w.p, sw.data(), sizeof(double) * NSEP, cudaMemcpyHostToDevice, st));
     if (S.ew_use_tab && !S.ew_tab) TG_TRY(ewald_table_acquire(S.dev, S.ew_real.p, S.ew_four.p, &S.ew_tab, st));
     TG_CUDA(cudaStreamSynchronize(st)); /* host vectors go out of scope */
     S.have_tables = true;

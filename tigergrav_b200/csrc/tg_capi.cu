@@ -340,7 +340,8 @@ int tg_destroy(tg_solver *s) {
     release(S.wk_kind);
     release(S.scratch); release(S.dev_err); release(S.dev_cnt);
     release(S.ew_real); release(S.ew_four); release(S.ew_Hf); release(S.ew_Hd); release(S.ew_Pf); release(S.ew_Pd);
-    release(S.ew_cnt); release(S.ew_off); release(S.ew_part); release(S.ew_nt); release(S.ew_sf); release(S.ew_tpart);
+    release(S.ew_cnt); release(S.ew_off); release(S.ew_part); release(S.ew_sf); release(S.ew_sep_h);
+    release(S.ew_sep_w); release(S.ew_slot); release(S.ew_src); release(S.ew_tpart);
     release(S.ck_x); release(S.ck_v); release(S.adj_x); release(S.adj_v); release(S.tid_u); release(S.tid_o);
     release(S.tid_U); release(S.tid_V);
     release(S.fof_P); release(S.fof_leaves); release(S.fof_key); release(S.fof_mem); release(S.fof_runs);
@@ -737,7 +738,7 @@ int tg_memory_report(tg_solver *s, char *buf, int64_t cap) {
     TG_MEM(loff[0]); TG_MEM(llen[0]); TG_MEM(pool[0]); TG_MEM(pool[1]); TG_MEM(pool[2]); TG_MEM(pool[3]);
     TG_MEM(pool[4]); TG_MEM(pool[5]); TG_MEM(pool[6]); TG_MEM(pool[7]); TG_MEM(nxt_pool[0]); TG_MEM(nxt_pool[1]);
     TG_MEM(nxt_off[0]); TG_MEM(nxt_len[0]); TG_MEM(scratch); TG_MEM(ew_cnt); TG_MEM(ew_off); TG_MEM(ew_part);
-    TG_MEM(ew_nt); TG_MEM(ew_sf); TG_MEM(ew_tpart); TG_MEM(ck_x); TG_MEM(ck_v); TG_MEM(adj_x); TG_MEM(adj_v);
+    TG_MEM(ew_slot); TG_MEM(ew_src); TG_MEM(ew_sf); TG_MEM(ew_tpart); TG_MEM(ck_x); TG_MEM(ck_v); TG_MEM(adj_x); TG_MEM(adj_v);
     TG_MEM(tid_u); TG_MEM(tid_o); TG_MEM(tid_U); TG_MEM(tid_V); TG_MEM(fof_P); TG_MEM(fof_key); TG_MEM(fof_mem);
     TG_MEM(fof_pairs); TG_MEM(rung_flag); TG_MEM(rung_scan); TG_MEM(rung_nact);
 #undef TG_MEM

@@ -116,14 +116,15 @@ __device__ __forceinline__ void pp_direct_pair(const GParams &P, const T *dX, T 
 
 /* Nearest image (n = 0) of the real-space sum together with the removal of
  * the direct 1/r that the Ewald kernels perform (src/gravity.cpp:594-600):
- *   -erfc(2r)/r + 1/r = erf(2r)/r
- *   force factor (1 - erfc(2r) - (4r/sqrt(pi)) e^{-4r^2}) / r^3
- * written without the cancellation of the two large 1/r terms.  With x = 2r,
+ *   -erfc(alpha r)/r + 1/r = erf(alpha r)/r
+ *   force factor (1 - erfc(alpha r) - (2 alpha r/sqrt(pi)) e^{-alpha^2 r^2}) / r^3
+ * written without the cancellation of the two large 1/r terms (alpha: the
+ * Ewald split, 2 in the reference).  With x = alpha r,
  * F(x) = erf(x) - (2x/sqrt(pi)) e^{-x^2} = (2/sqrt(pi)) sum_{k>=1} (-1)^{k+1} 2k x^{2k+1} / (k! (2k+1))
  * (Taylor series of erf and of x e^{-x^2}), used below x = 0.5. */
 template <class T>
-__device__ __forceinline__ void ewald_nearest(T r, T rinv, T &p0, T &f0) {
-    const T x = T(2) * r;
+__device__ __forceinline__ void ewald_nearest(T alpha, T r, T rinv, T &p0, T &f0) {
+    const T x = alpha * r;
     const T erfx = erf(x);
     p0 = erfx * rinv;
     if (x < T(0.5)) {
@@ -136,7 +137,7 @@ __device__ __forceinline__ void ewald_nearest(T r, T rinv, T &p0, T &f0) {
         s = fma(s, y, T(1.0 / 7.0));
         s = fma(s, y, T(-0.4));
         s = fma(s, y, T(2.0 / 3.0));
-        f0 = T(8.0 * 1.1283791670955126) * s; /* F / r^3 = 8 F / x^3 */
+        f0 = T(1.1283791670955126) * (alpha * alpha * alpha) * s; /* F / r^3 = alpha^3 F / x^3 */
     } else {
         const T F = erfx - T(1.1283791670955126) * x * exp(-x * x);
         f0 = F * rinv * rinv * rinv;
@@ -189,7 +190,7 @@ __device__ __forceinline__ void pp_ewald_pair(const EwaldTables &E, const T *dX0
     }
     const T rinv = t_rsqrt(r2);
     T p0, f0;
-    ewald_nearest<T>(r2 * rinv, rinv, p0, f0);
+    ewald_nearest<T>(T(2), r2 * rinv, rinv, p0, f0);
     phi = ph + (T(0.78539816339744831) + p0);
     g[0] = gx + dX0[0] * f0;
     g[1] = gy + dX0[1] * f0;
@@ -632,7 +633,8 @@ __global__ void k_seam_node(GParams P, int kind_ewald, int is_cc, int64_t ngroup
 }
 
 static EwaldTables tables(Solver &S) {
-    return EwaldTables{S.ew_real.p, S.ew_four.p, S.ew_Hf.p, S.ew_Hd.p, S.ew_Pf.p, S.ew_Pd.p, S.ew_tab};
+    return EwaldTables{S.ew_real.p,  S.ew_four.p, S.ew_Hf.p,  S.ew_Hd.p,  S.ew_Pf.p, S.ew_Pd.p,
+                       S.ew_sep_h.p, S.ew_sep_w.p, S.ew_sep_k, S.ew_sep_r0, S.ew_sep_r2, S.ew_tab};
 }
 
 static ListView listview(Solver &S) {
@@ -680,40 +682,67 @@ static int node_ewald(Solver &S, const GParams &P, const ListView &LV, const Ewa
 static int leaf_ewald(Solver &S, const GParams &P, const ListView &LV, const EwaldTables &E, bool f64,
                       cudaStream_t st) {
     const int32_t nleaves = (int32_t)S.st.leaves;
-    TG_TRY(ensure(S.ew_cnt, (size_t)nleaves + 1));
-    TG_TRY(ensure(S.ew_off, (size_t)nleaves + 1));
-    k_ewald_count<<<(nleaves + 1 + 127) / 128, 128, 0, st>>>(S.idx.p, nleaves, LV, S.ew_cnt.p);
+    const int64_t nn = S.nnodes;
+    const size_t nc = 2 * ((size_t)nleaves + 1);
+    TG_TRY(ensure(S.ew_cnt, nc));
+    TG_TRY(ensure(S.ew_off, nc + 1));
+    int32_t *slot = nullptr, *nsrc_d = S.ew_off.p + nc; /* the source count sits behind the scan: one readback */
+    if (!f64) {
+        TG_TRY(ensure(S.ew_slot, (size_t)nn));
+        TG_TRY(ensure(S.ew_src, (size_t)nn));
+        slot = S.ew_slot.p;
+        TG_CUDA(cudaMemsetAsync(slot, 0xff, sizeof(int32_t) * nn, st));
+    }
+    TG_CUDA(cudaMemsetAsync(nsrc_d, 0, sizeof(int32_t), st));
+    k_ewald_count<<<(int)(((int64_t)(nleaves + 1) * 32 + 127) / 128), 128, 0, st>>>(S.idx.p, nleaves, LV, S.ew_cnt.p,
+                                                                                  slot);
     TG_TRY(launched(S));
+    if (!f64) {
+        k_ewald_slots<<<(int)((nn + 255) / 256), 256, 0, st>>>(nn, slot, S.ew_src.p, nsrc_d);
+        TG_TRY(launched(S));
+    }
     size_t stmp = 0;
-    TG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, stmp, S.ew_cnt.p, S.ew_off.p, nleaves + 1, st));
+    TG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, stmp, S.ew_cnt.p, S.ew_off.p, (int)nc, st));
     TG_TRY(ensure(S.cub_tmp, stmp));
-    TG_CUDA(cub::DeviceScan::ExclusiveSum(S.cub_tmp.p, stmp, S.ew_cnt.p, S.ew_off.p, nleaves + 1, st));
-    int32_t total = 0;
-    TG_TRY(read_small(S, st, &total, S.ew_off.p + nleaves, sizeof(int32_t)));
+    TG_CUDA(cub::DeviceScan::ExclusiveSum(S.cub_tmp.p, stmp, S.ew_cnt.p, S.ew_off.p, (int)nc, st));
+    /* off[nleaves]: PP_E chunks; off[nc - 1]: all chunks; then the PP_E source leaves */
+    TG_CUDA(cudaMemcpyAsync(S.h_small + 2048, S.ew_off.p + nleaves, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    TG_CUDA(cudaMemcpyAsync(S.h_small + 2052, S.ew_off.p + nc - 1, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    TG_CUDA(cudaStreamSynchronize(st));
+    int32_t tot[3];
+    std::memcpy(tot, S.h_small + 2048, sizeof(tot));
+    const int32_t npp = tot[0], total = tot[1], nsrc = tot[2];
     if (total <= 0) return TG_OK;
     TG_TRY(ensure(S.ew_part, (size_t)total * 64 * 4));
-    float *tpart = nullptr;
-    if (f64) {
-        k_ewald_chunk<double, false><<<total, 64, 0, st>>>(P, S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p,
-                                                           S.nd_ms.p, S.pos.p, S.nd_aabb.p, LV, E, S.ew_part.p, nullptr,
-                                                           nullptr, nullptr);
-    } else {
-        /* reciprocal terms per sink leaf: (cos, sin) tables per node, sums per leaf */
-        const int64_t nn = S.nnodes;
-        TG_TRY(ensure(S.ew_nt, (size_t)nn * NFOUR_HALF));
-        TG_TRY(ensure(S.ew_sf, (size_t)nn * NFOUR_HALF));
-        TG_TRY(ensure(S.ew_tpart, (size_t)total * NFOUR_HALF * EW_SEP_K));
+    float2 *tpart = nullptr;
+    if (!f64 && npp > 0) {
+        TG_TRY(ensure(S.ew_sf, (size_t)nsrc * NSEP));
+        TG_TRY(ensure(S.ew_tpart, (size_t)npp * NSEP));
         tpart = S.ew_tpart.p;
-        k_ewald_sf<<<(int)((nn * 32 + 127) / 128), 128, 0, st>>>(nn, S.nd_pb.p, S.nd_pe.p, S.nd_child0.p, S.nd_ms.p,
-                                                                S.pos.p, E, S.ew_nt.p, S.ew_sf.p);
+        k_ewald_sf<<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E, S.ew_sf.p);
         TG_TRY(launched(S));
-        k_ewald_chunk<float, true><<<total, 64, 0, st>>>(P, S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p,
-                                                         S.nd_ms.p, S.pos.p, S.nd_aabb.p, LV, E, S.ew_part.p, S.ew_nt.p,
-                                                         S.ew_sf.p, tpart);
     }
-    TG_TRY(launched(S));
-    k_ewald_reduce<<<nleaves, 64, 0, st>>>(S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.ew_part.p, S.accd.p,
-                                           tpart, S.pos.p, E);
+    const int32_t *offp = S.ew_off.p + nleaves + 1;
+    if (npp > 0) {
+        if (f64)
+            k_ewald_pp<double><<<npp, 64, 0, st>>>(P, S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, E,
+                                                   S.ew_part.p, nullptr, nullptr, nullptr);
+        else
+            k_ewald_pp<float><<<npp, 64, 0, st>>>(P, S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, E,
+                                                  S.ew_part.p, slot, S.ew_sf.p, tpart);
+        TG_TRY(launched(S));
+    }
+    if (total > npp) {
+        if (f64)
+            k_ewald_pc<double><<<total - npp, 64, 0, st>>>(S.idx.p, nleaves, npp, offp, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p,
+                                                           S.pos.p, LV, E, S.ew_part.p);
+        else
+            k_ewald_pc<float><<<total - npp, 64, 0, st>>>(S.idx.p, nleaves, npp, offp, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p,
+                                                          S.pos.p, LV, E, S.ew_part.p);
+        TG_TRY(launched(S));
+    }
+    k_ewald_reduce<<<nleaves, 256, 0, st>>>(S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.ew_part.p, S.accd.p,
+                                            tpart, S.pos.p, E);
     TG_TRY(launched(S));
     return TG_OK;
 }

@@ -137,8 +137,12 @@ struct Solver {
     DevBuf<double> ew_Hd;
     DevBuf<float4> ew_Pf;
     DevBuf<double2> ew_Pd;
-    DevBuf<float2> ew_nt, ew_sf; /* per node and h: (cos, sin) at the centre of mass; per leaf: sums over particles */
-    DevBuf<float> ew_tpart;      /* per leaf Ewald chunk and h: 8 reciprocal-space source sums */
+    DevBuf<int4> ew_sep_h;       /* PP Ewald split: reciprocal vectors and weights */
+    DevBuf<double> ew_sep_w;
+    float ew_sep_k = 0.0f, ew_sep_r0 = 0.0f, ew_sep_r2 = 0.0f;
+    DevBuf<int32_t> ew_slot, ew_src; /* per node: its row of ew_sf, or -1; the nodes of the rows, then their count */
+    DevBuf<float2> ew_sf;        /* per PP_E source leaf and h: (cos, sin) sums over its particles */
+    DevBuf<float2> ew_tpart;     /* per PP_E chunk and h: source sums */
     bool ew_use_tab = false;       /* a periodic solver of the FP32 path */
     const float *ew_tab = nullptr; /* the device's table of local expansions (FP32 path), shared by its solvers */
     bool have_tables = false;
