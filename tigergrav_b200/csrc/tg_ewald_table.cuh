@@ -41,9 +41,14 @@ static_assert(ET_ROW == 64 && ET_A == 36, "row layout");
 /* slot of x^i y^j in a plane of constant k, by order i + j */
 __host__ __device__ constexpr int et_ij(int i, int j) { return (i + j) * (i + j + 1) / 2 + j; }
 
-/* ---- generation: one block of 64 threads per cell, a thread per coefficient ---- */
+/* ---- generation: one block of 64 threads per cell with ix >= iy, a thread per
+ * coefficient (psi is symmetric in x and y: the mirrored cell holds the same
+ * coefficients with i and j exchanged).  2.4 ms of FP64 in all. ---- */
 
-constexpr int ET_IMG = 128;       /* images within ET_CUT2 of a point of the cube: at most 110 */
+/* slot of (j, n >= j) among the pairs of 0..ET_P */
+__device__ __forceinline__ int et_jn(int j, int n) { return j * (ET_P + 1) - j * (j - 1) / 2 + n - j; }
+
+constexpr int ET_IMG = 96;        /* images within ET_CUT2 of a point of the octant: at most 94 */
 constexpr double ET_CUT2 = 7.29;  /* r < 2.7: the images beyond add 1e-12 to D0 and 1e-7 of D4's rms */
 
 /* the centre of cell q along one axis, the same FP32 value in generation and evaluation */
@@ -51,14 +56,15 @@ __device__ __forceinline__ float et_centre(int q) { return __fmul_rn((float)q + 
 
 __global__ void __launch_bounds__(64) k_ewald_table(const float4 *__restrict__ real, const float4 *__restrict__ four,
                                                     float *__restrict__ table) {
-    __shared__ double sxp[ET_IMG][ET_P + 1], syp[ET_IMG][ET_P + 1], sd[ET_IMG][ET_P + 1], sz[ET_IMG];
+    __shared__ double sxp[ET_IMG][ET_P + 1], sw[ET_IMG][ET_A], sz[ET_IMG];
     __shared__ double hp[7][ET_P + 1], hc[NFOUR_HALF], hs[NFOUR_HALF];
     __shared__ int s_img[ET_IMG], s_w[2];
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    const int c = blockIdx.x; /* ((ix ET_N) + iy) ET_N + iz */
-    const double X[3] = {(double)et_centre(c / (ET_N * ET_N)), (double)et_centre(c / ET_N % ET_N),
-                         (double)et_centre(c % ET_N)};
+    const int iz = blockIdx.x, iy = blockIdx.y, ix = blockIdx.z;
+    if (ix < iy) return; /* block-uniform */
+    const double X[3] = {(double)et_centre(ix), (double)et_centre(iy), (double)et_centre(iz)};
     const double alpha = 2.0, pi = 3.141592653589793, cexp = 2.0 * alpha / 1.7724538509055159; /* 2 alpha / sqrt(pi) */
+    const double ch[4] = {1.0, 0.5, 0.125, 1.0 / 48.0}; /* 1 / (p! 2^p) */
     const double rfact[ET_P + 1] = {1.0, 1.0, 1.0 / 2, 1.0 / 6, 1.0 / 24, 1.0 / 120, 1.0 / 720, 1.0 / 5040};
     /* the images inside the cut, in table order */
     int nimg = 0;
@@ -85,10 +91,11 @@ __global__ void __launch_bounds__(64) k_ewald_table(const float4 *__restrict__ r
         const double r2 = dx * dx + dy * dy + dz * dz;
         const double r = sqrt(r2), e2 = exp(-alpha * alpha * r2);
         sz[q] = dz;
-        double px = 1.0, py = 1.0;
+        double px = 1.0, py = 1.0, yp[ET_P + 1], rd[ET_P + 1];
+#pragma unroll
         for (int e = 0; e <= ET_P; e++) {
             sxp[q][e] = px * rfact[e];
-            syp[q][e] = py * rfact[e];
+            yp[e] = py * rfact[e];
             px *= dx;
             py *= dy;
         }
@@ -103,9 +110,11 @@ __global__ void __launch_bounds__(64) k_ewald_table(const float4 *__restrict__ r
             }
             F *= e2;
             double w = cexp;
+#pragma unroll
             for (int m = 0; m < ET_P; m++) w *= -2.0 * alpha * alpha;
+#pragma unroll
             for (int m = ET_P; m >= 0; m--) {
-                sd[q][m] = w * F;
+                rd[m] = w * F;
                 w /= -2.0 * alpha * alpha;
                 if (m > 0) F = (2.0 * T * F + e2) / (2 * m - 1);
             }
@@ -113,12 +122,23 @@ __global__ void __launch_bounds__(64) k_ewald_table(const float4 *__restrict__ r
             /* g_0 = erfc(alpha r)/r, r^2 g_(n+1) = -(2n+1) g_n - (-2 alpha^2)^n cexp e^(-alpha^2 r^2) */
             double g = erfc(alpha * r) / r, w = cexp * e2;
             const double r2inv = 1.0 / r2;
+#pragma unroll
             for (int m = 0; m <= ET_P; m++) {
-                sd[q][m] = -g;
+                rd[m] = -g;
                 g = -((2 * m + 1) * g + w) * r2inv;
                 w *= -2.0 * alpha * alpha;
             }
         }
+        /* the y part: sum_s y^(j-2s)/(j-2s)! d_(n-s) / (s! 2^s) */
+#pragma unroll
+        for (int j = 0; j <= ET_P; j++)
+#pragma unroll
+            for (int n = j; n <= ET_P; n++) {
+                double u = 0.0;
+#pragma unroll
+                for (int s = 0; 2 * s <= j; s++) u += ch[s] * yp[j - 2 * s] * rd[n - s];
+                sw[q][et_jn(j, n)] = u;
+            }
     }
     /* reciprocal vectors (one of each pair +-h): -(2/pi) c_h (cos, sin)(2 pi h.X), and (2 pi h)^e / e! */
     if (tid < NFOUR_HALF) {
@@ -146,17 +166,12 @@ __global__ void __launch_bounds__(64) k_ewald_table(const float4 *__restrict__ r
         i = s + 1;
     }
     i -= j; /* i held the order */
-    const double ch[4] = {1.0, 0.5, 0.125, 1.0 / 48.0}; /* 1 / (p! 2^p) */
     double t = 0.0;
     for (int q = 0; q < nimg; q++) {
         /* D_ij0 / (i! j!) = sum_{p,s} x^(i-2p)/(i-2p)! y^(j-2s)/(j-2s)! d_(i+j-p-s) / (p! 2^p s! 2^s);
          * one more radial derivative times z for k = 1 */
         double v = 0.0;
-        for (int p = 0; 2 * p <= i; p++) {
-            double u = 0.0;
-            for (int s = 0; 2 * s <= j; s++) u += ch[s] * syp[q][j - 2 * s] * sd[q][i + j - p - s + kz];
-            v += ch[p] * sxp[q][i - 2 * p] * u;
-        }
+        for (int p = 0; 2 * p <= i; p++) v += ch[p] * sxp[q][i - 2 * p] * sw[q][et_jn(j, i + j - p + kz)];
         t += kz ? v * sz[q] : v;
     }
     const int n = i + j + kz; /* cos differentiated n times: cos, -sin, -cos, sin */
@@ -169,7 +184,8 @@ __global__ void __launch_bounds__(64) k_ewald_table(const float4 *__restrict__ r
     }
     t += ((n & 3) == 1 || (n & 3) == 2) ? -rec : rec;
     if (tid == 0) t += 0.78539816339744831 + ET_OFFSET; /* pi/4 (tigergrav/green.hpp:270) */
-    table[(int64_t)c * ET_ROW + tid] = (float)t;
+    table[(((int64_t)ix * ET_N + iy) * ET_N + iz) * ET_ROW + tid] = (float)t;
+    table[(((int64_t)iy * ET_N + ix) * ET_N + iz) * ET_ROW + (kz ? ET_A : 0) + et_ij(j, i)] = (float)t;
 }
 
 /* ---- evaluation ---- */
@@ -344,7 +360,7 @@ int ewald_table_acquire(int dev, const float4 *real, const float4 *four, const f
             cudaGetLastError();
             return TG_ERR_NOMEM;
         }
-        k_ewald_table<<<ET_N * ET_N * ET_N, 64, 0, st>>>(real, four, p);
+        k_ewald_table<<<dim3(ET_N, ET_N, ET_N), 64, 0, st>>>(real, four, p);
         /* complete before any other stream or thread may read it */
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
