@@ -52,6 +52,12 @@ struct __align__(16) MSrc {
 };
 static_assert(sizeof(MSrc) == 80, "multi_src layout");
 
+/* a node as a check item, one 32-byte sector: COM x, y, z and r (float bits);
+ * child0, or NODE_EMPTY for a node without particles */
+struct __align__(32) WalkRec {
+    int4 x, kind;
+};
+
 template <class T>
 struct DevBuf {
     T *p = nullptr;
@@ -102,8 +108,7 @@ struct Solver {
     DevBuf<int32_t *> wk_pools, wk_llen; /* device copies of the list pointer tables */
     DevBuf<int64_t *> wk_loff;
     DevBuf<int64_t> wk_caps;
-    DevBuf<int4> wk_wx;                  /* per node: COM and r packed for the opening tests */
-    DevBuf<int32_t> wk_kind;             /* per node: child0, or empty */
+    DevBuf<WalkRec> wk_rec;              /* per node: what the opening tests read */
     DevBuf<int32_t> scratch;             /* leaf drain per-warp scratch */
     int64_t scratch_per_warp = 0;
     int drain_warps = 0;

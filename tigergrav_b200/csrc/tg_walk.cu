@@ -29,6 +29,7 @@
  * write out of bounds: they set a flag and the host regrows and repeats.
  */
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "tg_solver.cuh"
@@ -40,6 +41,8 @@ struct WalkParams {
     double h;
     float r_ewald;
     int ewald;
+    int quick;              /* theta_inv and h are in FP32's range: far_quick may decide */
+    float theta_inv_f, h_f;
     const int32_t *nact; /* active particles per node (rung steps); nullptr: every particle is a sink */
 };
 
@@ -50,23 +53,21 @@ struct NodeView {
     const int32_t *pb, *pe, *child0;
     const MSrc *ms;
     const float *r, *rmax;
-    /* what the opening test reads of a check item, packed: (COM x, y, z, r
-     * bits) and child0, or NODE_EMPTY for a node without particles -- two
-     * loads per item instead of six scattered ones */
-    const int4 *wx;
-    const int32_t *kind;
+    const WalkRec *rec; /* what the opening test reads of a check item */
 };
 
 constexpr int32_t NODE_EMPTY = -2;
 
-/* the packed records of NodeView::wx / kind, one thread per node */
+/* the packed records, one thread per node */
 __global__ void k_walk_records(int64_t nn, const int32_t *__restrict__ pb, const int32_t *__restrict__ pe,
                                const int32_t *__restrict__ child0, const MSrc *__restrict__ ms,
-                               const float *__restrict__ r, int4 *__restrict__ wx, int32_t *__restrict__ kind) {
+                               const float *__restrict__ r, WalkRec *__restrict__ rec) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nn) return;
-    wx[i] = make_int4(ms[i].x[0], ms[i].x[1], ms[i].x[2], __float_as_int(r[i]));
-    kind[i] = pe[i] == pb[i] ? NODE_EMPTY : child0[i];
+    WalkRec q;
+    q.x = make_int4(ms[i].x[0], ms[i].x[1], ms[i].x[2], __float_as_int(r[i]));
+    q.kind = make_int4(pe[i] == pb[i] ? NODE_EMPTY : child0[i], 0, 0, 0);
+    rec[i] = q;
 }
 
 __device__ __forceinline__ double near_sep(const double *x) {
@@ -117,22 +118,94 @@ __device__ __forceinline__ bool far_ewald(const WalkParams &W, const double *X, 
 /* classification codes */
 enum { C_SKIP = 0, C_FAR_OPEN = 1, C_FAR = 2, C_NEAR_LEAF = 3, C_NEAR_INT = 4 };
 
-__device__ __forceinline__ int classify(const WalkParams &W, const NodeView &V, bool ewald_list, const double *X,
-                                        float r, float rmax, uint32_t item, int32_t nnodes, uint32_t *err) {
-    const int32_t c = (int32_t)(item & ID_MASK);
-    if (c >= nnodes) {
-        atomicOr(err, DEV_ERR_BADINDEX);
-        return C_SKIP;
+/* The opening test in FP32 where its outcome is certain: 1 far, 0 near, -1
+ * undecided (the FP64 test above decides).  The squared distance comes from the
+ * fixed-point difference (exact; its int32 wrap is the minimum image) and is
+ * compared with the squared threshold max(rs / theta, rs + h); both are within
+ * 1e-6 of the FP64 test's values, and a pair closer to the threshold than 4e-6
+ * is left to it, so every decision is the reference's.  The FP64 test costs ~60
+ * FP64 instructions with a square root; about 1 item in 10^5 takes it. */
+__device__ __forceinline__ int far_quick(const WalkParams &W, bool ewald_list, const int32_t *Xi, float r, int4 c) {
+    const float u = 2.3283064365386963e-10f;
+    float dx, dy, dz;
+    if (W.ewald) {
+        dx = __int2float_rn((int32_t)((uint32_t)Xi[0] - (uint32_t)c.x)) * u;
+        dy = __int2float_rn((int32_t)((uint32_t)Xi[1] - (uint32_t)c.y)) * u;
+        dz = __int2float_rn((int32_t)((uint32_t)Xi[2] - (uint32_t)c.z)) * u;
+    } else {
+        dx = __ll2float_rn((long long)Xi[0] - c.x) * u;
+        dy = __ll2float_rn((long long)Xi[1] - c.y) * u;
+        dz = __ll2float_rn((long long)Xi[2] - c.z) * u;
     }
-    const int32_t k = V.kind[c];
-    if (k == NODE_EMPTY) return C_SKIP;
-    const int4 q = V.wx[c];
-    const int32_t cx[3] = {q.x, q.y, q.z};
-    const float cr = __int_as_float(q.w);
-    const bool far = ewald_list ? far_ewald(W, X, r, rmax, cx, cr) : far_direct(W, X, r, cx, cr);
-    if (far) return (item & OPENED) ? C_FAR_OPEN : C_FAR;
-    return k < 0 ? C_NEAR_LEAF : C_NEAR_INT;
+    float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    if (ewald_list) {
+        if (Xi[0] == c.x && Xi[1] == c.y && Xi[2] == c.z) return -1; /* the self test is another one */
+        d2 = fmaxf(0.0625f, d2); /* ewald_far_separation: at least 1/4 */
+    }
+    const float rs = __fadd_rn(r, __int_as_float(c.w));
+    const float t = fmaxf(rs * W.theta_inv_f, rs + W.h_f), t2 = t * t;
+    if (d2 > t2 * 1.000004f) return 1;
+    if (d2 < t2 * 0.999996f) return 0;
+    return -1;
 }
+
+/* the sink node of a walk */
+struct WalkSink {
+    int32_t Xi[3];
+    float r, rmax;
+};
+
+__device__ __forceinline__ int classify(const WalkParams &W, bool ewald_list, const WalkSink &A, uint32_t item, int4 q,
+                                        int32_t kind) {
+    if (kind == NODE_EMPTY) return C_SKIP;
+    int far = W.quick ? far_quick(W, ewald_list, A.Xi, A.r, q) : -1;
+    if (far < 0) {
+        const double X[3] = {pos2d(A.Xi[0]), pos2d(A.Xi[1]), pos2d(A.Xi[2])};
+        const int32_t cx[3] = {q.x, q.y, q.z};
+        const float cr = __int_as_float(q.w);
+        far = ewald_list ? far_ewald(W, X, A.r, A.rmax, cx, cr) : far_direct(W, X, A.r, cx, cr);
+    }
+    if (far) return (item & OPENED) ? C_FAR_OPEN : C_FAR;
+    return kind < 0 ? C_NEAR_LEAF : C_NEAR_INT;
+}
+
+/* Classify items [base, base + 32 WK_ILP) of a check list, WK_ILP per lane
+ * (item base + 32 u + lane): all loads of a step are issued before any is used.
+ * The walk waits on these records (one 32-byte sector per item, scattered over
+ * L2), so the items in flight per warp set its pace. */
+constexpr int WK_ILP = 4;
+__device__ __forceinline__ void classify_step(const WalkParams &W, const NodeView &V, bool ewald_list, const WalkSink &A,
+                                              const int32_t *in, int32_t base, int32_t nin, int32_t nnodes,
+                                              uint32_t *item, int *code, uint32_t *err) {
+    const int lane = threadIdx.x & 31;
+    int4 q[WK_ILP];
+    int32_t kind[WK_ILP];
+#pragma unroll
+    for (int u = 0; u < WK_ILP; u++) {
+        const int32_t j = base + 32 * u + lane;
+        item[u] = j < nin ? (uint32_t)in[j] : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < WK_ILP; u++) {
+        const int32_t c = (int32_t)(item[u] & ID_MASK);
+        const bool ok = base + 32 * u + lane < nin && c < nnodes;
+        kind[u] = NODE_EMPTY;
+        q[u] = make_int4(0, 0, 0, 0);
+        if (ok) {
+            q[u] = V.rec[c].x;
+            kind[u] = V.rec[c].kind.x;
+        } else if (base + 32 * u + lane < nin) {
+            atomicOr(err, DEV_ERR_BADINDEX);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < WK_ILP; u++) code[u] = classify(W, ewald_list, A, item[u], q[u], kind[u]);
+}
+
+/* codes of the first WK_CODES items, kept from the counting pass for the
+ * writing pass (a byte per item, each read by the lane that wrote it) */
+constexpr int WK_CODES = 2048;
+constexpr int WK_TPB = 128; /* threads per block of both walk kernels */
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
@@ -141,8 +214,8 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 }
 
 /* Node stage for one list of one node (src/tree.cpp:424-476). */
-__device__ void node_stage_list(const WalkParams &W, const NodeView &V, bool ewald_list, const double *X, float r,
-                                float rmax, const int32_t *in, int32_t nin, int32_t nnodes, int32_t *pool_cc,
+__device__ void node_stage_list(const WalkParams &W, const NodeView &V, bool ewald_list, const WalkSink &A,
+                                const int32_t *in, int32_t nin, int32_t nnodes, unsigned char *codes, int32_t *pool_cc,
                                 int64_t cap_cc, unsigned long long *top_cc, int64_t *off_cc, int32_t *len_cc,
                                 int32_t *pool_cp, int64_t cap_cp, unsigned long long *top_cp, int64_t *off_cp,
                                 int32_t *len_cp, int32_t *pool_nx, int64_t cap_nx, unsigned long long *top_nx,
@@ -150,15 +223,23 @@ __device__ void node_stage_list(const WalkParams &W, const NodeView &V, bool ewa
     const int lane = threadIdx.x & 31;
     /* pass 1: counts */
     int n_cc = 0, n_cp = 0, n_lf = 0, n_int = 0;
-    for (int32_t base = 0; base < nin; base += 32) {
-        const int32_t j = base + lane;
-        int code = C_SKIP;
-        if (j < nin) code = classify(W, V, ewald_list, X, r, rmax, (uint32_t)in[j], nnodes, err);
-        n_cp += __popc(__ballot_sync(0xffffffffu, code == C_FAR_OPEN));
-        n_cc += __popc(__ballot_sync(0xffffffffu, code == C_FAR));
-        n_lf += __popc(__ballot_sync(0xffffffffu, code == C_NEAR_LEAF));
-        n_int += __popc(__ballot_sync(0xffffffffu, code == C_NEAR_INT));
+    for (int32_t base = 0; base < nin; base += 32 * WK_ILP) {
+        uint32_t item[WK_ILP];
+        int code[WK_ILP];
+        classify_step(W, V, ewald_list, A, in, base, nin, nnodes, item, code, err);
+#pragma unroll
+        for (int u = 0; u < WK_ILP; u++) {
+            n_cp += code[u] == C_FAR_OPEN;
+            n_cc += code[u] == C_FAR;
+            n_lf += code[u] == C_NEAR_LEAF;
+            n_int += code[u] == C_NEAR_INT;
+            if (base < WK_CODES) codes[base + 32 * u + lane] = (unsigned char)code[u];
+        }
     }
+    n_cp = __reduce_add_sync(0xffffffffu, n_cp);
+    n_cc = __reduce_add_sync(0xffffffffu, n_cc);
+    n_lf = __reduce_add_sync(0xffffffffu, n_lf);
+    n_int = __reduce_add_sync(0xffffffffu, n_int);
     const int n_nx = n_lf + 2 * n_int;
     unsigned long long b_cc = 0, b_cp = 0, b_nx = 0;
     int ok = 1;
@@ -189,32 +270,41 @@ __device__ void node_stage_list(const WalkParams &W, const NodeView &V, bool ewa
     /* pass 2: write */
     int r_cc = 0, r_cp = 0, r_lf = 0, r_int = 0;
     const uint32_t lt = lanemask_lt();
-    for (int32_t base = 0; base < nin; base += 32) {
-        const int32_t j = base + lane;
-        int code = C_SKIP;
-        uint32_t item = 0;
-        if (j < nin) {
-            item = (uint32_t)in[j];
-            code = classify(W, V, ewald_list, X, r, rmax, item, nnodes, err);
+    for (int32_t base = 0; base < nin; base += 32 * WK_ILP) {
+        uint32_t item[WK_ILP];
+        int code[WK_ILP];
+        if (base < WK_CODES) {
+#pragma unroll
+            for (int u = 0; u < WK_ILP; u++) {
+                const int32_t j = base + 32 * u + lane;
+                item[u] = j < nin ? (uint32_t)in[j] : 0u;
+                code[u] = codes[j];
+            }
+        } else {
+            classify_step(W, V, ewald_list, A, in, base, nin, nnodes, item, code, err);
         }
-        const uint32_t m_cp = __ballot_sync(0xffffffffu, code == C_FAR_OPEN);
-        const uint32_t m_cc = __ballot_sync(0xffffffffu, code == C_FAR);
-        const uint32_t m_lf = __ballot_sync(0xffffffffu, code == C_NEAR_LEAF);
-        const uint32_t m_in = __ballot_sync(0xffffffffu, code == C_NEAR_INT);
-        const int32_t id = (int32_t)(item & ID_MASK);
-        if (code == C_FAR_OPEN) pool_cp[b_cp + r_cp + __popc(m_cp & lt)] = id;
-        if (code == C_FAR) pool_cc[b_cc + r_cc + __popc(m_cc & lt)] = id;
-        if (code == C_NEAR_LEAF) pool_nx[b_nx + r_lf + __popc(m_lf & lt)] = (int32_t)(item | OPENED);
-        if (code == C_NEAR_INT) {
-            const int32_t c0 = V.kind[id]; /* an internal node: its child0 */
-            const int64_t q = b_nx + n_lf + 2 * (r_int + __popc(m_in & lt));
-            pool_nx[q] = c0;
-            pool_nx[q + 1] = c0 + 1;
+#pragma unroll
+        for (int u = 0; u < WK_ILP; u++) {
+            if (base + 32 * u >= nin) break;
+            const uint32_t m_cp = __ballot_sync(0xffffffffu, code[u] == C_FAR_OPEN);
+            const uint32_t m_cc = __ballot_sync(0xffffffffu, code[u] == C_FAR);
+            const uint32_t m_lf = __ballot_sync(0xffffffffu, code[u] == C_NEAR_LEAF);
+            const uint32_t m_in = __ballot_sync(0xffffffffu, code[u] == C_NEAR_INT);
+            const int32_t id = (int32_t)(item[u] & ID_MASK);
+            if (code[u] == C_FAR_OPEN) pool_cp[b_cp + r_cp + __popc(m_cp & lt)] = id;
+            if (code[u] == C_FAR) pool_cc[b_cc + r_cc + __popc(m_cc & lt)] = id;
+            if (code[u] == C_NEAR_LEAF) pool_nx[b_nx + r_lf + __popc(m_lf & lt)] = (int32_t)(item[u] | OPENED);
+            if (code[u] == C_NEAR_INT) {
+                const int32_t c0 = V.rec[id].kind.x; /* an internal node: its child0 */
+                const int64_t q = b_nx + n_lf + 2 * (r_int + __popc(m_in & lt));
+                pool_nx[q] = c0;
+                pool_nx[q + 1] = c0 + 1;
+            }
+            r_cp += __popc(m_cp);
+            r_cc += __popc(m_cc);
+            r_lf += __popc(m_lf);
+            r_int += __popc(m_in);
         }
-        r_cp += __popc(m_cp);
-        r_cc += __popc(m_cc);
-        r_lf += __popc(m_lf);
-        r_int += __popc(m_in);
     }
 }
 
@@ -224,6 +314,8 @@ __global__ void k_node_stage(WalkParams W, NodeView V, int64_t first, int64_t co
                              const int32_t *nx_in_e, int32_t *nx_out_d, int32_t *nx_out_e, int64_t cap_nx_d,
                              int64_t cap_nx_e, unsigned long long *nx_top, int64_t *nx_off_d, int32_t *nx_len_d,
                              int64_t *nx_off_e, int32_t *nx_len_e, uint32_t *err) {
+    __shared__ unsigned char s_codes[WK_TPB / 32][WK_CODES];
+    unsigned char *const codes = s_codes[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (k >= count) return;
@@ -238,8 +330,7 @@ __global__ void k_node_stage(WalkParams W, NodeView V, int64_t first, int64_t co
         return;
     }
     const MSrc &s = V.ms[i];
-    const double X[3] = {pos2d(s.x[0]), pos2d(s.x[1]), pos2d(s.x[2])};
-    const float r = V.r[i], rmax = V.rmax[i];
+    const WalkSink A{{s.x[0], s.x[1], s.x[2]}, V.r[i], V.rmax[i]};
     const int32_t root_item = 0;
     const int32_t *in_d, *in_e;
     int32_t nin_d, nin_e;
@@ -254,20 +345,31 @@ __global__ void k_node_stage(WalkParams W, NodeView V, int64_t first, int64_t co
         in_e = nx_in_e + nx_off_e[p];
         nin_e = W.ewald ? nx_len_e[p] : 0;
     }
-    node_stage_list(W, V, false, X, r, rmax, in_d, nin_d, nnodes, pools[TG_CC_D], caps[TG_CC_D], &tops[TG_CC_D],
+    node_stage_list(W, V, false, A, in_d, nin_d, nnodes, codes, pools[TG_CC_D], caps[TG_CC_D], &tops[TG_CC_D],
                     &loff[TG_CC_D][i], &llen[TG_CC_D][i], pools[TG_CP_D], caps[TG_CP_D], &tops[TG_CP_D],
                     &loff[TG_CP_D][i], &llen[TG_CP_D][i], nx_out_d, cap_nx_d, &nx_top[0], &nx_off_d[i],
                     &nx_len_d[i], err);
-    node_stage_list(W, V, true, X, r, rmax, in_e, nin_e, nnodes, pools[TG_CC_E], caps[TG_CC_E], &tops[TG_CC_E],
+    node_stage_list(W, V, true, A, in_e, nin_e, nnodes, codes, pools[TG_CC_E], caps[TG_CC_E], &tops[TG_CC_E],
                     &loff[TG_CC_E][i], &llen[TG_CC_E][i], pools[TG_CP_E], caps[TG_CP_E], &tops[TG_CP_E],
                     &loff[TG_CP_E][i], &llen[TG_CP_E][i], nx_out_e, cap_nx_e, &nx_top[1], &nx_off_e[i],
                     &nx_len_e[i], err);
 }
 
+/* classify_step for the drain: an opened leaf goes to PP regardless of distance
+ * (C_FAR_OPEN), any other far item to PC (C_FAR) */
+__device__ __forceinline__ void drain_step(const WalkParams &W, const NodeView &V, bool ewald_list, const WalkSink &A,
+                                           const int32_t *in, int32_t base, int32_t nin, int32_t nnodes, uint32_t *item,
+                                           int *code, uint32_t *err) {
+    classify_step(W, V, ewald_list, A, in, base, nin, nnodes, item, code, err);
+#pragma unroll
+    for (int u = 0; u < WK_ILP; u++)
+        if (code[u] != C_SKIP && (item[u] & OPENED)) code[u] = C_FAR_OPEN;
+}
+
 /* Leaf drain for one list (src/tree.cpp:530-602); scratch layout per warp:
  * [bufA | bufB | outPP | outPC], each `cap` entries. */
-__device__ void drain_list(const WalkParams &W, const NodeView &V, bool ewald_list, const double *X, float r,
-                           float rmax, const int32_t *in, int32_t nin, int32_t nnodes, int32_t *scr, int64_t cap,
+__device__ void drain_list(const WalkParams &W, const NodeView &V, bool ewald_list, const WalkSink &A,
+                           const int32_t *in, int32_t nin, int32_t nnodes, unsigned char *codes, int32_t *scr, int64_t cap,
                            int32_t *pool_pp, int64_t cap_pp, unsigned long long *top_pp, int64_t *off_pp,
                            int32_t *len_pp, int32_t *pool_pc, int64_t cap_pc, unsigned long long *top_pc,
                            int64_t *off_pc, int32_t *len_pc, uint32_t *err) {
@@ -286,58 +388,67 @@ __device__ void drain_list(const WalkParams &W, const NodeView &V, bool ewald_li
             break;
         }
         int32_t *nxt = (cur == bufA) ? bufB : bufA;
-        /* pass 1: count opened-leaf entries of the next list (to order children after them) */
+        /* pass 1: count opened-leaf entries of the next list (to order children after them);
+         * an item's code: C_FAR_OPEN opened (PP), C_FAR far (PC), C_NEAR_LEAF, C_NEAR_INT */
         int n_lf = 0, n_int = 0, c_pp = 0, c_pc = 0;
-        for (int32_t base = 0; base < ncur; base += 32) {
-            const int32_t j = base + lane;
-            int code = C_SKIP;
-            uint32_t item = 0;
-            if (j < ncur) {
-                item = (uint32_t)cur[j];
-                code = classify(W, V, ewald_list, X, r, rmax, item, nnodes, err);
+        for (int32_t base = 0; base < ncur; base += 32 * WK_ILP) {
+            uint32_t item[WK_ILP];
+            int code[WK_ILP];
+            drain_step(W, V, ewald_list, A, cur, base, ncur, nnodes, item, code, err);
+#pragma unroll
+            for (int u = 0; u < WK_ILP; u++) {
+                c_pp += code[u] == C_FAR_OPEN;
+                c_pc += code[u] == C_FAR;
+                n_lf += code[u] == C_NEAR_LEAF;
+                n_int += code[u] == C_NEAR_INT;
+                if (base < WK_CODES) codes[base + 32 * u + lane] = (unsigned char)code[u];
             }
-            const bool opened = (item & OPENED) && code != C_SKIP;
-            c_pp += __popc(__ballot_sync(0xffffffffu, opened));
-            c_pc += __popc(__ballot_sync(0xffffffffu, !opened && (code == C_FAR || code == C_FAR_OPEN)));
-            n_lf += __popc(__ballot_sync(0xffffffffu, !opened && code == C_NEAR_LEAF));
-            n_int += __popc(__ballot_sync(0xffffffffu, !opened && code == C_NEAR_INT));
         }
+        c_pp = __reduce_add_sync(0xffffffffu, c_pp);
+        c_pc = __reduce_add_sync(0xffffffffu, c_pc);
+        n_lf = __reduce_add_sync(0xffffffffu, n_lf);
+        n_int = __reduce_add_sync(0xffffffffu, n_int);
         if (n_pp + c_pp > cap || n_pc + c_pc > cap || n_lf + 2 * n_int > cap) {
             if (lane == 0) atomicOr(err, DEV_ERR_OVERFLOW_SCRATCH);
             ok = false;
             break;
         }
         int r_lf = 0, r_int = 0;
-        for (int32_t base = 0; base < ncur; base += 32) {
-            const int32_t j = base + lane;
-            int code = C_SKIP;
-            uint32_t item = 0;
-            if (j < ncur) {
-                item = (uint32_t)cur[j];
-                code = classify(W, V, ewald_list, X, r, rmax, item, nnodes, err);
+        for (int32_t base = 0; base < ncur; base += 32 * WK_ILP) {
+            uint32_t item[WK_ILP];
+            int code[WK_ILP];
+            if (base < WK_CODES) {
+#pragma unroll
+                for (int u = 0; u < WK_ILP; u++) {
+                    const int32_t j = base + 32 * u + lane;
+                    item[u] = j < ncur ? (uint32_t)cur[j] : 0u;
+                    code[u] = codes[j];
+                }
+            } else {
+                drain_step(W, V, ewald_list, A, cur, base, ncur, nnodes, item, code, err);
             }
-            const bool opened = (item & OPENED) && code != C_SKIP;
-            const bool pc = !opened && (code == C_FAR || code == C_FAR_OPEN);
-            const bool lf = !opened && code == C_NEAR_LEAF;
-            const bool in_ = !opened && code == C_NEAR_INT;
-            const uint32_t m_pp = __ballot_sync(0xffffffffu, opened);
-            const uint32_t m_pc = __ballot_sync(0xffffffffu, pc);
-            const uint32_t m_lf = __ballot_sync(0xffffffffu, lf);
-            const uint32_t m_in = __ballot_sync(0xffffffffu, in_);
-            const int32_t id = (int32_t)(item & ID_MASK);
-            if (opened) outPP[n_pp + __popc(m_pp & lt)] = id;
-            if (pc) outPC[n_pc + __popc(m_pc & lt)] = id;
-            if (lf) nxt[r_lf + __popc(m_lf & lt)] = (int32_t)(item | OPENED);
-            if (in_) {
-                const int32_t c0 = V.kind[id]; /* an internal node: its child0 */
-                const int32_t q = n_lf + 2 * (r_int + __popc(m_in & lt));
-                nxt[q] = c0;
-                nxt[q + 1] = c0 + 1;
+#pragma unroll
+            for (int u = 0; u < WK_ILP; u++) {
+                if (base + 32 * u >= ncur) break;
+                const uint32_t m_pp = __ballot_sync(0xffffffffu, code[u] == C_FAR_OPEN);
+                const uint32_t m_pc = __ballot_sync(0xffffffffu, code[u] == C_FAR);
+                const uint32_t m_lf = __ballot_sync(0xffffffffu, code[u] == C_NEAR_LEAF);
+                const uint32_t m_in = __ballot_sync(0xffffffffu, code[u] == C_NEAR_INT);
+                const int32_t id = (int32_t)(item[u] & ID_MASK);
+                if (code[u] == C_FAR_OPEN) outPP[n_pp + __popc(m_pp & lt)] = id;
+                if (code[u] == C_FAR) outPC[n_pc + __popc(m_pc & lt)] = id;
+                if (code[u] == C_NEAR_LEAF) nxt[r_lf + __popc(m_lf & lt)] = (int32_t)(item[u] | OPENED);
+                if (code[u] == C_NEAR_INT) {
+                    const int32_t c0 = V.rec[id].kind.x; /* an internal node: its child0 */
+                    const int32_t q = n_lf + 2 * (r_int + __popc(m_in & lt));
+                    nxt[q] = c0;
+                    nxt[q + 1] = c0 + 1;
+                }
+                n_pp += __popc(m_pp);
+                n_pc += __popc(m_pc);
+                r_lf += __popc(m_lf);
+                r_int += __popc(m_in);
             }
-            n_pp += __popc(m_pp);
-            n_pc += __popc(m_pc);
-            r_lf += __popc(m_lf);
-            r_int += __popc(m_in);
         }
         __syncwarp();
         cur = nxt;
@@ -375,6 +486,8 @@ __global__ void k_leaf_drain(WalkParams W, NodeView V, int64_t first, int64_t co
                              const int64_t *nx_off_d, const int32_t *nx_len_d, const int64_t *nx_off_e,
                              const int32_t *nx_len_e, int32_t *scratch, int64_t scr_cap,
                              unsigned long long *work_counter, uint32_t *err) {
+    __shared__ unsigned char s_codes[WK_TPB / 32][WK_CODES];
+    unsigned char *const codes = s_codes[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int32_t *scr = scratch + warp * 4 * scr_cap;
@@ -387,13 +500,12 @@ __global__ void k_leaf_drain(WalkParams W, NodeView V, int64_t first, int64_t co
         /* the leaves of this level with (active) particles */
         if (V.child0[i] >= 0 || V.pe[i] == V.pb[i] || (W.nact && W.nact[i] == 0)) continue;
         const MSrc &s = V.ms[i];
-        const double X[3] = {pos2d(s.x[0]), pos2d(s.x[1]), pos2d(s.x[2])};
-        const float r = V.r[i], rmax = V.rmax[i];
-        drain_list(W, V, false, X, r, rmax, nx_pool_d + nx_off_d[i], nx_len_d[i], nnodes, scr, scr_cap,
+        const WalkSink A{{s.x[0], s.x[1], s.x[2]}, V.r[i], V.rmax[i]};
+        drain_list(W, V, false, A, nx_pool_d + nx_off_d[i], nx_len_d[i], nnodes, codes, scr, scr_cap,
                    pools[TG_PP_D], caps[TG_PP_D], &tops[TG_PP_D], &loff[TG_PP_D][i], &llen[TG_PP_D][i],
                    pools[TG_PC_D], caps[TG_PC_D], &tops[TG_PC_D], &loff[TG_PC_D][i], &llen[TG_PC_D][i], err);
         if (W.ewald) {
-            drain_list(W, V, true, X, r, rmax, nx_pool_e + nx_off_e[i], nx_len_e[i], nnodes, scr, scr_cap,
+            drain_list(W, V, true, A, nx_pool_e + nx_off_e[i], nx_len_e[i], nnodes, codes, scr, scr_cap,
                        pools[TG_PP_E], caps[TG_PP_E], &tops[TG_PP_E], &loff[TG_PP_E][i], &llen[TG_PP_E][i],
                        pools[TG_PC_E], caps[TG_PC_E], &tops[TG_PC_E], &loff[TG_PC_E][i], &llen[TG_PC_E][i], err);
         } else if (lane == 0) {
@@ -431,12 +543,14 @@ int tree_walk(Solver &S, cudaStream_t st) {
     W.r_ewald = (float)(2.0 * S.prm.theta * std::pow(1.0e-3 / 8.0, 1.0 / 3.0));
     W.ewald = S.prm.ewald ? 1 : 0;
     W.nact = S.walk_nact;
-    TG_TRY(ensure(S.wk_wx, nn));
-    TG_TRY(ensure(S.wk_kind, nn));
+    W.theta_inv_f = (float)W.theta_inv;
+    W.h_f = (float)W.h;
+    W.quick = W.theta_inv < 1.0e15 && W.h < 1.0e15; /* squares stay finite; NaN cannot occur */
+    TG_TRY(ensure(S.wk_rec, nn));
     k_walk_records<<<(int)((nn + 255) / 256), 256, 0, st>>>(nn, S.nd_pb.p, S.nd_pe.p, S.nd_child0.p, S.nd_ms.p,
-                                                            S.nd_r.p, S.wk_wx.p, S.wk_kind.p);
+                                                            S.nd_r.p, S.wk_rec.p);
     TG_TRY(launched(S));
-    NodeView V{S.nd_pb.p, S.nd_pe.p, S.nd_child0.p, S.nd_ms.p, S.nd_r.p, S.nd_rmax.p, S.wk_wx.p, S.wk_kind.p};
+    NodeView V{S.nd_pb.p, S.nd_pe.p, S.nd_child0.p, S.nd_ms.p, S.nd_r.p, S.nd_rmax.p, S.wk_rec.p};
 
     for (int k = 0; k < NLIST; k++) {
         TG_TRY(ensure(S.loff[k], nn));
@@ -543,7 +657,7 @@ int tree_walk(Solver &S, cudaStream_t st) {
             int32_t *const ne_out = S.nxt_pool[1].p + out_h * cap_nx[1];
             unsigned long long *const lt = S.nx_top.p + 4 * (size_t)L; /* direct, ewald, drain counter */
             {
-                const int TPB = 128;
+                const int TPB = WK_TPB;
                 const int g = (int)((count * 32 + TPB - 1) / TPB);
                 k_node_stage<<<g, TPB, 0, st>>>(W, V, first, count, (int32_t)nn, S.nd_parent.p, d_pools.p, d_caps.p,
                                                 S.pool_top.p, d_loff.p, d_llen.p, nd_in, ne_in, nd_out, ne_out,
@@ -552,7 +666,7 @@ int tree_walk(Solver &S, cudaStream_t st) {
                 TG_TRY(launched(S));
             }
             if (S.level_leaves[L] > 0) { /* drain this level's leaves while their next lists are live */
-                const int TPB = 128;
+                const int TPB = WK_TPB;
                 const int64_t want = std::min<int64_t>(S.drain_warps, S.level_leaves[L]);
                 const int g = (int)((want * 32 + TPB - 1) / TPB);
                 k_leaf_drain<<<g, TPB, 0, st>>>(W, V, first, count, (int32_t)nn, d_pools.p, d_caps.p, S.pool_top.p,
