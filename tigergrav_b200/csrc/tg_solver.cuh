@@ -86,7 +86,8 @@ struct Solver {
     std::vector<int64_t> level_off;    /* host: first node of each level, size depth+2 */
     std::vector<int64_t> level_leaves; /* host: leaves (childless nodes) of each level, size depth+1 */
     int depth = 0;
-    DevBuf<int32_t> nd_pb, nd_pe, nd_child0, nd_parent, nd_flag, nd_scan;
+    DevBuf<int32_t> nd_pb, nd_pe, nd_child0, nd_parent;
+    DevBuf<long long> tb_out; /* the tree build's level table and status */
     DevBuf<unsigned long long> nd_key;
     DevBuf<unsigned char> nd_level;
     DevBuf<MSrc> nd_ms;
