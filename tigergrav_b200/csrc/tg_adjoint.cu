@@ -105,16 +105,39 @@ __device__ __forceinline__ void sym_mul_add(const T *T6, const T *u, Acc<T> *o) 
     o[2].add(T6[I2(0, 2)] * u[0] + T6[I2(1, 2)] * u[1] + T6[I2(2, 2)] * u[2]);
 }
 
+/* sums of u over tiles of USUM_TILE particles (sorted order), one warp each */
+constexpr int USUM_TILE = 256;
+__global__ void k_tile_usum(int64_t n, const double *__restrict__ u, double *__restrict__ tile) {
+    const int lane = threadIdx.x & 31;
+    const int64_t k = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (k * USUM_TILE >= n) return;
+    double s[3] = {0.0, 0.0, 0.0};
+    const int64_t e = min(n, (k + 1) * USUM_TILE);
+    for (int64_t q = k * USUM_TILE + lane; q < e; q += 32)
+        for (int d = 0; d < 3; d++) s[d] += u[3 * q + d];
+    for (int d = 0; d < 3; d++) {
+        const double v = warp_sum(s[d]);
+        if (lane == 0) tile[3 * k + d] = v;
+    }
+}
 /* U_B = sum over the node's particles of m u_j (the mass-weighted upstream
  * gradient, i.e. M_B times the first-order shift of its centre of mass):
- * one warp per node, u in sorted order */
+ * one warp per node, u in sorted order; whole tiles from their sums (without
+ * them the root's warp walked all particles: 0.68 ms at 64^3) */
 __global__ void k_node_usum(int64_t nn, double m, const int32_t *__restrict__ pb, const int32_t *__restrict__ pe,
-                            const double *__restrict__ u, double *__restrict__ U) {
+                            const double *__restrict__ u, const double *__restrict__ tile, double *__restrict__ U) {
     const int lane = threadIdx.x & 31;
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= nn) return;
     double s[3] = {0.0, 0.0, 0.0};
-    for (int64_t q = pb[i] + lane; q < pe[i]; q += 32)
+    const int64_t b = pb[i], e = pe[i];
+    const int64_t k0 = (b + USUM_TILE - 1) / USUM_TILE, k1 = e / USUM_TILE; /* the whole tiles [k0, k1) */
+    const int64_t b1 = k0 < k1 ? k0 * USUM_TILE : e, e0 = k0 < k1 ? k1 * USUM_TILE : e;
+    for (int64_t q = b + lane; q < b1; q += 32)
+        for (int d = 0; d < 3; d++) s[d] += u[3 * q + d];
+    for (int64_t k = k0 + lane; k < k1; k += 32)
+        for (int d = 0; d < 3; d++) s[d] += tile[3 * k + d];
+    for (int64_t q = e0 + lane; q < e; q += 32)
         for (int d = 0; d < 3; d++) s[d] += u[3 * q + d];
     for (int d = 0; d < 3; d++) {
         const double v = warp_sum(s[d]);
@@ -148,7 +171,7 @@ __global__ void __launch_bounds__(128) k_vfield_node(GParams P, int64_t nn, cons
                 const int32_t src = lcc[j];
                 T dX[3], D[LP];
                 for (int d = 0; d < 3; d++) dX[d] = sep<T>(X[d], ms[src].x[d], ew ? true : per);
-                if (ew) green_ewald_full<T>(E, dX, D);
+                if (ew) green_ewald_any<T>(E, dX, D);
                 else green_direct<T>(dX, D);
                 const double Ub[3] = {U[3 * (int64_t)src], U[3 * (int64_t)src + 1], U[3 * (int64_t)src + 2]};
                 for (int a = 0; a < 3; a++)
@@ -163,7 +186,7 @@ __global__ void __launch_bounds__(128) k_vfield_node(GParams P, int64_t nn, cons
                     const int32_t yy[3] = {y.x, y.y, y.z};
                     T dX[3], D[LP];
                     for (int d = 0; d < 3; d++) dX[d] = sep<T>(X[d], yy[d], ew ? true : per);
-                    if (ew) green_ewald_full<T>(E, dX, D);
+                    if (ew) green_ewald_any<T>(E, dX, D);
                     else green_direct<T>(dX, D);
                     for (int a = 0; a < 3; a++)
                         acc[a] += P.m_d * ((double)D[E2(a, 0)] * us[3 * (int64_t)q] +
@@ -190,8 +213,9 @@ __global__ void k_vfield_down(int64_t first, int64_t count, const int32_t *__res
 }
 
 /* out_i = (J u)_i for the sinks of each leaf; u and out in sorted order
- * (3 doubles per particle).  One block per leaf, one thread per sink. */
-template <class T, int BLOCK>
+ * (3 doubles per particle).  One block per leaf, one thread per sink.  PP: with
+ * the pair lists (leaf_max > 64; else k_tidal_pp and k_tidal_ewald_pp). */
+template <class T, int BLOCK, bool PP>
 __global__ void __launch_bounds__(BLOCK) k_tidal_leaf(GParams P, const int32_t *__restrict__ leaves, int32_t nleaves,
                                                       const int32_t *__restrict__ pb, const int32_t *__restrict__ pe,
                                                       const MSrc *__restrict__ ms, const int4 *__restrict__ pos,
@@ -239,7 +263,7 @@ __global__ void __launch_bounds__(BLOCK) k_tidal_leaf(GParams P, const int32_t *
                 for (int d = 0; d < 3; d++) dX[d] = sep<T>(xi[d], s.x[d], ew ? true : per);
 #pragma unroll
                 for (int q = 0; q < MP; q++) M[q] = T(s.m[q]);
-                if (ew) green_ewald_full<T>(E, dX, D);
+                if (ew) green_ewald_any<T>(E, dX, D);
                 else green_direct<T>(dX, D);
                 M2T<T>(M, D, T6);
                 sym_mul_add<T>(T6, ui, o);
@@ -250,7 +274,7 @@ __global__ void __launch_bounds__(BLOCK) k_tidal_leaf(GParams P, const int32_t *
         }
         /* PP direct and Ewald: pair Hessians times (u_i - u_j) */
         const T m = T(P.m_d);
-        for (int ew = 0; ew < (per ? 2 : 1); ew++) {
+        for (int ew = 0; ew < (!PP ? 0 : (per ? 2 : 1)); ew++) {
             const int kind = ew ? TG_PP_E : TG_PP_D;
             const int32_t *lst = LV.pool[kind] + LV.off[kind][leaf];
             const int32_t len = LV.len[kind][leaf];
@@ -281,7 +305,7 @@ __global__ void __launch_bounds__(BLOCK) k_tidal_leaf(GParams P, const int32_t *
                             T dX[3] = {wrap_sep_t<T>(xi[0], y.x), wrap_sep_t<T>(xi[1], y.y), wrap_sep_t<T>(xi[2], y.z)};
                             if (!(dX[0] * dX[0] + dX[1] * dX[1] + dX[2] * dX[2] > T(1.0e-12))) continue;
                             T D[LP];
-                            green_ewald_full<T>(E, dX, D);
+                            green_ewald_any<T>(E, dX, D);
                             for (int a = 0; a < 3; a++)
                                 o[a].add(-m * (D[E2(a, 0)] * du[0] + D[E2(a, 1)] * du[1] + D[E2(a, 2)] * du[2]));
                         }
@@ -292,6 +316,334 @@ __global__ void __launch_bounds__(BLOCK) k_tidal_leaf(GParams P, const int32_t *
         if (active)
             for (int d = 0; d < 3; d++) out[3 * (int64_t)i + d] = o[d].get();
     }
+}
+
+/*
+ * PP direct: out_i += -sum_j m H(x_i - x_j) (u_i - u_j), H the Hessian of the
+ * softened pair force (pp_pair_deriv).  One block per leaf of at most 64 sinks,
+ * C = 128 / ns copies of them (copy p takes every C-th source of a stage), sums
+ * over 8 pairs folded into the compensated totals, copies added in order.  In
+ * k_tidal_leaf, at the registers of the PC tensors and with every pair folded,
+ * this was 2.2 of 5 ms of a 64^3 Jacobian product.
+ */
+template <class T>
+__global__ void __launch_bounds__(128) k_tidal_pp(GParams P, const int32_t *__restrict__ leaves,
+                                                  const int32_t *__restrict__ pb, const int32_t *__restrict__ pe,
+                                                  const int4 *__restrict__ pos, ListView LV,
+                                                  const double *__restrict__ u, double *__restrict__ out) {
+    __shared__ int4 sy[128];
+    __shared__ T su[128][3];
+    __shared__ double red[128][3];
+    const int t = threadIdx.x;
+    const bool per = P.ewald != 0;
+    const int32_t leaf = leaves[blockIdx.x];
+    const int32_t b = pb[leaf], ns = pe[leaf] - b;
+    if (ns <= 0) return;
+    const int C = 128 / ns, phase = t / ns;
+    const int64_t i = b + t % ns;
+    const int4 xi = pos[i];
+    const T ui[3] = {T(u[3 * i]), T(u[3 * i + 1]), T(u[3 * i + 2])};
+    const T m = T(P.m_d);
+    Acc<T> o[3];
+    for (int d = 0; d < 3; d++) o[d].init(0.0);
+    const int32_t *lst = LV.pool[TG_PP_D] + LV.off[TG_PP_D][leaf];
+    const int32_t len = LV.len[TG_PP_D][leaf];
+    int32_t c = 0, done = 0; /* the next source: leaf c of the list, its particle `done` */
+    for (;;) {
+        /* stage up to 128 particles of consecutive source leaves */
+        int32_t nt = 0;
+        __syncthreads();
+        while (c < len && nt < 128) {
+            const int32_t sb = pb[lst[c]], sn = pe[lst[c]] - sb, k = min(sn - done, 128 - nt);
+            if (t >= nt && t < nt + k) {
+                const int64_t q = sb + done + t - nt;
+                sy[t] = pos[q];
+                for (int d = 0; d < 3; d++) su[t][d] = T(u[3 * q + d]);
+            }
+            nt += k;
+            done += k;
+            if (done == sn) {
+                c++;
+                done = 0;
+            }
+        }
+        if (nt == 0) break;
+        __syncthreads();
+        if (phase >= C) continue;
+        for (int32_t q0 = phase; q0 < nt; q0 += 8 * C) {
+            T s[3] = {T(0), T(0), T(0)};
+            const int32_t q1 = min(nt, q0 + 8 * C);
+            for (int32_t q = q0; q < q1; q += C) {
+                const int4 y = sy[q];
+                const T du[3] = {ui[0] - su[q][0], ui[1] - su[q][1], ui[2] - su[q][2]};
+                const T dX[3] = {sep<T>(xi.x, y.x, per), sep<T>(xi.y, y.y, per), sep<T>(xi.z, y.z, per)};
+                const T r2 = dX[0] * dX[0] + dX[1] * dX[1] + dX[2] * dX[2];
+                T f, fpr;
+                pp_pair_deriv<T>(P, r2, f, fpr);
+                const T w = (dX[0] * du[0] + dX[1] * du[1] + dX[2] * du[2]) * fpr;
+                for (int d = 0; d < 3; d++) s[d] += f * du[d] + dX[d] * w;
+            }
+            for (int d = 0; d < 3; d++) o[d].add(-m * s[d]);
+        }
+    }
+    for (int d = 0; d < 3; d++) red[t][d] = phase < C ? o[d].get() : 0.0;
+    __syncthreads();
+    if (t < ns)
+        for (int d = 0; d < 3; d++) {
+            double v = 0.0;
+            for (int p = 0; p < C; p++) v += red[t + p * ns][d];
+            out[3 * i + d] += v;
+        }
+}
+
+/*
+ * PP Ewald: sum_j m D2(x_i - x_j) (u_i - u_j) with the split of
+ * tg_ewald_sep.cuh.  The reciprocal part of D2 is sum_h 4 pi w_h h h^T
+ * cos(th_i - th_j), so a source leaf gives per h the sums of (cos, sin) th_j and
+ * of (h.u_j)(cos, sin) th_j; the real-space part is the Hessians of the nearest
+ * image and its neighbours towards the near corner.  The whole green_ewald
+ * per pair took 0.9 of a 64^3 Jacobian product (12e6 pairs).
+ */
+template <class T> struct Sep4 {
+    T c, s, uc, us;
+};
+
+template <class T>
+__global__ void __launch_bounds__(128) k_tidal_sf(const int32_t *__restrict__ src, const int32_t *__restrict__ pb,
+                                                  const int32_t *__restrict__ pe, const int4 *__restrict__ pos,
+                                                  const double *__restrict__ u, EwaldTables E, Sep4<T> *__restrict__ sf) {
+    const int32_t node = src[blockIdx.x];
+    const int32_t b = pb[node], e = pe[node];
+    for (int t = threadIdx.x; t < Sep<T>::N; t += 128) {
+        const int4 h = __ldg(&E.sep_h[t]);
+        Sep4<T> a{T(0), T(0), T(0), T(0)};
+        for (int32_t j = b; j < e; j++) {
+            const int4 p = __ldg(&pos[j]);
+            const typename Sep<T>::T2 q = sep_cs<T>(p.x, p.y, p.z, h);
+            const T hu = T(h.x * u[3 * (int64_t)j] + h.y * u[3 * (int64_t)j + 1] + h.z * u[3 * (int64_t)j + 2]);
+            a.c += q.x;
+            a.s += q.y;
+            a.uc = fma(hu, q.x, a.uc);
+            a.us = fma(hu, q.y, a.us);
+        }
+        sf[(int64_t)blockIdx.x * Sep<T>::N + t] = a;
+    }
+}
+
+/* r += (d1 + d2 x x^T) du for one image at displacement x */
+template <class T>
+__device__ __forceinline__ void tidal_image(T x0, T x1, T x2, T r2, const T *du, T *r) {
+    const T alpha = T(Sep<T>::ALPHA);
+    const T rinv = t_rsqrt(r2), r2inv = rinv * rinv, rr = r2 * rinv;
+    T e;
+    const T erfc = t_erfcexp(alpha * rr, &e);
+    const T ce = T(Sep<T>::ALPHA * 1.1283791670955126) * e; /* 2 alpha / sqrt(pi) e^(-alpha^2 r^2) */
+    const T d1 = fma(ce, rr, erfc) * rinv * r2inv;
+    const T d2 = -fma(T(3), d1, T(2) * alpha * alpha * ce) * r2inv;
+    const T s = (x0 * du[0] + x1 * du[1] + x2 * du[2]) * d2;
+    r[0] = fma(x0, s, fma(d1, du[0], r[0]));
+    r[1] = fma(x1, s, fma(d1, du[1], r[1]));
+    r[2] = fma(x2, s, fma(d1, du[2], r[2]));
+}
+
+/* the real-space part of D2(x) du; nothing (with the leaf sums' reciprocal part
+ * taken back) for r <= 1e-6 */
+template <class T>
+__device__ __forceinline__ void tidal_ewald_pair(const EwaldTables &E, const T *x, const T *du, T *r) {
+    r[0] = r[1] = r[2] = T(0);
+    const T r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+    if (!(r2 > T(1.0e-12))) {
+        for (int d = 0; d < 3; d++) r[d] = -T(E.sep_r2) * du[d];
+        return;
+    }
+    T a[3], b[3], u[3], v[3], w[3], q[3] = {T(0), T(0), T(0)};
+#pragma unroll
+    for (int d = 0; d < 3; d++) { /* in the octant of |x| */
+        a[d] = fabs(x[d]);
+        b[d] = a[d] - T(1);
+        u[d] = a[d] * a[d];
+        v[d] = b[d] * b[d];
+        w[d] = copysign(T(1), x[d]) * du[d];
+    }
+#pragma unroll
+    for (int k = 1; k < 8; k++) {
+        const T s = (k & 1 ? v[0] : u[0]) + (k & 2 ? v[1] : u[1]) + (k & 4 ? v[2] : u[2]);
+        if (s < T(1)) tidal_image<T>(k & 1 ? b[0] : a[0], k & 2 ? b[1] : a[1], k & 4 ? b[2] : a[2], s, w, q);
+    }
+    /* nearest image with the direct 1/r removed: d1 = -f0, d2 = (3 f0 - 2 alpha^2 c e) / r^2, or the
+     * derivative of f0's series (ewald_nearest) for alpha r < 1/2, where the two cancel */
+    const T alpha = T(Sep<T>::ALPHA);
+    const T rinv = t_rsqrt(r2), rr = r2 * rinv, y = alpha * alpha * r2;
+    T p0, f0, d2;
+    ewald_nearest<T>(alpha, rr, rinv, p0, f0);
+    if (y < T(0.25)) {
+        T s = T(0);
+        if constexpr (sizeof(T) == 8) {
+            s = T(10.0 / 41731200.0);
+            s = fma(s, y, T(-9.0 / 3810240.0));
+            s = fma(s, y, T(8.0 / 383040.0));
+        }
+        s = fma(s, y, T(-7.0 / 42840.0));
+        s = fma(s, y, T(6.0 / 5400.0));
+        s = fma(s, y, T(-5.0 / 780.0));
+        s = fma(s, y, T(4.0 / 132.0));
+        s = fma(s, y, T(-3.0 / 27.0));
+        s = fma(s, y, T(2.0 / 7.0));
+        s = fma(s, y, T(-0.4));
+        d2 = T(-2.0 * 1.1283791670955126) * (alpha * alpha * alpha * alpha * alpha) * s;
+    } else {
+        const T ce = T(Sep<T>::ALPHA * 1.1283791670955126) * exp(-y);
+        d2 = (T(3) * f0 - T(2) * alpha * alpha * ce) * rinv * rinv;
+    }
+    const T s = (a[0] * w[0] + a[1] * w[1] + a[2] * w[2]) * d2;
+#pragma unroll
+    for (int d = 0; d < 3; d++) r[d] = copysign(T(1), x[d]) * (q[d] + a[d] * s - f0 * w[d]);
+}
+
+/* one chunk of a PP_E list (as k_ewald_pp): the real-space part per pair into
+ * part (3 per sink), the reciprocal source sums into tpart */
+template <class T>
+__global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, const int32_t *__restrict__ leaves, int32_t nleaves,
+                                                       const int32_t *__restrict__ off, const int32_t *__restrict__ pb,
+                                                       const int32_t *__restrict__ pe, const int4 *__restrict__ pos,
+                                                       ListView LV, EwaldTables E, const double *__restrict__ u,
+                                                       double *__restrict__ part, const int32_t *__restrict__ slot,
+                                                       const Sep4<T> *__restrict__ sf, Sep4<T> *__restrict__ tpart) {
+    __shared__ int4 sy[64];
+    __shared__ T su[64][3];
+    __shared__ int32_t s_row[EW_KPP_MAX];
+    const int tid = threadIdx.x;
+    const int64_t c = blockIdx.x;
+    const int32_t li = ew_leaf(off, nleaves, c), k = (int32_t)(c - off[li]);
+    const int32_t leaf = leaves[li];
+    const int32_t b = pb[leaf], cnt = pe[leaf] - b;
+    const int64_t i = b + (tid < cnt ? tid : 0);
+    const int4 xi = pos[i];
+    const T ui[3] = {T(u[3 * i]), T(u[3 * i + 1]), T(u[3 * i + 2])};
+    Acc<T> o[3];
+    for (int d = 0; d < 3; d++) o[d].init(0.0);
+    const int32_t *lst = LV.pool[TG_PP_E] + LV.off[TG_PP_E][leaf];
+    const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len), e0 = k * kpp, e1 = min(len, e0 + kpp);
+    const T m = T(P.m_d);
+    if (tid < e1 - e0) s_row[tid] = slot[lst[e0 + tid]];
+    for (int32_t e = e0; e < e1; e++) {
+        const int32_t src = lst[e];
+        const int32_t sb = pb[src], sn = pe[src] - sb; /* leaf_max <= 64: one stage */
+        __syncthreads();
+        if (tid < sn) {
+            const int64_t q = sb + tid;
+            sy[tid] = pos[q];
+            for (int d = 0; d < 3; d++) su[tid][d] = T(u[3 * q + d]);
+        }
+        __syncthreads();
+        if (tid < ((cnt + 31) & ~31))
+            for (int32_t q = 0; q < sn; q++) {
+                const int4 y = sy[q];
+                const T dX[3] = {wrap_sep_t<T>(xi.x, y.x), wrap_sep_t<T>(xi.y, y.y), wrap_sep_t<T>(xi.z, y.z)};
+                const T du[3] = {ui[0] - su[q][0], ui[1] - su[q][1], ui[2] - su[q][2]};
+                T r[3];
+                tidal_ewald_pair<T>(E, dX, du, r);
+                for (int d = 0; d < 3; d++) o[d].add(-m * r[d]);
+            }
+    }
+    if (tid < cnt)
+        for (int d = 0; d < 3; d++) part[3 * (c * 64 + tid) + d] = o[d].get();
+    for (int t = tid; t < Sep<T>::N; t += 64) {
+        Sep4<T> a{T(0), T(0), T(0), T(0)};
+#pragma unroll 4
+        for (int q = 0; q < e1 - e0; q++) {
+            const Sep4<T> f = sf[(int64_t)s_row[q] * Sep<T>::N + t];
+            a.c = fma(m, f.c, a.c);
+            a.s = fma(m, f.s, a.s);
+            a.uc = fma(m, f.uc, a.uc);
+            a.us = fma(m, f.us, a.us);
+        }
+        tpart[c * Sep<T>::N + t] = a;
+    }
+}
+
+/* out += the chunk sums of each leaf, in chunk order, and the reciprocal part
+ * -sum_h 4 pi w_h h ((h.u_i) cos(th_i - th_j) - (h.u_j) cos(th_i - th_j)) from
+ * the chunks' source sums.  One block per leaf, four threads per sink. */
+template <class T>
+__global__ void __launch_bounds__(256) k_tidal_ewald_reduce(const int32_t *__restrict__ leaves,
+                                                            const int32_t *__restrict__ off,
+                                                            const int32_t *__restrict__ pb, const int32_t *__restrict__ pe,
+                                                            const int4 *__restrict__ pos, EwaldTables E,
+                                                            const double *__restrict__ u, const double *__restrict__ part,
+                                                            const Sep4<T> *__restrict__ tpart, double *__restrict__ out) {
+    constexpr int TILE = 384; /* vectors whose sums are held at a time */
+    __shared__ double4 sT[TILE];
+    __shared__ double sv[4][64][3];
+    const int32_t li = blockIdx.x;
+    const int tid = threadIdx.x, t = tid & 63, grp = tid >> 6;
+    const int32_t a0 = off[li], a1 = off[li + 1];
+    if (a1 == a0) return; /* block-uniform */
+    const int32_t leaf = leaves[li];
+    const int32_t b = pb[leaf], cnt = pe[leaf] - b;
+    const int64_t i = b + (t < cnt ? t : 0);
+    const int4 p = pos[i];
+    const double ui[3] = {u[3 * i], u[3 * i + 1], u[3 * i + 2]};
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int t0 = 0; t0 < Sep<T>::N; t0 += TILE) {
+        const int nt = min(TILE, Sep<T>::N - t0);
+        __syncthreads();
+        for (int q = tid; q < nt; q += 256) {
+            double4 s = make_double4(0.0, 0.0, 0.0, 0.0);
+            for (int64_t c = a0; c < a1; c++) {
+                const Sep4<T> f = tpart[c * Sep<T>::N + t0 + q];
+                s.x += (double)f.c;
+                s.y += (double)f.s;
+                s.z += (double)f.uc;
+                s.w += (double)f.us;
+            }
+            sT[q] = s;
+        }
+        __syncthreads();
+        if (t < cnt)
+            for (int q = grp; q < nt; q += 4) {
+                const int4 h = __ldg(&E.sep_h[t0 + q]);
+                const typename Sep<T>::T2 cs = sep_cs<T>(p.x, p.y, p.z, h);
+                const double4 s = sT[q];
+                const double hu = h.x * ui[0] + h.y * ui[1] + h.z * ui[2];
+                const double C = cs.x, Sn = cs.y;
+                const double f = __ldg(&E.sep_w[t0 + q]) * (hu * (C * s.x + Sn * s.y) - (C * s.z + Sn * s.w));
+                v[0] += f * h.x;
+                v[1] += f * h.y;
+                v[2] += f * h.z;
+            }
+    }
+    for (int d = 0; d < 3; d++) sv[grp][t][d] = v[d];
+    __syncthreads();
+    if (t >= cnt || grp != 0) return;
+    for (int d = 0; d < 3; d++) {
+        double w = 0.0;
+        for (int64_t c = a0; c < a1; c++) w += part[3 * (c * 64 + t) + d];
+        const double rec = (sv[0][t][d] + sv[1][t][d]) + (sv[2][t][d] + sv[3][t][d]);
+        out[3 * i + d] += w - 12.566370614359172 * rec; /* 4 pi */
+    }
+}
+
+/* the PP_E lists' part of J u, added to tid_o (leaf_max <= 64) */
+template <class T>
+static int tidal_ewald(Solver &S, const GParams &P, const ListView &LV, const EwaldTables &E, cudaStream_t st) {
+    const int32_t nleaves = (int32_t)S.st.leaves;
+    int32_t npp = 0, total = 0, nsrc = 0;
+    TG_TRY(leaf_chunks(S, LV, npp, total, nsrc, st));
+    if (npp <= 0) return TG_OK;
+    TG_TRY(ensure(S.ew_part, (size_t)npp * 64 * 3));
+    TG_TRY(ensure(S.ew_sf, (size_t)nsrc * Sep<T>::N * sizeof(Sep4<T>)));
+    TG_TRY(ensure(S.ew_tpart, (size_t)npp * Sep<T>::N * sizeof(Sep4<T>)));
+    Sep4<T> *sf = reinterpret_cast<Sep4<T> *>(S.ew_sf.p), *tpart = reinterpret_cast<Sep4<T> *>(S.ew_tpart.p);
+    k_tidal_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, S.tid_u.p, E, sf);
+    TG_TRY(launched(S));
+    k_tidal_ewald_pp<T><<<npp, 64, 0, st>>>(P, S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, E,
+                                            S.tid_u.p, S.ew_part.p, S.ew_slot.p, sf, tpart);
+    TG_TRY(launched(S));
+    k_tidal_ewald_reduce<T><<<nleaves, 256, 0, st>>>(S.idx.p, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E, S.tid_u.p,
+                                                    S.ew_part.p, tpart, S.tid_o.p);
+    TG_TRY(launched(S));
+    return TG_OK;
 }
 
 /* u_sorted[i] = u[caller index of i] */
@@ -319,6 +671,27 @@ __global__ void k_axpy3(int64_t n, double c, const double *__restrict__ x, doubl
     y[i] += c * x[i];
 }
 
+/* the buffers and kernels of tidal_apply, taken ahead of the first backward pass */
+int tidal_reserve(Solver &S) {
+    TG_TRY(ensure(S.adj_x, 3 * S.n));
+    TG_TRY(ensure(S.adj_v, 3 * S.n));
+    TG_TRY(ensure(S.tid_u, 3 * S.n));
+    TG_TRY(ensure(S.tid_o, 3 * S.n));
+    TG_TRY(ensure(S.tid_U, 3 * S.nnodes));
+    TG_TRY(ensure(S.tid_V, 6 * S.nnodes));
+    TG_TRY(ensure(S.tid_tile, 3 * ((S.n + USUM_TILE - 1) / USUM_TILE)));
+    const bool f64 = S.prm.precision == TG_PREC_F64;
+    const void *k[] = {f64 ? (const void *)k_vfield_node<double> : (const void *)k_vfield_node<float>,
+                       f64 ? (const void *)k_tidal_leaf<double, 64, false> : (const void *)k_tidal_leaf<float, 64, false>,
+                       f64 ? (const void *)k_tidal_pp<double> : (const void *)k_tidal_pp<float>,
+                       f64 ? (const void *)k_tidal_sf<double> : (const void *)k_tidal_sf<float>,
+                       f64 ? (const void *)k_tidal_ewald_pp<double> : (const void *)k_tidal_ewald_pp<float>,
+                       f64 ? (const void *)k_tidal_ewald_reduce<double> : (const void *)k_tidal_ewald_reduce<float>};
+    cudaFuncAttributes a;
+    for (const void *f : k) TG_CUDA(cudaFuncGetAttributes(&a, f)); /* loads the kernel's code */
+    return TG_OK;
+}
+
 /* acc += c J u (u, acc: n x 3 doubles in caller order, device) for the
  * particles and lists currently in S; runs the node stage for the local
  * expansions first */
@@ -340,7 +713,11 @@ int tidal_apply(Solver &S, const double *u, double *acc, double c, cudaStream_t 
     TG_TRY(launched(S));
     const bool f64n = S.prm.precision == TG_PREC_F64;
     const int gw = (int)((nn * 32 + 127) / 128);
-    k_node_usum<<<gw, 128, 0, st>>>(nn, S.prm.m, S.nd_pb.p, S.nd_pe.p, S.tid_u.p, S.tid_U.p);
+    const int64_t ntile = (n + USUM_TILE - 1) / USUM_TILE;
+    TG_TRY(ensure(S.tid_tile, 3 * ntile));
+    k_tile_usum<<<(int)((ntile * 32 + 127) / 128), 128, 0, st>>>(n, S.tid_u.p, S.tid_tile.p);
+    TG_TRY(launched(S));
+    k_node_usum<<<gw, 128, 0, st>>>(nn, S.prm.m, S.nd_pb.p, S.nd_pe.p, S.tid_u.p, S.tid_tile.p, S.tid_U.p);
     TG_TRY(launched(S));
     double *V = S.tid_V.p, *Vtot = S.tid_V.p + 3 * nn;
     if (f64n)
@@ -361,22 +738,33 @@ int tidal_apply(Solver &S, const double *u, double *acc, double c, cudaStream_t 
         const bool f64 = S.prm.precision == TG_PREC_F64;
         if (S.prm.leaf_max <= 64) {
             if (f64)
-                k_tidal_leaf<double, 64><<<nleaves, 64, 0, st>>>(P, S.idx.p, nleaves, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p,
+                k_tidal_leaf<double, 64, false><<<nleaves, 64, 0, st>>>(P, S.idx.p, nleaves, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p,
                                                                  S.pos.p, LV, E, S.nd_L.p, S.tid_U.p, Vtot, S.tid_u.p, S.tid_o.p);
             else
-                k_tidal_leaf<float, 64><<<nleaves, 64, 0, st>>>(P, S.idx.p, nleaves, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p,
+                k_tidal_leaf<float, 64, false><<<nleaves, 64, 0, st>>>(P, S.idx.p, nleaves, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p,
                                                                 S.pos.p, LV, E, S.nd_L.p, S.tid_U.p, Vtot, S.tid_u.p, S.tid_o.p);
         } else {
             if (f64)
-                k_tidal_leaf<double, 128><<<nleaves, 128, 0, st>>>(P, S.idx.p, nleaves, S.nd_pb.p, S.nd_pe.p,
+                k_tidal_leaf<double, 128, true><<<nleaves, 128, 0, st>>>(P, S.idx.p, nleaves, S.nd_pb.p, S.nd_pe.p,
                                                                    S.nd_ms.p, S.pos.p, LV, E, S.nd_L.p, S.tid_U.p,
                                                                    Vtot, S.tid_u.p, S.tid_o.p);
             else
-                k_tidal_leaf<float, 128><<<nleaves, 128, 0, st>>>(P, S.idx.p, nleaves, S.nd_pb.p, S.nd_pe.p,
+                k_tidal_leaf<float, 128, true><<<nleaves, 128, 0, st>>>(P, S.idx.p, nleaves, S.nd_pb.p, S.nd_pe.p,
                                                                   S.nd_ms.p, S.pos.p, LV, E, S.nd_L.p, S.tid_U.p,
                                                                   Vtot, S.tid_u.p, S.tid_o.p);
         }
         TG_TRY(launched(S));
+        if (S.prm.leaf_max <= 64) {
+            if (f64)
+                k_tidal_pp<double><<<nleaves, 128, 0, st>>>(P, S.idx.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, S.tid_u.p,
+                                                            S.tid_o.p);
+            else
+                k_tidal_pp<float><<<nleaves, 128, 0, st>>>(P, S.idx.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, S.tid_u.p,
+                                                           S.tid_o.p);
+            TG_TRY(launched(S));
+        }
+        if (S.prm.ewald && S.prm.leaf_max <= 64)
+            TG_TRY(f64 ? tidal_ewald<double>(S, P, LV, E, st) : tidal_ewald<float>(S, P, LV, E, st));
     }
     k_scatter_axpy3<<<gn, 256, 0, st>>>(n, S.pos.p, c, S.tid_o.p, acc);
     TG_TRY(launched(S));

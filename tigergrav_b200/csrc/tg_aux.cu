@@ -134,26 +134,29 @@ int ewald_tables(Solver &S, cudaStream_t st) {
     std::vector<int4> sh;
     std::vector<double> sw;
     double r0 = 0.0, r2 = 0.0;
-    const auto rec = lattice(30);
+    const bool f64 = S.prm.precision == TG_PREC_F64;
+    const double alpha = f64 ? Sep<double>::ALPHA : Sep<float>::ALPHA;
+    const size_t nsep = f64 ? Sep<double>::N : Sep<float>::N;
+    const auto rec = lattice(f64 ? Sep<double>::H2MAX : Sep<float>::H2MAX);
     for (auto v = rec.rbegin(); v != rec.rend(); ++v) {
         const int lead = (*v)[0] != 0 ? (*v)[0] : ((*v)[1] != 0 ? (*v)[1] : (*v)[2]);
         if (lead <= 0) continue;
         const double pi = 3.141592653589793;
         const double h2 = (double)((*v)[0] * (*v)[0] + (*v)[1] * (*v)[1] + (*v)[2] * (*v)[2]);
-        const double w = 2.0 * std::exp(-pi * pi * h2 / (SEP_ALPHA_D * SEP_ALPHA_D)) / h2;
+        const double w = 2.0 * std::exp(-pi * pi * h2 / (alpha * alpha)) / h2;
         sh.push_back(make_int4((*v)[0], (*v)[1], (*v)[2], 0));
         sw.push_back(w);
         r0 -= w / pi;
         r2 += 4.0 * pi / 3.0 * w * h2;
     }
-    if ((int)sh.size() != NSEP) return TG_ERR_STATE;
-    S.ew_sep_k = (float)(3.141592653589793 / (SEP_ALPHA_D * SEP_ALPHA_D));
-    S.ew_sep_r0 = (float)r0;
-    S.ew_sep_r2 = (float)r2;
-    TG_TRY(ensure(S.ew_sep_h, NSEP));
-    TG_TRY(ensure(S.ew_sep_w, NSEP));
-    TG_CUDA(cudaMemcpyAsync(S.ew_sep_h.p, sh.data(), sizeof(int4) * NSEP, cudaMemcpyHostToDevice, st));
-    TG_CUDA(cudaMemcpyAsync(S.ew_sep_w.p, sw.data(), sizeof(double) * NSEP, cudaMemcpyHostToDevice, st));
+    if (sh.size() != nsep) return TG_ERR_STATE;
+    S.ew_sep_k = 3.141592653589793 / (alpha * alpha);
+    S.ew_sep_r0 = r0;
+    S.ew_sep_r2 = r2;
+    TG_TRY(ensure(S.ew_sep_h, nsep));
+    TG_TRY(ensure(S.ew_sep_w, nsep));
+    TG_CUDA(cudaMemcpyAsync(S.ew_sep_h.p, sh.data(), sizeof(int4) * nsep, cudaMemcpyHostToDevice, st));
+    TG_CUDA(cudaMemcpyAsync(S.ew_sep_w.p, sw.data(), sizeof(double) * nsep, cudaMemcpyHostToDevice, st));
     if (S.ew_use_tab && !S.ew_tab) TG_TRY(ewald_table_acquire(S.dev, S.ew_real.p, S.ew_four.p, &S.ew_tab, st));
     TG_CUDA(cudaStreamSynchronize(st)); /* host vectors go out of scope */
     S.have_tables = true;

@@ -342,7 +342,7 @@ int tg_destroy(tg_solver *s) {
     release(S.ew_cnt); release(S.ew_off); release(S.ew_part); release(S.ew_sf); release(S.ew_sep_h);
     release(S.ew_sep_w); release(S.ew_slot); release(S.ew_src); release(S.ew_tpart);
     release(S.ck_x); release(S.ck_v); release(S.adj_x); release(S.adj_v); release(S.tid_u); release(S.tid_o);
-    release(S.tid_U); release(S.tid_V);
+    release(S.tid_U); release(S.tid_V); release(S.tid_tile);
     release(S.fof_P); release(S.fof_leaves); release(S.fof_key); release(S.fof_mem); release(S.fof_runs);
     release(S.fof_gmin); release(S.fof_group); release(S.fof_has); release(S.fof_pairs); release(S.fof_radii);
     release(S.fof_stats);
@@ -564,6 +564,7 @@ int tg_forward(tg_solver *s, double dt, int n_steps, void *stream) {
     TG_TRY(ensure(S.ck_v, (size_t)3 * n * (n_steps + 1)));
     S.ck_steps = -1;
     if (!S.have_forces) TG_TRY(tg_solve_gravity(s, stream));
+    TG_TRY(tidal_reserve(S));
     const int gn = (int)((n + 255) / 256);
     k_unpack<<<gn, 256, 0, st>>>(n, S.pos.p, S.vel.p, S.ck_x.p, S.ck_v.p);
     TG_TRY(launched(S));

@@ -24,11 +24,23 @@ constexpr int NREAL = 305;  /* |n|^2 <= 17 (tigergrav/green.hpp:3,8-28) */
 constexpr int NREAL_F32 = 123; /* |n|^2 <= 9: every n that can lie within the FP32 cut 2.1 of |X| <= sqrt(3)/2 */
 constexpr int NFOUR = 123;  /* |h|^2 <= 9 */
 constexpr int NFOUR_HALF = 61; /* one of each pair +-h (h != 0) */
-constexpr int NSEP = 369;      /* 0 < |h|^2 <= 30, one of each pair +-h */
-constexpr double SEP_ALPHA_D = 4.2; /* the split alpha of the FP32 path's PP Ewald (tg_ewald_sep.cuh) */
 constexpr int HS = 36;         /* row stride of the coefficient tables (16-byte rows) */
 constexpr float EWALD_RCUT = 1.0e-6f;
 constexpr float EWALD_PHI0 = 2.8372975f; /* r -> 0 limit (tigergrav/green.hpp:272) */
+
+/* The split of the PP Ewald sums (tg_ewald_sep.cuh): alpha, the largest |h|^2 of
+ * the reciprocal vectors, and their number (one of each pair +-h) */
+template <class T> struct Sep;
+template <> struct Sep<float> {
+    static constexpr double ALPHA = 4.2;
+    static constexpr int H2MAX = 30, N = 369;
+    typedef float2 T2;
+};
+template <> struct Sep<double> {
+    static constexpr double ALPHA = 5.2;
+    static constexpr int H2MAX = 70, N = 1258;
+    typedef double2 T2;
+};
 
 /* ---- symmetric index arithmetic (constant-folded after unrolling) ---- */
 __host__ __device__ constexpr int cmin(int a, int b) { return a < b ? a : b; }
@@ -254,9 +266,9 @@ struct EwaldTables {
     const double *Hd;   /* NFOUR_HALF rows of HS, double */
     const float4 *Pf;   /* NFOUR_HALF x (H0, Hx, Hy, Hz): the potential and force terms, float */
     const double2 *Pd;  /* NFOUR_HALF x 2, double */
-    const int4 *sep_h;  /* NSEP reciprocal vectors of the PP Ewald split (tg_ewald_sep.cuh) */
+    const int4 *sep_h;  /* reciprocal vectors of the PP Ewald split (tg_ewald_sep.cuh; Sep<T>::N of them) */
     const double *sep_w; /* their weights 2 exp(-pi^2 h^2 / alpha^2) / h^2 */
-    float sep_k, sep_r0, sep_r2; /* pi / alpha^2; the reciprocal part near r = 0: phi = r0, g = -r2 x */
+    double sep_k, sep_r0, sep_r2; /* pi / alpha^2; the reciprocal part near r = 0: phi = r0, g = -r2 x */
     const float *tab;   /* local expansions of green_ewald (tg_ewald_table.cuh); solvers of the FP32 path only */
 };
 

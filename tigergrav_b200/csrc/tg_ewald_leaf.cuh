@@ -8,7 +8,7 @@
  * at theta = 0.2 on a clustered box 1% of the leaves hold half the PP_Ewald
  * pairs (up to 9e6 for one leaf); and a box of a few thousand particles has
  * fewer leaves than the GPU has SMs, each with every other leaf in its list.
- * So each leaf's PP_E list is cut into chunks of EW_KPP source leaves and its
+ * So each leaf's PP_E list is cut into chunks of ew_kpp source leaves and its
  * PC_E list into chunks of EW_KPC source nodes; one 64-thread block (a thread
  * per sink) evaluates one chunk and writes its sinks' partial sums to its own
  * slot of a scratch array; k_ewald_reduce then adds a leaf's chunk sums in
@@ -19,7 +19,14 @@
  */
 #pragma once
 
-constexpr int EW_KPP = 8;  /* PP_E source leaves per chunk (<= 8 * 64 * 64 pairs) */
+constexpr int EW_KPP_MAX = 32;
+/* PP_E source leaves per chunk: 16 chunks of a list, of 8 to 32 leaves (at most
+ * 32 * 64 * 64 pairs).  Each chunk's slots take 5 KB in FP32, so chunks of 8
+ * throughout hold 225 MB for 32768 particles where these hold 60 MB. */
+__host__ __device__ __forceinline__ int32_t ew_kpp(int32_t len) {
+    const int32_t k = (len + 15) >> 4;
+    return k < 8 ? 8 : (k > EW_KPP_MAX ? EW_KPP_MAX : k);
+}
 constexpr int EW_KPC = 64; /* PC_E source nodes per chunk */
 
 /* one warp per leaf: chunk counts (zeros at li = nleaves, so that the scan ends
@@ -39,7 +46,7 @@ __global__ void k_ewald_count(const int32_t *__restrict__ leaves, int32_t nleave
         }
     }
     if (lane == 0) {
-        cnt[li] = (npp + EW_KPP - 1) / EW_KPP;
+        cnt[li] = (npp + ew_kpp(npp) - 1) / ew_kpp(npp);
         cnt[nleaves + 1 + li] = (npc + EW_KPC - 1) / EW_KPC;
     }
 }
@@ -73,15 +80,17 @@ __device__ __forceinline__ int32_t ew_leaf(const int32_t *__restrict__ off, int3
     return lo;
 }
 
-/* one chunk of a PP_E list: entries [k EW_KPP, ...) of its leaf.  FP32: the
+/* one chunk of a PP_E list: entries [k ew_kpp, ...) of its leaf.  The
  * real-space part per pair and the chunk's reciprocal source sums (tpart). */
 template <class T>
 __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
     k_ewald_pp(GParams P, const int32_t *__restrict__ leaves, int32_t nleaves, const int32_t *__restrict__ off,
                const int32_t *__restrict__ pb, const int32_t *__restrict__ pe, const int4 *__restrict__ pos, ListView LV,
                EwaldTables E, double *__restrict__ part, const int32_t *__restrict__ slot,
-               const float2 *__restrict__ sf, float2 *__restrict__ tpart) {
+               const typename Sep<T>::T2 *__restrict__ sf, typename Sep<T>::T2 *__restrict__ tpart) {
+    typedef typename Sep<T>::T2 T2;
     __shared__ int4 sy[64];
+    __shared__ int32_t s_row[EW_KPP_MAX];
     const int tid = threadIdx.x;
     const int64_t c = blockIdx.x;
     const int32_t li = ew_leaf(off, nleaves, c), k = (int32_t)(c - off[li]);
@@ -93,8 +102,9 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
     aphi.init(0.0);
     for (int d = 0; d < 3; d++) ag[d].init(0.0);
     const int32_t *lst = LV.pool[TG_PP_E] + LV.off[TG_PP_E][leaf];
-    const int32_t e0 = k * EW_KPP, e1 = min(LV.len[TG_PP_E][leaf], e0 + EW_KPP);
+    const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len), e0 = k * kpp, e1 = min(len, e0 + kpp);
     const T m = T(P.m_d);
+    if (tid < e1 - e0) s_row[tid] = slot[lst[e0 + tid]];
     for (int32_t e = e0; e < e1; e++) {
         const int32_t src = lst[e];
         const int32_t sb = pb[src], sn = pe[src] - sb; /* leaf_max <= 64: one stage */
@@ -106,8 +116,7 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
                 const int4 y = sy[q];
                 const T dX[3] = {wrap_sep_t<T>(xi.x, y.x), wrap_sep_t<T>(xi.y, y.y), wrap_sep_t<T>(xi.z, y.z)};
                 T ph, g[3];
-                if constexpr (sizeof(T) == 4) pp_ewald_pair_sep(E, dX, ph, g);
-                else pp_ewald_pair<T>(E, dX, ph, g);
+                pp_ewald_pair_sep<T>(E, dX, ph, g);
                 aphi.add(m * ph);
                 for (int d = 0; d < 3; d++) ag[d].add(m * g[d]);
             }
@@ -117,22 +126,17 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
         o[0] = aphi.get();
         for (int d = 0; d < 3; d++) o[1 + d] = ag[d].get();
     }
-    if constexpr (sizeof(T) == 4) {
-        /* this chunk's reciprocal source sums, a thread per vector */
-        int32_t row[EW_KPP];
-#pragma unroll
-        for (int u = 0; u < EW_KPP; u++) row[u] = e0 + u < e1 ? slot[lst[e0 + u]] : -1;
-        for (int t = tid; t < NSEP; t += 64) {
-            float2 a = make_float2(0.0f, 0.0f);
-#pragma unroll
-            for (int u = 0; u < EW_KPP; u++)
-                if (row[u] >= 0) {
-                    const float2 f = sf[(int64_t)row[u] * NSEP + t];
-                    a.x = fmaf(m, f.x, a.x);
-                    a.y = fmaf(m, f.y, a.y);
-                }
-            tpart[c * NSEP + t] = a;
+    /* this chunk's reciprocal source sums, a thread per vector (s_row: written before the loop's barriers) */
+    for (int t = tid; t < Sep<T>::N; t += 64) {
+        T2 a;
+        a.x = a.y = T(0);
+#pragma unroll 8
+        for (int u = 0; u < e1 - e0; u++) {
+            const T2 f = sf[(int64_t)s_row[u] * Sep<T>::N + t];
+            a.x = fma(m, f.x, a.x);
+            a.y = fma(m, f.y, a.y);
         }
+        tpart[c * Sep<T>::N + t] = a;
     }
 }
 
@@ -173,16 +177,18 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 8 : 6)
     for (int d = 0; d < 3; d++) o[1 + d] = ag[d].get();
 }
 
-/* Add each leaf's chunk sums, in chunk order, to its FP64 accumulators; with
- * tpart, also the reciprocal part from the PP_E chunks' source sums (in chunk
+/* Add each leaf's chunk sums, in chunk order, to its FP64 accumulators, and
+ * the reciprocal part from the PP_E chunks' source sums (in chunk
  * order).  One block per leaf; the four groups of 64 threads take a quarter
  * of the vectors each. */
+template <class T>
 __global__ void __launch_bounds__(256) k_ewald_reduce(const int32_t *__restrict__ leaves, int32_t nleaves,
                                                       const int32_t *__restrict__ off, const int32_t *__restrict__ pb,
                                                       const int32_t *__restrict__ pe, const double *__restrict__ part,
-                                                      double *__restrict__ acc, const float2 *__restrict__ tpart,
+                                                      double *__restrict__ acc,
+                                                      const typename Sep<T>::T2 *__restrict__ tpart,
                                                       const int4 *__restrict__ pos, EwaldTables E) {
-    __shared__ double2 sT[NSEP];
+    __shared__ double2 sT[Sep<T>::N];
     __shared__ double sv[4][64][4];
     const int32_t li = blockIdx.x;
     const int tid = threadIdx.x, t = tid & 63, grp = tid >> 6;
@@ -192,18 +198,18 @@ __global__ void __launch_bounds__(256) k_ewald_reduce(const int32_t *__restrict_
     const int32_t leaf = leaves[li];
     const int32_t b = pb[leaf], cnt = pe[leaf] - b;
     double v[4] = {0.0, 0.0, 0.0, 0.0};
-    if (tpart && a1 > a0) { /* block-uniform */
-        for (int i = tid; i < NSEP; i += 256) {
+    if (a1 > a0) { /* block-uniform */
+        for (int i = tid; i < Sep<T>::N; i += 256) {
             double sx = 0.0, sy = 0.0;
             for (int64_t c = a0; c < a1; c++) {
-                const float2 f = tpart[c * NSEP + i];
+                const typename Sep<T>::T2 f = tpart[c * Sep<T>::N + i];
                 sx += (double)f.x;
                 sy += (double)f.y;
             }
             sT[i] = make_double2(sx, sy);
         }
         __syncthreads();
-        if (t < cnt) sep_eval(E, sT, grp, 4, pos[b + t], v[0], v + 1);
+        if (t < cnt) sep_eval<T>(E, sT, grp, 4, pos[b + t], v[0], v + 1);
     }
 #pragma unroll
     for (int q = 0; q < 4; q++) sv[grp][t][q] = v[q];

@@ -20,7 +20,9 @@ constexpr int EN_KCP = 4;   /* CP_E source leaves per chunk */
 #ifndef EN_MINB
 #define EN_MINB 3 /* resident 128-thread blocks per SM the FP32 kernel is compiled for */
 #endif
-#define EN_MINB_D 6
+#ifndef EN_MINB_D
+#define EN_MINB_D 2 /* and the FP64 kernel */
+#endif
 
 __global__ void k_node_ewald_count(int64_t nn, const int32_t *__restrict__ pb, const int32_t *__restrict__ pe,
                                    ListView LV, int32_t *__restrict__ cnt) {

@@ -129,7 +129,13 @@ __device__ __forceinline__ void ewald_nearest(T alpha, T r, T rinv, T &p0, T &f0
     p0 = erfx * rinv;
     if (x < T(0.5)) {
         const T y = x * x;
-        T s = T(-1.0 / 42840.0);
+        T s = T(0);
+        if constexpr (sizeof(T) == 8) { /* FP32 ends at y^7 */
+            s = T(1.0 / 41731200.0);
+            s = fma(s, y, T(-1.0 / 3810240.0));
+            s = fma(s, y, T(1.0 / 383040.0));
+        }
+        s = fma(s, y, T(-1.0 / 42840.0));
         s = fma(s, y, T(1.0 / 5400.0));
         s = fma(s, y, T(-1.0 / 780.0));
         s = fma(s, y, T(1.0 / 132.0));
@@ -677,30 +683,25 @@ static int node_ewald(Solver &S, const GParams &P, const ListView &LV, const Ewa
     return TG_OK;
 }
 
-/* the leaf Ewald lists (PP_E, PC_E) of every leaf, in balanced chunks, added
- * to the FP64 accumulators accd (leaf_max <= 64) */
-static int leaf_ewald(Solver &S, const GParams &P, const ListView &LV, const EwaldTables &E, bool f64,
-                      cudaStream_t st) {
+/* The leaf Ewald lists cut into chunks (tg_ewald_leaf.cuh): their offsets in
+ * ew_off, the PP_E source leaves in ew_src with their rows in ew_slot, and the
+ * numbers of PP_E chunks, of all chunks and of source leaves. */
+static int leaf_chunks(Solver &S, const ListView &LV, int32_t &npp, int32_t &total, int32_t &nsrc, cudaStream_t st) {
     const int32_t nleaves = (int32_t)S.st.leaves;
     const int64_t nn = S.nnodes;
     const size_t nc = 2 * ((size_t)nleaves + 1);
     TG_TRY(ensure(S.ew_cnt, nc));
     TG_TRY(ensure(S.ew_off, nc + 1));
-    int32_t *slot = nullptr, *nsrc_d = S.ew_off.p + nc; /* the source count sits behind the scan: one readback */
-    if (!f64) {
-        TG_TRY(ensure(S.ew_slot, (size_t)nn));
-        TG_TRY(ensure(S.ew_src, (size_t)nn));
-        slot = S.ew_slot.p;
-        TG_CUDA(cudaMemsetAsync(slot, 0xff, sizeof(int32_t) * nn, st));
-    }
+    TG_TRY(ensure(S.ew_slot, (size_t)nn));
+    TG_TRY(ensure(S.ew_src, (size_t)nn));
+    int32_t *slot = S.ew_slot.p, *nsrc_d = S.ew_off.p + nc; /* the source count sits behind the scan: one readback */
+    TG_CUDA(cudaMemsetAsync(slot, 0xff, sizeof(int32_t) * nn, st));
     TG_CUDA(cudaMemsetAsync(nsrc_d, 0, sizeof(int32_t), st));
     k_ewald_count<<<(int)(((int64_t)(nleaves + 1) * 32 + 127) / 128), 128, 0, st>>>(S.idx.p, nleaves, LV, S.ew_cnt.p,
                                                                                   slot);
     TG_TRY(launched(S));
-    if (!f64) {
-        k_ewald_slots<<<(int)((nn + 255) / 256), 256, 0, st>>>(nn, slot, S.ew_src.p, nsrc_d);
-        TG_TRY(launched(S));
-    }
+    k_ewald_slots<<<(int)((nn + 255) / 256), 256, 0, st>>>(nn, slot, S.ew_src.p, nsrc_d);
+    TG_TRY(launched(S));
     size_t stmp = 0;
     TG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, stmp, S.ew_cnt.p, S.ew_off.p, (int)nc, st));
     TG_TRY(ensure(S.cub_tmp, stmp));
@@ -711,38 +712,40 @@ static int leaf_ewald(Solver &S, const GParams &P, const ListView &LV, const Ewa
     TG_CUDA(cudaStreamSynchronize(st));
     int32_t tot[3];
     std::memcpy(tot, S.h_small + 2048, sizeof(tot));
-    const int32_t npp = tot[0], total = tot[1], nsrc = tot[2];
+    npp = tot[0], total = tot[1], nsrc = tot[2];
+    return TG_OK;
+}
+
+/* the leaf Ewald lists (PP_E, PC_E) of every leaf, in balanced chunks, added
+ * to the FP64 accumulators accd (leaf_max <= 64) */
+template <class T>
+static int leaf_ewald(Solver &S, const GParams &P, const ListView &LV, const EwaldTables &E, cudaStream_t st) {
+    typedef typename Sep<T>::T2 T2;
+    const int32_t nleaves = (int32_t)S.st.leaves;
+    int32_t npp = 0, total = 0, nsrc = 0;
+    TG_TRY(leaf_chunks(S, LV, npp, total, nsrc, st));
     if (total <= 0) return TG_OK;
     TG_TRY(ensure(S.ew_part, (size_t)total * 64 * 4));
-    float2 *tpart = nullptr;
-    if (!f64 && npp > 0) {
-        TG_TRY(ensure(S.ew_sf, (size_t)nsrc * NSEP));
-        TG_TRY(ensure(S.ew_tpart, (size_t)npp * NSEP));
-        tpart = S.ew_tpart.p;
-        k_ewald_sf<<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E, S.ew_sf.p);
-        TG_TRY(launched(S));
-    }
     const int32_t *offp = S.ew_off.p + nleaves + 1;
+    T2 *tpart = nullptr;
     if (npp > 0) {
-        if (f64)
-            k_ewald_pp<double><<<npp, 64, 0, st>>>(P, S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, E,
-                                                   S.ew_part.p, nullptr, nullptr, nullptr);
-        else
-            k_ewald_pp<float><<<npp, 64, 0, st>>>(P, S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, E,
-                                                  S.ew_part.p, slot, S.ew_sf.p, tpart);
+        TG_TRY(ensure(S.ew_sf, (size_t)nsrc * Sep<T>::N * sizeof(T2)));
+        TG_TRY(ensure(S.ew_tpart, (size_t)npp * Sep<T>::N * sizeof(T2)));
+        T2 *sf = reinterpret_cast<T2 *>(S.ew_sf.p);
+        tpart = reinterpret_cast<T2 *>(S.ew_tpart.p);
+        k_ewald_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E, sf);
+        TG_TRY(launched(S));
+        k_ewald_pp<T><<<npp, 64, 0, st>>>(P, S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, E,
+                                          S.ew_part.p, S.ew_slot.p, sf, tpart);
         TG_TRY(launched(S));
     }
     if (total > npp) {
-        if (f64)
-            k_ewald_pc<double><<<total - npp, 64, 0, st>>>(S.idx.p, nleaves, npp, offp, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p,
-                                                           S.pos.p, LV, E, S.ew_part.p);
-        else
-            k_ewald_pc<float><<<total - npp, 64, 0, st>>>(S.idx.p, nleaves, npp, offp, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p,
-                                                          S.pos.p, LV, E, S.ew_part.p);
+        k_ewald_pc<T><<<total - npp, 64, 0, st>>>(S.idx.p, nleaves, npp, offp, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p, S.pos.p,
+                                                  LV, E, S.ew_part.p);
         TG_TRY(launched(S));
     }
-    k_ewald_reduce<<<nleaves, 256, 0, st>>>(S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.ew_part.p, S.accd.p,
-                                            tpart, S.pos.p, E);
+    k_ewald_reduce<T><<<nleaves, 256, 0, st>>>(S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.ew_part.p, S.accd.p,
+                                               tpart, S.pos.p, E);
     TG_TRY(launched(S));
     return TG_OK;
 }
@@ -803,7 +806,7 @@ int gravity_forces(Solver &S, cudaStream_t st) {
                                                                   S.nd_ms.p, S.pos.p, LV, E, S.nd_L.p, nullptr,
                                                                   S.accd.p);
             TG_TRY(launched(S));
-            if (S.prm.ewald) TG_TRY(leaf_ewald(S, P, LV, E, f64, st));
+            if (S.prm.ewald) TG_TRY(f64 ? leaf_ewald<double>(S, P, LV, E, st) : leaf_ewald<float>(S, P, LV, E, st));
             if (!f64) {
                 if (S.have_events) {
                     TG_CUDA(cudaEventRecord(S.ev[6], st));

@@ -135,7 +135,7 @@ struct Solver {
     DevBuf<float> ck_v;
     int ck_steps = -1;
     double ck_dt = 0.0;
-    DevBuf<double> adj_x, adj_v, tid_u, tid_o, tid_U, tid_V;
+    DevBuf<double> adj_x, adj_v, tid_u, tid_o, tid_U, tid_V, tid_tile;
     DevBuf<int32_t> ew_cnt, ew_off; /* leaf Ewald chunks per leaf, and their exclusive scan */
     DevBuf<double> ew_part;          /* 64 x 4 partial sums per chunk */
     DevBuf<float4> ew_real, ew_four;
@@ -145,10 +145,10 @@ struct Solver {
     DevBuf<double2> ew_Pd;
     DevBuf<int4> ew_sep_h;       /* PP Ewald split: reciprocal vectors and weights */
     DevBuf<double> ew_sep_w;
-    float ew_sep_k = 0.0f, ew_sep_r0 = 0.0f, ew_sep_r2 = 0.0f;
+    double ew_sep_k = 0.0, ew_sep_r0 = 0.0, ew_sep_r2 = 0.0;
     DevBuf<int32_t> ew_slot, ew_src; /* per node: its row of ew_sf, or -1; the nodes of the rows, then their count */
-    DevBuf<float2> ew_sf;        /* per PP_E source leaf and h: (cos, sin) sums over its particles */
-    DevBuf<float2> ew_tpart;     /* per PP_E chunk and h: source sums */
+    DevBuf<unsigned char> ew_sf;    /* per PP_E source leaf and h: (cos, sin) sums over its particles (Sep<T>::T2) */
+    DevBuf<unsigned char> ew_tpart; /* per PP_E chunk and h: source sums (Sep<T>::T2) */
     bool ew_use_tab = false;       /* a periodic solver of the FP32 path */
     const float *ew_tab = nullptr; /* the device's table of local expansions (FP32 path), shared by its solvers */
     bool have_tables = false;
