@@ -337,6 +337,8 @@ int tg_destroy(tg_solver *s) {
     release(S.wk_loff);
     release(S.wk_caps);
     release(S.wk_rec);
+    release(S.pp_rec);
+    release(S.pp_part);
     release(S.scratch); release(S.dev_err); release(S.dev_cnt);
     release(S.ew_real); release(S.ew_four); release(S.ew_Hf); release(S.ew_Hd); release(S.ew_Pf); release(S.ew_Pd);
     release(S.ew_cnt); release(S.ew_off); release(S.ew_part); release(S.ew_sf); release(S.ew_sep_h);
@@ -737,7 +739,7 @@ int tg_memory_report(tg_solver *s, char *buf, int64_t cap) {
     TG_MEM(nd_r); TG_MEM(nd_rmax); TG_MEM(nd_aabb); TG_MEM(nd_prange); TG_MEM(nd_L); TG_MEM(nd_Lloc);
     TG_MEM(loff[0]); TG_MEM(llen[0]); TG_MEM(pool[0]); TG_MEM(pool[1]); TG_MEM(pool[2]); TG_MEM(pool[3]);
     TG_MEM(pool[4]); TG_MEM(pool[5]); TG_MEM(pool[6]); TG_MEM(pool[7]); TG_MEM(nxt_pool[0]); TG_MEM(nxt_pool[1]);
-    TG_MEM(nxt_off[0]); TG_MEM(nxt_len[0]); TG_MEM(scratch); TG_MEM(ew_cnt); TG_MEM(ew_off); TG_MEM(ew_part);
+    TG_MEM(nxt_off[0]); TG_MEM(nxt_len[0]); TG_MEM(pp_rec); TG_MEM(pp_part); TG_MEM(scratch); TG_MEM(ew_cnt); TG_MEM(ew_off); TG_MEM(ew_part);
     TG_MEM(ew_slot); TG_MEM(ew_src); TG_MEM(ew_sf); TG_MEM(ew_tpart); TG_MEM(ck_x); TG_MEM(ck_v); TG_MEM(adj_x); TG_MEM(adj_v);
     TG_MEM(tid_u); TG_MEM(tid_o); TG_MEM(tid_U); TG_MEM(tid_V); TG_MEM(fof_P); TG_MEM(fof_key); TG_MEM(fof_mem);
     TG_MEM(fof_pairs); TG_MEM(rung_flag); TG_MEM(rung_scan); TG_MEM(rung_nact);

@@ -14,7 +14,7 @@
  *            PC_direct, PP_direct (source leaves staged in shared memory),
  *            PC_ewald, PP_ewald; -phi_self once (src/gravity.cpp:295).
  *            The FP32 path with leaf_max <= 64 runs it without PP_direct
- *            (into an FP64 buffer) and then k_pp_leaf (tg_pp2.cuh), which adds
+ *            (into an FP64 buffer) and then pp_direct (tg_pp2.cuh), which adds
  *            PP_direct and phi_self and writes the float4 result.
  *
  * Precision: T = float (FP32 path: FP32 arithmetic, per-tile FP32 partial
@@ -504,26 +504,6 @@ __global__ void __launch_bounds__(BLOCK) k_leaf(GParams P, const int32_t *__rest
     }
 }
 
-/* ---- PP direct for the FP32 path (leaf_max <= 64) ----
- * Source positions are staged in split fixed point relative to the sink
- * leaf's centre Xr: for a = wrap(Y - Xr),
- *     hi = (a >> 16) 2^-16,   lo = (a & 0xffff) 2^-32
- * are exact in FP32, and dX = (hi_i - hi_j) + (lo_i - lo_j) is the correctly
- * rounded FP32 value of (X_i - Y_j) 2^-32 -- exactly the reference's dX
- * (src/gravity.cpp:223) -- from three FP32 additions and no integer-to-float
- * conversion per pair.  The identity needs |a_i - a_j| < 2^31, checked per
- * staged batch; otherwise that batch's pairs take the per-pair wrap. */
-__device__ __forceinline__ void split_hl(int32_t a, float &h, float &l) {
-    h = __int2float_rn(a >> 16) * 1.52587890625e-05f;
-    l = __int2float_rn(a & 0xffff) * 2.3283064365386963e-10f;
-}
-
-__device__ __forceinline__ uint32_t warp_max_u(uint32_t v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
 /* offset of Y from Xr: int32 wrap (periodic) or plain difference (free space);
  * mag accumulates the largest magnitude, saturated at 2^31 (a free-space
  * offset that does not fit an int32 reads as 2^31) */
@@ -777,15 +757,61 @@ static int node_stage(Solver &S, const GParams &P, const ListView &LV, const Ewa
     return TG_OK;
 }
 
+/* PP direct of the FP32 path (leaf_max <= 64): far + PP_direct - phi_self into acc.
+ * A list holds about 17 / theta^3 source leaves (leaves within (r_a + r_b) / theta,
+ * at most all of them).  From PPB_LONG on, or with fewer leaves than SMs,
+ * k_pp_long is the faster one: ms with k_pp_short / k_pp_long at 40 leaves per
+ * list (128^3, theta 0.7) 4.2 / 4.6, 95 (101^3, theta 0.5) 2.9 / 3.4, 1800 (128^3,
+ * theta 0.2) 112 / 102, 2100 (256^3, theta 0.19) 731 / 662; 92 leaves with 92 each
+ * (4096 uniform) 0.175 / 0.050 in quarters.  Fewer leaves than one wave of blocks:
+ * the lists are cut into shares so that the wave is full (4096 uniform: 0.79 ms
+ * without).  The choice depends on the tree alone, not on which leaves are
+ * active, so a rung step's forces equal a full solve's bit for bit. */
+constexpr int PPB_LONG = 512;
+static int pp_direct(Solver &S, const GParams &P, const ListView &LV, cudaStream_t st) {
+    const int64_t n = S.n, nn = S.nnodes;
+    const int32_t nleaves = (int32_t)S.st.leaves;
+    TG_TRY(ensure(S.pp_rec, 2 * (size_t)nn));
+    PPRec *rec = reinterpret_cast<PPRec *>(S.pp_rec.p);
+    k_pp_records<<<(int)((nn + 255) / 256), 256, 0, st>>>(nn, S.nd_pb.p, S.nd_pe.p, S.nd_child0.p, S.nd_aabb.p, rec);
+    TG_TRY(launched(S));
+    int64_t tree = 0; /* leaves of the tree */
+    for (int64_t l : S.level_leaves) tree += l;
+    const double list = std::min(17.0 / (S.prm.theta * S.prm.theta * S.prm.theta), (double)tree);
+    const bool few = tree < S.num_sms, longl = few || list >= PPB_LONG;
+    const int wave = S.num_sms * (longl ? PPL_MINB : PPS_MINB);
+    const int shares = tree >= wave ? 1 : (int)std::min<int64_t>((wave + tree - 1) / tree, PPB_SHARES);
+    double *part = nullptr;
+    if (shares > 1) {
+        TG_TRY(ensure(S.pp_part, (size_t)shares * 4 * n));
+        part = S.pp_part.p;
+    }
+    const dim3 g(nleaves, shares);
+    if (few)
+        k_pp_long<true><<<g, PPB_T, 0, st>>>(P, S.idx.p, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p, rec, S.pos.p, LV, S.accd.p,
+                                             S.acc.p, part, n);
+    else if (longl)
+        k_pp_long<false><<<g, PPB_T, 0, st>>>(P, S.idx.p, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p, rec, S.pos.p, LV, S.accd.p,
+                                              S.acc.p, part, n);
+    else
+        k_pp_short<<<g, PPB_T, 0, st>>>(P, S.idx.p, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p, rec, S.pos.p, LV, S.accd.p,
+                                        S.acc.p, part, n);
+    TG_TRY(launched(S));
+    if (shares > 1) {
+        k_pp_reduce<<<nleaves, 64, 0, st>>>(P, S.idx.p, S.nd_pb.p, S.nd_pe.p, S.accd.p, part, shares, n, S.acc.p);
+        TG_TRY(launched(S));
+    }
+    return TG_OK;
+}
+
 int gravity_forces(Solver &S, cudaStream_t st) {
     if (!S.have_lists) return TG_ERR_STATE;
     TG_TRY(ewald_tables(S, st));
-    const int64_t nn = S.nnodes, n = S.n;
+    const int64_t n = S.n;
     const GParams P = make_gparams(S.prm);
     const EwaldTables E = tables(S);
     const ListView LV = listview(S);
     const bool f64 = S.prm.precision == TG_PREC_F64;
-    (void)nn;
     const bool split_pp = !f64 && S.prm.leaf_max <= 64;
     if (f64 || split_pp) TG_TRY(ensure(S.accd, 4 * n));
     if (!f64) TG_TRY(ensure(S.acc, n));
@@ -812,8 +838,7 @@ int gravity_forces(Solver &S, cudaStream_t st) {
                     TG_CUDA(cudaEventRecord(S.ev[6], st));
                     S.pp_timed = true;
                 }
-                k_pp_leaf<<<g, PPB_T, 0, st>>>(P, S.idx.p, nleaves, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p, S.nd_aabb.p,
-                                               S.pos.p, LV, S.accd.p, S.acc.p);
+                TG_TRY(pp_direct(S, P, LV, st));
             }
         } else {
             if (f64)
@@ -822,8 +847,8 @@ int gravity_forces(Solver &S, cudaStream_t st) {
             else
                 k_leaf<float, 128><<<g, 128, 0, st>>>(P, S.idx.p, nleaves, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p, S.pos.p, LV,
                                                       E, S.nd_L.p, S.acc.p, nullptr);
+            TG_TRY(launched(S));
         }
-        TG_TRY(launched(S));
     }
     if (S.have_events) TG_CUDA(cudaEventRecord(S.ev[5], st));
     S.have_forces = true;

@@ -110,6 +110,8 @@ struct Solver {
     DevBuf<int64_t *> wk_loff;
     DevBuf<int64_t> wk_caps;
     DevBuf<WalkRec> wk_rec;              /* per node: what the opening tests read */
+    DevBuf<int4> pp_rec;                 /* 2 per node: source leaves as PP direct selects them */
+    DevBuf<double> pp_part;              /* list shares' sums, 4 per share and particle */
     DevBuf<int32_t> scratch;             /* leaf drain per-warp scratch */
     int64_t scratch_per_warp = 0;
     int drain_warps = 0;
