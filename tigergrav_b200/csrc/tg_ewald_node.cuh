@@ -18,7 +18,7 @@
 constexpr int EN_KCC = 128; /* CC_E source nodes per chunk (4 per lane) */
 constexpr int EN_KCP = 4;   /* CP_E source leaves per chunk */
 #ifndef EN_MINB
-#define EN_MINB 3 /* resident 128-thread blocks per SM the FP32 kernel is compiled for */
+#define EN_MINB 4 /* resident 128-thread blocks per SM the FP32 kernel is compiled for (3: 126, 4: 125 ms at 256^3) */
 #endif
 #ifndef EN_MINB_D
 #define EN_MINB_D 2 /* and the FP64 kernel */
@@ -61,8 +61,10 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? EN_MINB : EN_MINB_D)
     /* each lane's expansion sums (odd stride LP: no bank conflicts).  FP64
      * keeps them here throughout, which leaves the registers to green_ewald;
      * FP32, in registers until the end */
-    __shared__ T sL[128 * LP];
-    T *const sl = sL + threadIdx.x * LP;
+    constexpr int WARP_FLOATS = sizeof(T) == 4 ? 32 * ET_STRIDE : 32 * LP; /* FP32: a warp's table rows before that */
+    __shared__ __align__(16) T s_buf[4 * WARP_FLOATS];
+    T *const sL = s_buf + (threadIdx.x >> 5) * WARP_FLOATS;
+    T *const sl = sL + lane * LP;
     T Lreg[sizeof(T) == 4 ? LP : 1];
     T *const L = sizeof(T) == 4 ? Lreg : sl;
 #pragma unroll
@@ -72,7 +74,21 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? EN_MINB : EN_MINB_D)
     if (k < kcc) {
         const int32_t *lst = LV.pool[TG_CC_E] + LV.off[TG_CC_E][i];
         const int32_t e0 = k * EN_KCC, e1 = min(ncc, e0 + EN_KCC);
-        if (sizeof(T) == 4 || e1 - e0 >= EWALD_WARP_LIST) {
+        if constexpr (sizeof(T) == 4) {
+            for (int32_t j0 = e0; j0 < e1; j0 += 32) {
+                const MSrc &s = ms[lst[min(j0 + lane, e1 - 1)]];
+                float dX[3], o[3], D[LP], M[MP];
+                uint32_t sg[3];
+#pragma unroll
+                for (int d = 0; d < 3; d++) dX[d] = sep<float>(X[d], s.x[d], true);
+                et_stage(E.tab, et_locate(dX, o, sg), min(32, e1 - j0), sL);
+                if (j0 + lane >= e1) continue;
+                et_eval(reinterpret_cast<const float4 *>(sL + lane * ET_STRIDE), dX, o, sg, D);
+#pragma unroll
+                for (int q = 0; q < MP; q++) M[q] = s.m[q];
+                contract_M2L<float, float>(L, M, D);
+            }
+        } else if (e1 - e0 >= EWALD_WARP_LIST) {
             for (int32_t j = e0 + lane; j < e1; j += 32) {
                 const MSrc &s = ms[lst[j]];
                 T dX[3], D[LP], M[MP];
@@ -83,7 +99,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? EN_MINB : EN_MINB_D)
                 for (int q = 0; q < MP; q++) M[q] = T(s.m[q]);
                 contract_M2L<T, T>(L, M, D);
             }
-        } else if constexpr (sizeof(T) == 8) {
+        } else {
             for (int32_t j = e0; j < e1; j++) {
                 const MSrc &s = ms[lst[j]];
                 T dX[3], D[LP], M[MP];
@@ -118,6 +134,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? EN_MINB : EN_MINB_D)
             if (lane >= o) incl += v;
         }
         const int32_t total = __shfl_sync(0xffffffffu, incl, EN_KCP - 1);
+        const int32_t sb0 = __shfl_sync(0xffffffffu, sb, 0);
         for (int32_t q0 = 0; q0 < total; q0 += 32) {
             const int32_t q = q0 + lane;
             int32_t at = 0, lo = 0; /* this lane's particle */
@@ -127,12 +144,20 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? EN_MINB : EN_MINB_D)
                 if (q >= lo && q < hi) at = b + q - lo;
                 lo = hi;
             }
-            if (q < total) {
-                const int4 y = pos[at];
-                const int32_t yy[3] = {y.x, y.y, y.z};
-                T dX[3], D[LP];
+            const int4 y = pos[q < total ? at : sb0];
+            const int32_t yy[3] = {y.x, y.y, y.z};
+            T dX[3], D[LP];
 #pragma unroll
-                for (int d = 0; d < 3; d++) dX[d] = sep<T>(X[d], yy[d], true);
+            for (int d = 0; d < 3; d++) dX[d] = sep<T>(X[d], yy[d], true);
+            if constexpr (sizeof(T) == 4) {
+                float o[3];
+                uint32_t sg[3];
+                et_stage(E.tab, et_locate(dX, o, sg), min(32, total - q0), sL);
+                if (q < total) {
+                    et_eval(reinterpret_cast<const float4 *>(sL + lane * ET_STRIDE), dX, o, sg, D);
+                    contract_P2L<T, T>(L, m, D);
+                }
+            } else if (q < total) {
                 green_ewald_any<T>(E, dX, D);
                 contract_P2L<T, T>(L, m, D);
             }
@@ -140,11 +165,12 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? EN_MINB : EN_MINB_D)
     }
     /* the warp's sum in FP64, a lane per term */
     if constexpr (sizeof(T) == 4) {
+        __syncwarp(); /* the last rows are read */
 #pragma unroll
         for (int q = 0; q < LP; q++) sl[q] = L[q];
     }
     __syncwarp();
-    const T *w = sL + (threadIdx.x & ~31) * LP;
+    const T *w = sL;
     for (int q = lane; q < LP; q += 32) {
         double v = 0.0;
 #pragma unroll 8

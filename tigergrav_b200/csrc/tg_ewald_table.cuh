@@ -241,18 +241,21 @@ __device__ __forceinline__ int et_axis(float X, float &o, uint32_t &sg) {
     return q;
 }
 
-/* green_ewald(X) for |X_d| <= 1/2 (tigergrav/green.hpp:189-286); r <= 1e-6 gives phi0 alone as there */
-__device__ __forceinline__ void green_ewald_table(const float *__restrict__ table, const float *X, float *D) {
-    float o[3];
-    uint32_t sg[3];
+/* the cell of X, X's offset from its centre in the octant of |X|, and X's signs */
+__device__ __forceinline__ int et_locate(const float *X, float *o, uint32_t *sg) {
     int cell = 0;
 #pragma unroll
     for (int d = 0; d < 3; d++) cell = cell * ET_N + et_axis(X[d], o[d], sg[d]);
+    return cell;
+}
+
+/* green_ewald(X) for |X_d| <= 1/2 (tigergrav/green.hpp:189-286) from the row of
+ * X's cell; r <= 1e-6 gives phi0 alone as there */
+__device__ __forceinline__ void et_eval(const float4 *row, const float *X, const float *o, const uint32_t *sg, float *D) {
     float R[ET_ROW];
-    const float4 *row = reinterpret_cast<const float4 *>(table + (int64_t)cell * ET_ROW);
 #pragma unroll
     for (int q = 0; q < ET_ROW / 4; q++) {
-        const float4 v = __ldg(row + q);
+        const float4 v = row[q];
         R[4 * q] = v.x, R[4 * q + 1] = v.y, R[4 * q + 2] = v.z, R[4 * q + 3] = v.w;
     }
     float *A = R, *B = R + ET_A;
@@ -329,6 +332,37 @@ __device__ __forceinline__ void green_ewald_table(const float *__restrict__ tabl
 #pragma unroll
         for (int q = 1; q < LP; q++) D[q] = 0.0f;
     }
+}
+
+__device__ __forceinline__ void green_ewald_table(const float *__restrict__ table, const float *X, float *D) {
+    float o[3];
+    uint32_t sg[3];
+    const int cell = et_locate(X, o, sg);
+    et_eval(reinterpret_cast<const float4 *>(table + (int64_t)cell * ET_ROW), X, o, sg, D);
+}
+
+/* The rows of a warp's cells into shared memory, row k at buf + k ET_STRIDE, for
+ * the first n lanes; all lanes call it.  Half a warp copies a row, 256
+ * consecutive bytes, where a lane reading its own row touches another cache line
+ * than every other lane with each load; those wavefronts bounded the node Ewald
+ * kernel (node phase at 128^3 theta 0.2: 63.7 -> 47.7 ms, 256^3 theta 0.19: 148 ->
+ * 125 ms; the 80-byte multipoles staged the same way as well: 144 ms).  The stride
+ * keeps the lanes' 16-byte reads free of bank conflicts. */
+constexpr int ET_STRIDE = ET_ROW + 4;
+__device__ __forceinline__ void et_stage(const float *__restrict__ table, int cell, int n, float *buf) {
+    const int lane = threadIdx.x & 31, h = lane >> 4, q = lane & 15;
+    __syncwarp(); /* the rows of the last call are read */
+#pragma unroll 8
+    for (int k = 0; k < n; k += 2) {
+        const int c = __shfl_sync(0xffffffffu, cell, (k + h) & 31);
+        if (k + h < n) {
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(buf + (k + h) * ET_STRIDE + 4 * q);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(table + (int64_t)c * ET_ROW + 4 * q)
+                         : "memory");
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
 }
 
 /* green_ewald of the solver's kernels: FP32 from the table, FP64 from the sums */
