@@ -503,7 +503,7 @@ __device__ __forceinline__ void tidal_ewald_pair(const EwaldTables &E, const T *
 /* one chunk of a PP_E list (as k_ewald_pp): the real-space part per pair into
  * part (3 per sink), the reciprocal source sums into tpart */
 template <class T>
-__global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, const int32_t *__restrict__ leaves, int32_t nleaves,
+__global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, bool fine, const int32_t *__restrict__ leaves, int32_t nleaves,
                                                        const int32_t *__restrict__ off, const int32_t *__restrict__ pb,
                                                        const int32_t *__restrict__ pe, const int4 *__restrict__ pos,
                                                        ListView LV, EwaldTables E, const double *__restrict__ u,
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, const int32_t 
     Acc<T> o[3];
     for (int d = 0; d < 3; d++) o[d].init(0.0);
     const int32_t *lst = LV.pool[TG_PP_E] + LV.off[TG_PP_E][leaf];
-    const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len), e0 = k * kpp, e1 = min(len, e0 + kpp);
+    const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len, fine), e0 = k * kpp, e1 = min(len, e0 + kpp);
     const T m = T(P.m_d);
     if (tid < e1 - e0) s_row[tid] = slot[lst[e0 + tid]];
     for (int32_t e = e0; e < e1; e++) {
@@ -637,7 +637,7 @@ static int tidal_ewald(Solver &S, const GParams &P, const ListView &LV, const Ew
     Sep4<T> *sf = reinterpret_cast<Sep4<T> *>(S.ew_sf.p), *tpart = reinterpret_cast<Sep4<T> *>(S.ew_tpart.p);
     k_tidal_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, S.tid_u.p, E, sf);
     TG_TRY(launched(S));
-    k_tidal_ewald_pp<T><<<npp, 64, 0, st>>>(P, S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, E,
+    k_tidal_ewald_pp<T><<<npp, 64, 0, st>>>(P, ew_fine(S), S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, E,
                                             S.tid_u.p, S.ew_part.p, S.ew_slot.p, sf, tpart);
     TG_TRY(launched(S));
     k_tidal_ewald_reduce<T><<<nleaves, 256, 0, st>>>(S.idx.p, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E, S.tid_u.p,

@@ -22,17 +22,20 @@
 constexpr int EW_KPP_MAX = 32;
 /* PP_E source leaves per chunk: 16 chunks of a list, of 8 to 32 leaves (at most
  * 32 * 64 * 64 pairs).  Each chunk's slots take 5 KB in FP32, so chunks of 8
- * throughout hold 225 MB for 32768 particles where these hold 60 MB. */
-__host__ __device__ __forceinline__ int32_t ew_kpp(int32_t len) {
-    const int32_t k = (len + 15) >> 4;
-    return k < 8 ? 8 : (k > EW_KPP_MAX ? EW_KPP_MAX : k);
+ * throughout hold 225 MB for 32768 particles where these hold 60 MB.  fine (a tree
+ * with fewer leaves than twice the SMs): up to 24 chunks, of 4 leaves on, which
+ * fill the GPU (4096 particles: leaf Ewald and L2P 0.41 -> 0.33 ms).  By the list and the tree alone, so the order of the sums does not
+ * depend on which leaves are active. */
+__host__ __device__ __forceinline__ int32_t ew_kpp(int32_t len, bool fine) {
+    const int32_t k = fine ? (len + 23) / 24 : (len + 15) >> 4, lo = fine ? 4 : 8;
+    return k < lo ? lo : (k > EW_KPP_MAX ? EW_KPP_MAX : k);
 }
 constexpr int EW_KPC = 64; /* PC_E source nodes per chunk */
 
 /* one warp per leaf: chunk counts (zeros at li = nleaves, so that the scan ends
  * in the totals); with slot, marks the source leaves of the PP_E lists */
 __global__ void k_ewald_count(const int32_t *__restrict__ leaves, int32_t nleaves, ListView LV,
-                              int32_t *__restrict__ cnt, int32_t *__restrict__ slot) {
+                              int32_t *__restrict__ cnt, int32_t *__restrict__ slot, bool fine) {
     const int32_t li = (int32_t)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (li > nleaves) return;
@@ -46,7 +49,7 @@ __global__ void k_ewald_count(const int32_t *__restrict__ leaves, int32_t nleave
         }
     }
     if (lane == 0) {
-        cnt[li] = (npp + ew_kpp(npp) - 1) / ew_kpp(npp);
+        cnt[li] = (npp + ew_kpp(npp, fine) - 1) / ew_kpp(npp, fine);
         cnt[nleaves + 1 + li] = (npc + EW_KPC - 1) / EW_KPC;
     }
 }
@@ -84,7 +87,7 @@ __device__ __forceinline__ int32_t ew_leaf(const int32_t *__restrict__ off, int3
  * real-space part per pair and the chunk's reciprocal source sums (tpart). */
 template <class T>
 __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
-    k_ewald_pp(GParams P, const int32_t *__restrict__ leaves, int32_t nleaves, const int32_t *__restrict__ off,
+    k_ewald_pp(GParams P, bool fine, const int32_t *__restrict__ leaves, int32_t nleaves, const int32_t *__restrict__ off,
                const int32_t *__restrict__ pb, const int32_t *__restrict__ pe, const int4 *__restrict__ pos, ListView LV,
                EwaldTables E, double *__restrict__ part, const int32_t *__restrict__ slot,
                const typename Sep<T>::T2 *__restrict__ sf, typename Sep<T>::T2 *__restrict__ tpart) {
@@ -102,7 +105,7 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
     aphi.init(0.0);
     for (int d = 0; d < 3; d++) ag[d].init(0.0);
     const int32_t *lst = LV.pool[TG_PP_E] + LV.off[TG_PP_E][leaf];
-    const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len), e0 = k * kpp, e1 = min(len, e0 + kpp);
+    const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len, fine), e0 = k * kpp, e1 = min(len, e0 + kpp);
     const T m = T(P.m_d);
     if (tid < e1 - e0) s_row[tid] = slot[lst[e0 + tid]];
     for (int32_t e = e0; e < e1; e++) {

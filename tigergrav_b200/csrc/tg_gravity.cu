@@ -705,6 +705,15 @@ static int node_ewald(Solver &S, const GParams &P, const ListView &LV, const Ewa
     return TG_OK;
 }
 
+/* leaves of the tree (the empty ones too) */
+static int64_t tree_leaves(const Solver &S) {
+    int64_t n = 0;
+    for (int64_t l : S.level_leaves) n += l;
+    return n;
+}
+/* whether the PP_E chunks are the fine ones (ew_kpp) */
+static bool ew_fine(const Solver &S) { return tree_leaves(S) < 2 * S.num_sms; }
+
 /* The leaf Ewald lists cut into chunks (tg_ewald_leaf.cuh): their offsets in
  * ew_off, the PP_E source leaves in ew_src with their rows in ew_slot, and the
  * numbers of PP_E chunks, of all chunks and of source leaves. */
@@ -720,7 +729,7 @@ static int leaf_chunks(Solver &S, const ListView &LV, int32_t &npp, int32_t &tot
     TG_CUDA(cudaMemsetAsync(slot, 0xff, sizeof(int32_t) * nn, st));
     TG_CUDA(cudaMemsetAsync(nsrc_d, 0, sizeof(int32_t), st));
     k_ewald_count<<<(int)(((int64_t)(nleaves + 1) * 32 + 127) / 128), 128, 0, st>>>(S.idx.p, nleaves, LV, S.ew_cnt.p,
-                                                                                  slot);
+                                                                                  slot, ew_fine(S));
     TG_TRY(launched(S));
     k_ewald_slots<<<(int)((nn + 255) / 256), 256, 0, st>>>(nn, slot, S.ew_src.p, nsrc_d);
     TG_TRY(launched(S));
@@ -757,7 +766,7 @@ static int leaf_ewald(Solver &S, const GParams &P, const ListView &LV, const Ewa
         tpart = reinterpret_cast<T2 *>(S.ew_tpart.p);
         k_ewald_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E, sf);
         TG_TRY(launched(S));
-        k_ewald_pp<T><<<npp, 64, 0, st>>>(P, S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, E,
+        k_ewald_pp<T><<<npp, 64, 0, st>>>(P, ew_fine(S), S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, E,
                                           S.ew_part.p, S.ew_slot.p, sf, tpart);
         TG_TRY(launched(S));
     }
@@ -817,8 +826,7 @@ static int pp_direct(Solver &S, const GParams &P, const ListView &LV, cudaStream
     PPRec *rec = reinterpret_cast<PPRec *>(S.pp_rec.p);
     k_pp_records<<<(int)((nn + 255) / 256), 256, 0, st>>>(nn, S.nd_pb.p, S.nd_pe.p, S.nd_child0.p, S.nd_aabb.p, rec);
     TG_TRY(launched(S));
-    int64_t tree = 0; /* leaves of the tree */
-    for (int64_t l : S.level_leaves) tree += l;
+    const int64_t tree = tree_leaves(S);
     const double list = std::min(17.0 / (S.prm.theta * S.prm.theta * S.prm.theta), (double)tree);
     const bool few = tree < S.num_sms, longl = few || list >= PPB_LONG;
     const int wave = S.num_sms * (longl ? PPL_MINB : PPS_MINB);
