@@ -84,7 +84,7 @@ WORKLOADS = {
 METRIC = "Mparticles/s per force eval at RMS err<=1e-4 vs FP64 Ewald; adjoint/fwd cost"
 KINDS = ("PP_D", "PP_E", "PC_D", "PC_E", "CC_D", "CC_E", "CP_D", "CP_E")
 
-# FP32 operations per PP pair in k_pp_leaf's inner loop for far source
+# FP32 operations per PP pair in the PP kernels' inner loop for far source
 # leaves (nearly all pairs at the headline workload), counted from the source
 # with an FMA as 2: separation 3, r^2 5 (1 mul + 2 fma), rsqrt 1, 1/r^3 2,
 # phi sum 1, three force FMAs 6 -> 18 (near leaves: 6 more for the split
@@ -92,29 +92,21 @@ KINDS = ("PP_D", "PP_E", "PC_D", "PC_E", "CC_D", "CC_E", "CP_D", "CP_E")
 # is not counted).
 PP_FLOPS = 18
 # FP32 operations per interaction of the Ewald and multipole kernels, counted
-# from the source the same way.  One real-space image: separation and r^2 8,
-# rsqrt and powers of 1/r 8, erfc/exp 18, d0..d4 31, the moment sums 120 ->
-# 185; 38.8 images on average inside the FP32 cut r < 2.1 (4/3 pi 2.1^3);
-# finish 105 -> 7.3k per green_ewald without its reciprocal terms.  The 61
-# reciprocal terms of PC_E / PP_E are not evaluated per interaction: each
-# chunk sums its sources' m_k (cos, sin) per vector h in the leaf kernels
-# (tg_ewald_sep.cuh): per PC_E source node 56 ops x 61 shared by the sink
-# leaf's particles (~32: +110 per interaction); per PP_E source leaf 4 x 61
-# shared by its pairs (negligible).  The per-particle evaluation of the sums
-# (61 terms) is not counted.  The node kernels keep the per-interaction
-# reciprocal sum: one term of the half sum h.X 5, reduction and sin/cos 5,
-# 35 FMAs 70 -> 80, x 61 = 4.9k.  Contractions: M2L 858, M2P 414, P2L 70
-# (direct kernels: the reference's constants).
-# PP_E pair (cut r < 2, origin separate): 32.5 images x 44 + 30 = 1.46k.
-NODE_FLOPS = {"CC_D": 1025, "CP_D": 455, "CC_E": 13100, "CP_E": 12300}
-LEAF_FLOPS = {"PC_D": 581, "PC_E": 7800, "PP_E": 1460}
+# from the source the same way.  A derivative tensor from the expansion table
+# (tg_ewald_table.cuh): ~510 instructions, mostly FMAs -> 950; contractions: M2L
+# 858, M2P 414, P2L 70 (direct kernels: the reference's constants).  PP_E pair
+# (tg_ewald_sep.cuh): squares 14, the nearest image 40, 3 of its 7 mirror
+# neighbours on average at 45 -> 190; the reciprocal terms are summed per source
+# leaf and evaluated per sink particle (not counted).
+NODE_FLOPS = {"CC_D": 1025, "CP_D": 455, "CC_E": 1810, "CP_E": 1020}
+LEAF_FLOPS = {"PC_D": 581, "PC_E": 1360, "PP_E": 190}
 # DRAM bytes per interaction of each kernel group, from ncu captures
 # (dram__bytes_read.sum + dram__bytes_write.sum over the capture's
-# interactions): k_pp_leaf and k_node_ewald on the 72^3 clustered box at
-# theta 0.19, leaf 48 (the clustered72 workload); k_ewald_chunk on the 128^3
-# clustered box at theta 0.3.  Scaled by this run's counts on the assumption
+# interactions) on the 72^3 clustered box at theta 0.19, leaf 48 (the
+# clustered72 workload); PP: an earlier kernel of the same reads (148 MB for
+# 3.2e10 pairs), leaf: k_ewald_pp.  Scaled by this run's counts on the assumption
 # that traffic grows with the interactions.
-TRAFFIC = {"pp": {"PP_D": 4.6e-3}, "nodes": {"CC_E": 2.65, "CP_E": 2.65}, "leaf": {"PP_E": 1.61, "PC_E": 1.61}}
+TRAFFIC = {"pp": {"PP_D": 4.6e-3}, "nodes": {"CC_E": 2.6, "CP_E": 2.6}, "leaf": {"PP_E": 0.127, "PC_E": 0.127}}
 TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum per interaction of a small capture, "
                   "scaled by this run's interaction counts")
 
@@ -514,9 +506,9 @@ def roofline(phase_ms, cnt, peak):
     achieved = executed FP32 operations (per-interaction counts from the
     kernel source, FMA = 2) / that kernel's CUDA-event phase time."""
     leaf_far = max(phase_ms["leaves"] - phase_ms.get("pp", 0.0), 1e-9)
-    kern = {"k_pp_leaf (PP direct)": (phase_ms.get("pp", 0.0), {"PP_D": PP_FLOPS}, "pp"),
+    kern = {"k_pp_long / k_pp_short (PP direct)": (phase_ms.get("pp", 0.0), {"PP_D": PP_FLOPS}, "pp"),
             "k_node + k_node_ewald<float> (CC/CP direct + Ewald)": (phase_ms["nodes"], NODE_FLOPS, "nodes"),
-            "k_ewald_chunk<float> + k_ewald_reduce + k_leaf (PC/PP Ewald, L2P, PC direct)":
+            "k_ewald_pp + k_ewald_pc + k_ewald_reduce + k_leaf (PC/PP Ewald, L2P, PC direct)":
                 (leaf_far, LEAF_FLOPS, "leaf")}
     name = max(kern, key=lambda k: kern[k][0])
     ms, fl, tk = kern[name]

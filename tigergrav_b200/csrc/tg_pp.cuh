@@ -2,8 +2,8 @@
  * tg_pp.cuh -- the packed FP32x2 pair arithmetic of PP direct
  * (gravity_PP_direct, src/gravity.cpp:171-300): two sources per packed
  * instruction (FADD2 / FMUL2 / FFMA2, sm_100), the sink replicated in both
- * halves.  The kernel that uses it is k_pp_leaf (tg_pp2.cuh).  Included by
- * tg_gravity.cu.
+ * halves.  The kernels that use it are k_pp_long and k_pp_short
+ * (tg_pp2.cuh).  Included by tg_gravity.cu.
  *
  * Coordinates are offsets from the sink leaf centre in units of 2^-32 of the
  * box, split by pp_split.  For a pair of sources staged as negated split
