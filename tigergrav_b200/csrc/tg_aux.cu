@@ -150,7 +150,7 @@ int ewald_tables(Solver &S, cudaStream_t st) {
         r2 += 4.0 * pi / 3.0 * w * h2;
     }
     if (sh.size() != nsep) return TG_ERR_STATE;
-    S.ew_sep_k = 3.141592653589793 / (alpha * alpha);
+    S.ew_sep_k = 3.141592653589793 / (alpha * alpha) + (S.prm.precision == TG_PREC_F32 ? SEP_OFFSET : 0.0);
     S.ew_sep_r0 = r0;
     S.ew_sep_r2 = r2;
     TG_TRY(ensure(S.ew_sep_h, nsep));
