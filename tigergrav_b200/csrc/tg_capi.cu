@@ -318,6 +318,7 @@ int tg_destroy(tg_solver *s) {
     release(S.pos); release(S.pos_alt); release(S.vel); release(S.vel_alt); release(S.acc); release(S.accd);
     release(S.keys); release(S.keys_alt); release(S.idx); release(S.idx_alt); release(S.cub_tmp);
     release(S.nd_pb); release(S.nd_pe); release(S.nd_child0); release(S.nd_parent); release(S.tb_out);
+    release(S.tb_flag); release(S.tb_scan);
     release(S.nd_key); release(S.nd_level); release(S.nd_ms); release(S.nd_r);
     release(S.nd_rmax); release(S.nd_aabb); release(S.nd_prange); release(S.nd_L); release(S.nd_Lloc);
     for (int k = 0; k < NLIST; k++) {
@@ -735,7 +736,7 @@ int tg_memory_report(tg_solver *s, char *buf, int64_t cap) {
 #define TG_MEM(b) add(#b, S.b.n * sizeof(*S.b.p))
     TG_MEM(pos); TG_MEM(pos_alt); TG_MEM(vel); TG_MEM(vel_alt); TG_MEM(acc); TG_MEM(accd); TG_MEM(keys);
     TG_MEM(keys_alt); TG_MEM(idx); TG_MEM(idx_alt); TG_MEM(cub_tmp); TG_MEM(nd_pb); TG_MEM(nd_pe); TG_MEM(nd_child0);
-    TG_MEM(nd_parent); TG_MEM(nd_key); TG_MEM(nd_level); TG_MEM(nd_ms);
+    TG_MEM(nd_parent); TG_MEM(tb_flag); TG_MEM(tb_scan); TG_MEM(nd_key); TG_MEM(nd_level); TG_MEM(nd_ms);
     TG_MEM(nd_r); TG_MEM(nd_rmax); TG_MEM(nd_aabb); TG_MEM(nd_prange); TG_MEM(nd_L); TG_MEM(nd_Lloc);
     TG_MEM(loff[0]); TG_MEM(llen[0]); TG_MEM(pool[0]); TG_MEM(pool[1]); TG_MEM(pool[2]); TG_MEM(pool[3]);
     TG_MEM(pool[4]); TG_MEM(pool[5]); TG_MEM(pool[6]); TG_MEM(pool[7]); TG_MEM(nxt_pool[0]); TG_MEM(nxt_pool[1]);

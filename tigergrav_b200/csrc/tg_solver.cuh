@@ -88,6 +88,7 @@ struct Solver {
     int depth = 0;
     DevBuf<int32_t> nd_pb, nd_pe, nd_child0, nd_parent;
     DevBuf<long long> tb_out; /* the tree build's level table and status */
+    DevBuf<int32_t> tb_flag, tb_scan; /* a wide level's nodes to split, and their exclusive scan */
     DevBuf<unsigned long long> nd_key;
     DevBuf<unsigned char> nd_level;
     DevBuf<MSrc> nd_ms;

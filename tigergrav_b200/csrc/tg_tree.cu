@@ -64,37 +64,68 @@ __global__ void k_gather(const int4 *__restrict__ pos, const float4 *__restrict_
     vel_out[i] = vel[j];
 }
 
+/* node i of level L gets its children q and q + 1, which stay leaves until their level is split */
+__device__ __forceinline__ void split_node(int64_t i, int64_t q, int L, const unsigned long long *__restrict__ keys,
+                                           int32_t *pb, int32_t *pe, int32_t *child0, int32_t *parent,
+                                           unsigned long long *nkey, unsigned char *level) {
+    const unsigned long long key = nkey[i], target = key | 1ull << (62 - L);
+    const int32_t b = pb[i], e = pe[i];
+    int32_t lo = b, hi = e;
+    while (lo < hi) { /* first key >= target */
+        const int32_t mid = lo + ((hi - lo) >> 1);
+        if (keys[mid] < target) lo = mid + 1;
+        else hi = mid;
+    }
+    child0[i] = (int32_t)q;
+    pb[q] = b;
+    pe[q] = lo;
+    pb[q + 1] = lo;
+    pe[q + 1] = e;
+    parent[q] = parent[q + 1] = (int32_t)i;
+    child0[q] = child0[q + 1] = -1;
+    nkey[q] = key;
+    nkey[q + 1] = target;
+    level[q] = level[q + 1] = (unsigned char)(L + 1);
+}
+
 /*
- * All levels of the tree in one launch: one cluster of TB_CTAS blocks, level by
- * level.  Block r takes the r-th of equal consecutive shares of a level's
- * nodes: it counts the nodes to split, learns the counts of the blocks before
- * it through distributed shared memory, and writes the children of its nodes in
- * node order, so ids equal those of one pass per level.  The cluster's hardware
- * barrier separates the levels.
+ * Levels of up to TB_WIDE nodes, any number of them in one launch: one cluster of
+ * TB_CTAS blocks, level by level.  Block r takes the r-th of equal consecutive
+ * shares of a level's nodes: it counts the nodes to split, learns the counts of
+ * the blocks before it through distributed shared memory, and writes the children
+ * of its nodes in node order, so ids equal those of one pass per level.  The
+ * cluster's hardware barrier separates the levels.  Wider levels go to k_flag, a
+ * scan and k_split on the whole GPU, one level at a time.
  *
  * What bounds it: latency, one barrier pair and one binary search (log2 n
- * dependent loads) per level and wave of 8192 nodes.  A launch per level with
- * its scan and a host round trip for the count took 45 us per level whatever
- * the size (build, with the sort: 0.37 -> 0.16 ms at 4096 particles, 0.48 -> 0.20 at
- * 32768, 1.00 -> 0.55 at 128^3, 2.76 -> 2.68 at 256^3).
+ * dependent loads) per level and wave of 8192 nodes.  A pass of its own with its
+ * scan and a host round trip for the count takes 45 us per level whatever the
+ * size (build, with the sort: 0.37 -> 0.16 ms at 4096 particles, 0.48 -> 0.20 at
+ * 32768, 1.00 -> 0.55 at 128^3, leaf 64), the cluster 0.38 ns per node against
+ * 0.04, so they meet at 1.3e5 nodes.  Build of 256^3 with leaf 4 / 16 / 48 (9.4e6,
+ * 2.6e6, 1.0e6 nodes): all levels in the cluster 5.86 / 3.36 / 2.68 ms, each in a
+ * pass of its own 3.15 / 2.92 / 2.83, by width 2.86 / 2.62 / 2.48 (TB_WIDE 65536:
+ * 2.86 / 2.57 / 2.44 and 128^3 leaf 16 0.69 for 0.66; 262144: 2.98 / 2.73 / 2.59).
  *
- * out: level_off[TB_LEVELS + 2], level_leaves[TB_LEVELS + 1], then (depth,
- * status, nodes needed): status 0 done, 1 the node arrays hold fewer than the
- * nodes needed (start again with more), 2 too deep.
+ * out: level_off[TB_LEVELS + 2], level_leaves[TB_LEVELS + 1], written from level
+ * L0 on, then (level, status, nodes needed): status 0 done, 1 the node arrays hold
+ * fewer than the nodes needed (start again with more), 2 too deep, 3 `level` is
+ * wider than TB_WIDE.
  */
 constexpr int TB_CTAS = 8, TB_THREADS = 1024;
 constexpr int TB_LEVELS = 63;
 constexpr int TB_OUT = 2 * TB_LEVELS + 3 + 3;
+constexpr int64_t TB_WIDE = 131072;
 
 __global__ void __cluster_dims__(TB_CTAS, 1, 1) __launch_bounds__(TB_THREADS, 1)
-    k_tree_levels(int64_t n, int leaf_max, int64_t cap, const unsigned long long *__restrict__ keys, int32_t *pb,
-                  int32_t *pe, int32_t *child0, int32_t *parent, unsigned long long *nkey, unsigned char *level,
-                  long long *__restrict__ out) {
+    k_tree_levels(int64_t n, int leaf_max, int64_t cap, int L0, int64_t first, int64_t next,
+                  const unsigned long long *__restrict__ keys, int32_t *pb, int32_t *pe, int32_t *child0,
+                  int32_t *parent, unsigned long long *nkey, unsigned char *level, long long *__restrict__ out) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     __shared__ int32_t s_warp[32], s_total, s_counts[2][TB_CTAS];
     const int r = (int)cl.block_rank(), t = threadIdx.x, lane = t & 31, w = t >> 5;
-    if (r == 0 && t == 0) {
+    if (L0 == 0 && r == 0 && t == 0) {
         pb[0] = 0;
         pe[0] = (int32_t)n;
         child0[0] = -1;
@@ -105,10 +136,13 @@ __global__ void __cluster_dims__(TB_CTAS, 1, 1) __launch_bounds__(TB_THREADS, 1)
         out[1] = 1;
     }
     cl.sync();
-    int64_t first = 0, next = 1;
-    int L = 0;
+    int L = L0;
     long long status = 0;
     for (;; L++) {
+        if (next - first > TB_WIDE) {
+            status = 3;
+            break;
+        }
         const int64_t count = next - first, share = (count + TB_CTAS - 1) / TB_CTAS;
         const int64_t k0 = min(count, share * r), k1 = min(count, share * (r + 1));
         /* this block's nodes to split */
@@ -139,7 +173,6 @@ __global__ void __cluster_dims__(TB_CTAS, 1, 1) __launch_bounds__(TB_THREADS, 1)
             next = need;
             break;
         }
-        const unsigned long long bit = 1ull << (62 - L);
         for (int64_t base = k0; base < k1; base += TB_THREADS) { /* windows in node order */
             const int64_t i = first + base + t;
             int32_t b = 0, e = 0;
@@ -162,24 +195,8 @@ __global__ void __cluster_dims__(TB_CTAS, 1, 1) __launch_bounds__(TB_THREADS, 1)
             }
             __syncthreads();
             if (split) {
-                const unsigned long long key = nkey[i], target = key | bit;
-                int32_t lo = b, hi = e;
-                while (lo < hi) { /* first key >= target */
-                    const int32_t mid = lo + ((hi - lo) >> 1);
-                    if (keys[mid] < target) lo = mid + 1;
-                    else hi = mid;
-                }
-                const int64_t q = next + 2 * (before + s_warp[w] + __popc(m & ((1u << lane) - 1u)));
-                child0[i] = (int32_t)q;
-                pb[q] = b;
-                pe[q] = lo;
-                pb[q + 1] = lo;
-                pe[q + 1] = e;
-                parent[q] = parent[q + 1] = (int32_t)i;
-                child0[q] = child0[q + 1] = -1;
-                nkey[q] = key;
-                nkey[q + 1] = target;
-                level[q] = level[q + 1] = (unsigned char)(L + 1);
+                split_node(i, next + 2 * (before + s_warp[w] + __popc(m & ((1u << lane) - 1u))), L, keys, pb, pe, child0,
+                           parent, nkey, level);
             }
             before += s_total;
         }
@@ -196,6 +213,21 @@ __global__ void __cluster_dims__(TB_CTAS, 1, 1) __launch_bounds__(TB_THREADS, 1)
     cl.sync(); /* no block leaves while its shared memory may be written */
 }
 
+__global__ void k_flag(int64_t first, int64_t count, const int32_t *__restrict__ pb, const int32_t *__restrict__ pe,
+                       int leaf_max, int32_t *__restrict__ flag) {
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k > count) return;
+    flag[k] = k < count && pe[first + k] - pb[first + k] > leaf_max; /* flag[count] = 0: the scan ends in the total */
+}
+
+__global__ void k_split(int64_t first, int64_t count, int64_t next, int L, const int32_t *__restrict__ flag,
+                        const int32_t *__restrict__ scan, const unsigned long long *__restrict__ keys, int32_t *pb,
+                        int32_t *pe, int32_t *child0, int32_t *parent, unsigned long long *nkey, unsigned char *level) {
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= count || !flag[k]) return;
+    split_node(first + k, next + 2 * (int64_t)scan[k], L, keys, pb, pe, child0, parent, nkey, level);
+}
+
 static int grow_nodes(Solver &S, size_t need) {
     TG_TRY(ensure(S.nd_pb, need));
     TG_TRY(ensure(S.nd_pe, need));
@@ -203,6 +235,53 @@ static int grow_nodes(Solver &S, size_t need) {
     TG_TRY(ensure(S.nd_parent, need));
     TG_TRY(ensure(S.nd_key, need));
     TG_TRY(ensure(S.nd_level, need));
+    return TG_OK;
+}
+
+/* Levels L on (nodes [first, next)) in the cluster kernel, to the first wide one,
+ * which L then is, or to the last.  status, and need for status 1, as k_tree_levels. */
+static int split_narrow_levels(Solver &S, int &L, int64_t first, int64_t next, size_t &need, long long &status,
+                               cudaStream_t st) {
+    long long out[TB_OUT];
+    static_assert(sizeof(out) <= 2048, "one small readback");
+    k_tree_levels<<<TB_CTAS, TB_THREADS, 0, st>>>(S.n, S.prm.leaf_max, (int64_t)need, L, first, next, S.keys.p, S.nd_pb.p,
+                                                  S.nd_pe.p, S.nd_child0.p, S.nd_parent.p, S.nd_key.p, S.nd_level.p,
+                                                  S.tb_out.p);
+    TG_TRY(launched(S));
+    TG_TRY(read_small(S, st, out, S.tb_out.p, sizeof(out)));
+    status = out[TB_OUT - 2];
+    if (status == 1) need = 2 * (size_t)out[TB_OUT - 1];
+    const int end = (int)out[TB_OUT - 3];
+    S.level_off.insert(S.level_off.end(), out + L + 2, out + end + 2);
+    S.level_leaves.insert(S.level_leaves.end(), out + TB_LEVELS + 2 + L, out + TB_LEVELS + 2 + end + (status == 0));
+    L = end;
+    return TG_OK;
+}
+
+/* level L alone, on the whole GPU: status 4 (go on), or 1 and 2 as k_tree_levels; 0 where it holds no node to split */
+static int split_wide_level(Solver &S, int L, int64_t first, int64_t next, size_t &need, long long &status,
+                            cudaStream_t st) {
+    const int64_t count = next - first;
+    const int TPB = 256, g = (int)((count + TPB) / TPB);
+    TG_TRY(ensure(S.tb_flag, (size_t)count + 1));
+    TG_TRY(ensure(S.tb_scan, (size_t)count + 1));
+    k_flag<<<g, TPB, 0, st>>>(first, count, S.nd_pb.p, S.nd_pe.p, S.prm.leaf_max, S.tb_flag.p);
+    TG_TRY(launched(S));
+    size_t tmp = 0;
+    TG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp, S.tb_flag.p, S.tb_scan.p, (int)count + 1, st));
+    TG_TRY(ensure(S.cub_tmp, tmp));
+    TG_CUDA(cub::DeviceScan::ExclusiveSum(S.cub_tmp.p, tmp, S.tb_flag.p, S.tb_scan.p, (int)count + 1, st));
+    int32_t nsplit = 0;
+    TG_TRY(read_small(S, st, &nsplit, S.tb_scan.p + count, sizeof(nsplit)));
+    S.level_leaves.push_back(count - nsplit);
+    const int64_t end = next + 2 * (int64_t)nsplit;
+    status = nsplit == 0 ? 0 : (L >= TB_LEVELS ? 2 : ((size_t)end > need ? 1 : 4));
+    if (status == 1) need = 2 * (size_t)end;
+    if (status != 4) return TG_OK;
+    k_split<<<g, TPB, 0, st>>>(first, count, next, L, S.tb_flag.p, S.tb_scan.p, S.keys.p, S.nd_pb.p, S.nd_pe.p,
+                               S.nd_child0.p, S.nd_parent.p, S.nd_key.p, S.nd_level.p);
+    TG_TRY(launched(S));
+    S.level_off.push_back(end);
     return TG_OK;
 }
 
@@ -232,22 +311,24 @@ int tree_build(Solver &S, cudaStream_t st) {
 
     size_t need = std::max(S.nd_pb.n, (size_t)(4 * n / (S.prm.leaf_max > 0 ? S.prm.leaf_max : 1) + 1024));
     TG_TRY(ensure(S.tb_out, TB_OUT));
-    long long out[TB_OUT];
-    static_assert(sizeof(out) <= 2048, "one small readback");
-    for (;;) {
-        TG_TRY(grow_nodes(S, need));
-        k_tree_levels<<<TB_CTAS, TB_THREADS, 0, st>>>(n, S.prm.leaf_max, (int64_t)need, S.keys.p, S.nd_pb.p, S.nd_pe.p,
-                                                      S.nd_child0.p, S.nd_parent.p, S.nd_key.p, S.nd_level.p,
-                                                      S.tb_out.p);
-        TG_TRY(launched(S));
-        TG_TRY(read_small(S, st, out, S.tb_out.p, sizeof(out)));
-        if (out[TB_OUT - 2] == 2) return TG_ERR_DEPTH;
-        if (out[TB_OUT - 2] == 0) break;
-        need = 2 * (size_t)out[TB_OUT - 1];
+    int L = 0;
+    for (long long status = 1; status != 0;) {
+        if (status == 1) { /* (again) from the root */
+            TG_TRY(grow_nodes(S, need));
+            L = 0;
+            S.level_off.assign({0, 1});
+            S.level_leaves.clear();
+        }
+        const int64_t first = S.level_off[L], next = S.level_off[L + 1];
+        if (status == 3) {
+            TG_TRY(split_wide_level(S, L, first, next, need, status, st));
+            if (status == 4) L++;
+        } else {
+            TG_TRY(split_narrow_levels(S, L, first, next, need, status, st));
+        }
+        if (status == 2) return TG_ERR_DEPTH;
     }
-    S.depth = (int)out[TB_OUT - 3];
-    S.level_off.assign(out, out + S.depth + 2);
-    S.level_leaves.assign(out + TB_LEVELS + 2, out + TB_LEVELS + 2 + S.depth + 1);
+    S.depth = L;
     S.nnodes = S.level_off.back();
     S.have_tree = true;
     S.fof_link = 0.0;
