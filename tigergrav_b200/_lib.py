@@ -55,7 +55,7 @@ class tg_stats(C.Structure):
 # every symbol the header declares (checked by the CPU test suite)
 EXPORTS = [
     "tg_error_string", "tg_version", "tg_create", "tg_destroy", "tg_set_particles", "tg_get_particles",
-    "tg_build", "tg_multipoles", "tg_walk", "tg_set_walk_capacity", "tg_forces", "tg_solve_gravity", "tg_get_forces",
+    "tg_build", "tg_multipoles", "tg_walk", "tg_set_walk_capacity", "tg_set_ewald_scratch", "tg_forces", "tg_solve_gravity", "tg_get_forces",
     "tg_get_forces_f64", "tg_kick", "tg_drift", "tg_kick_drift", "tg_energy", "tg_leapfrog", "tg_get_stats", "tg_memory_report",
     "tg_num_nodes",
     "tg_get_nodes", "tg_get_perm", "tg_list_size", "tg_get_list", "tg_gravity_PP_direct",
@@ -92,6 +92,7 @@ def _load():
     for f in ("tg_build", "tg_multipoles", "tg_walk", "tg_forces", "tg_solve_gravity"):
         getattr(L, f).argtypes = [vp, vp]
     L.tg_set_walk_capacity.argtypes = [vp, i64]
+    L.tg_set_ewald_scratch.argtypes = [vp, i64]
     L.tg_get_forces.argtypes = [vp, vp, vp, i32, vp]
     L.tg_get_forces_f64.argtypes = [vp, vp, vp, i32, vp]
     L.tg_kick.argtypes = [vp, d, vp]

@@ -407,14 +407,23 @@ __global__ void __launch_bounds__(128) k_tidal_pp(GParams P, const int32_t *__re
 template <class T> struct Sep4 {
     T c, s, uc, us;
 };
+template <> __device__ __forceinline__ Sep4<float> sep_zero<Sep4<float>>() { return {0.0f, 0.0f, 0.0f, 0.0f}; }
+template <> __device__ __forceinline__ Sep4<double> sep_zero<Sep4<double>>() { return {0.0, 0.0, 0.0, 0.0}; }
+template <class T> __device__ __forceinline__ void sep_madd(Sep4<T> &a, T m, const Sep4<T> &f) {
+    a.c = fma(m, f.c, a.c);
+    a.s = fma(m, f.s, a.s);
+    a.uc = fma(m, f.uc, a.uc);
+    a.us = fma(m, f.us, a.us);
+}
 
 template <class T>
 __global__ void __launch_bounds__(128) k_tidal_sf(const int32_t *__restrict__ src, const int32_t *__restrict__ pb,
                                                   const int32_t *__restrict__ pe, const int4 *__restrict__ pos,
-                                                  const double *__restrict__ u, EwaldTables E, Sep4<T> *__restrict__ sf) {
+                                                  const double *__restrict__ u, EwaldTables E, int t0, int t1,
+                                                  Sep4<T> *__restrict__ sf) {
     const int32_t node = src[blockIdx.x];
     const int32_t b = pb[node], e = pe[node];
-    for (int t = threadIdx.x; t < Sep<T>::N; t += 128) {
+    for (int t = t0 + threadIdx.x; t < t1; t += 128) {
         const int4 h = __ldg(&E.sep_h[t]);
         Sep4<T> a{T(0), T(0), T(0), T(0)};
         for (int32_t j = b; j < e; j++) {
@@ -426,7 +435,7 @@ __global__ void __launch_bounds__(128) k_tidal_sf(const int32_t *__restrict__ sr
             a.uc = fma(hu, q.x, a.uc);
             a.us = fma(hu, q.y, a.us);
         }
-        sf[(int64_t)blockIdx.x * Sep<T>::N + t] = a;
+        sf[(int64_t)blockIdx.x * (t1 - t0) + t - t0] = a;
     }
 }
 
@@ -501,10 +510,10 @@ __device__ __forceinline__ void tidal_ewald_pair(const EwaldTables &E, const T *
 }
 
 /* one chunk of a PP_E list (as k_ewald_pp): the real-space part per pair into
- * part (3 per sink), the reciprocal source sums into tpart */
+ * part (3 per sink) and, with sf, the reciprocal source sums into tpart */
 template <class T>
 __global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, bool fine, const int32_t *__restrict__ leaves, int32_t nleaves,
-                                                       const int32_t *__restrict__ off, const int32_t *__restrict__ pb,
+                                                       int32_t first, const int32_t *__restrict__ off, const int32_t *__restrict__ pb,
                                                        const int32_t *__restrict__ pe, const int4 *__restrict__ pos,
                                                        ListView LV, EwaldTables E, const double *__restrict__ u,
                                                        double *__restrict__ part, const int32_t *__restrict__ slot,
@@ -513,7 +522,7 @@ __global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, bool fine, con
     __shared__ T su[64][3];
     __shared__ int32_t s_row[EW_KPP_MAX];
     const int tid = threadIdx.x;
-    const int64_t c = blockIdx.x;
+    const int64_t c = (int64_t)first + blockIdx.x;
     const int32_t li = ew_leaf(off, nleaves, c), k = (int32_t)(c - off[li]);
     const int32_t leaf = leaves[li];
     const int32_t b = pb[leaf], cnt = pe[leaf] - b;
@@ -547,26 +556,15 @@ __global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, bool fine, con
             }
     }
     if (tid < cnt)
-        for (int d = 0; d < 3; d++) part[3 * (c * 64 + tid) + d] = o[d].get();
-    for (int t = tid; t < Sep<T>::N; t += 64) {
-        Sep4<T> a{T(0), T(0), T(0), T(0)};
-#pragma unroll 4
-        for (int q = 0; q < e1 - e0; q++) {
-            const Sep4<T> f = sf[(int64_t)s_row[q] * Sep<T>::N + t];
-            a.c = fma(m, f.c, a.c);
-            a.s = fma(m, f.s, a.s);
-            a.uc = fma(m, f.uc, a.uc);
-            a.us = fma(m, f.us, a.us);
-        }
-        tpart[c * Sep<T>::N + t] = a;
-    }
+        for (int d = 0; d < 3; d++) part[3 * ((int64_t)blockIdx.x * 64 + tid) + d] = o[d].get();
+    if (sf) ew_tsum<T, Sep4<T>>(s_row, e1 - e0, 0, Sep<T>::N, tid, sf, m, tpart + (int64_t)blockIdx.x * Sep<T>::N);
 }
 
 /* out += the chunk sums of each leaf, in chunk order, and the reciprocal part
  * -sum_h 4 pi w_h h ((h.u_i) cos(th_i - th_j) - (h.u_j) cos(th_i - th_j)) from
- * the chunks' source sums.  One block per leaf, four threads per sink. */
+ * the chunks' source sums.  One block per leaf of the batch, four threads per sink. */
 template <class T>
-__global__ void __launch_bounds__(256) k_tidal_ewald_reduce(const int32_t *__restrict__ leaves,
+__global__ void __launch_bounds__(256) k_tidal_ewald_reduce(EwBatch B, const int32_t *__restrict__ leaves,
                                                             const int32_t *__restrict__ off,
                                                             const int32_t *__restrict__ pb, const int32_t *__restrict__ pe,
                                                             const int4 *__restrict__ pos, EwaldTables E,
@@ -575,9 +573,9 @@ __global__ void __launch_bounds__(256) k_tidal_ewald_reduce(const int32_t *__res
     constexpr int TILE = 384; /* vectors whose sums are held at a time */
     __shared__ double4 sT[TILE];
     __shared__ double sv[4][64][3];
-    const int32_t li = blockIdx.x;
+    const int32_t li = B.l0 + blockIdx.x;
     const int tid = threadIdx.x, t = tid & 63, grp = tid >> 6;
-    const int32_t a0 = off[li], a1 = off[li + 1];
+    const int32_t a0 = off[li] - B.a0, a1 = off[li + 1] - B.a0;
     if (a1 == a0) return; /* block-uniform */
     const int32_t leaf = leaves[li];
     const int32_t b = pb[leaf], cnt = pe[leaf] - b;
@@ -631,18 +629,39 @@ static int tidal_ewald(Solver &S, const GParams &P, const ListView &LV, const Ew
     int32_t npp = 0, total = 0, nsrc = 0;
     TG_TRY(leaf_chunks(S, LV, npp, total, nsrc, st));
     if (npp <= 0) return TG_OK;
-    TG_TRY(ensure(S.ew_part, (size_t)npp * 64 * 3));
-    TG_TRY(ensure(S.ew_sf, (size_t)nsrc * Sep<T>::N * sizeof(Sep4<T>)));
-    TG_TRY(ensure(S.ew_tpart, (size_t)npp * Sep<T>::N * sizeof(Sep4<T>)));
-    Sep4<T> *sf = reinterpret_cast<Sep4<T> *>(S.ew_sf.p), *tpart = reinterpret_cast<Sep4<T> *>(S.ew_tpart.p);
-    k_tidal_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, S.tid_u.p, E, sf);
-    TG_TRY(launched(S));
-    k_tidal_ewald_pp<T><<<npp, 64, 0, st>>>(P, ew_fine(S), S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, E,
-                                            S.tid_u.p, S.ew_part.p, S.ew_slot.p, sf, tpart);
-    TG_TRY(launched(S));
-    k_tidal_ewald_reduce<T><<<nleaves, 256, 0, st>>>(S.idx.p, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E, S.tid_u.p,
-                                                    S.ew_part.p, tpart, S.tid_o.p);
-    TG_TRY(launched(S));
+    typedef Sep4<T> T4;
+    constexpr int N = Sep<T>::N;
+    std::vector<EwBatch> batches;
+    TG_TRY(leaf_batches(S, npp, npp, 192 * sizeof(double) + N * sizeof(T4), 0, batches, st));
+    size_t slots = 0;
+    for (const EwBatch &B : batches) slots = std::max(slots, (size_t)B.na);
+    const int nv = ew_vectors(S, nsrc, sizeof(T4), N);
+    TG_TRY(ensure(S.ew_part, slots * 64 * 3));
+    TG_TRY(ensure(S.ew_sf, (size_t)nsrc * nv * sizeof(T4)));
+    TG_TRY(ensure(S.ew_tpart, slots * N * sizeof(T4)));
+    T4 *sf = reinterpret_cast<T4 *>(S.ew_sf.p), *tpart = reinterpret_cast<T4 *>(S.ew_tpart.p);
+    const bool fine = ew_fine(S);
+    if (nv == N) {
+        k_tidal_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, S.tid_u.p, E, 0, N, sf);
+        TG_TRY(launched(S));
+    }
+    for (const EwBatch &B : batches) {
+        if (B.na == 0) continue;
+        k_tidal_ewald_pp<T><<<B.na, 64, 0, st>>>(P, fine, S.idx.p, nleaves, B.a0, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p,
+                                                 LV, E, S.tid_u.p, S.ew_part.p, S.ew_slot.p, nv == N ? sf : nullptr, tpart);
+        TG_TRY(launched(S));
+        for (int t0 = 0; nv < N && t0 < N; t0 += nv) {
+            const int t1 = std::min(N, t0 + nv);
+            k_tidal_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, S.tid_u.p, E, t0, t1, sf);
+            TG_TRY(launched(S));
+            k_ewald_tsum<T, T4><<<B.na, 64, 0, st>>>(T(P.m_d), fine, S.idx.p, nleaves, B.a0, S.ew_off.p, LV, S.ew_slot.p,
+                                                     t0, t1, sf, tpart);
+            TG_TRY(launched(S));
+        }
+        k_tidal_ewald_reduce<T><<<B.l1 - B.l0, 256, 0, st>>>(B, S.idx.p, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E,
+                                                             S.tid_u.p, S.ew_part.p, tpart, S.tid_o.p);
+        TG_TRY(launched(S));
+    }
     return TG_OK;
 }
 

@@ -458,6 +458,13 @@ int tg_set_walk_capacity(tg_solver *s, int64_t entries) {
     return TG_OK;
 }
 
+int tg_set_ewald_scratch(tg_solver *s, int64_t bytes) {
+    CHECK_HANDLE(s);
+    if (bytes < 0) return TG_ERR_ARG;
+    s->S.ew_scratch = bytes > 0 ? (size_t)bytes : tg::EW_SCRATCH;
+    return TG_OK;
+}
+
 int tg_forces(tg_solver *s, void *stream) {
     CHECK_HANDLE(s);
     return gravity_forces(s->S, STREAM(stream));

@@ -16,6 +16,13 @@
  * scheduling.  Chunks are numbered PP_E first, then PC_E: off[0, nleaves] is
  * the scan of the leaves' PP_E chunk counts, off[nleaves + 1, 2 nleaves + 1]
  * that of their PC_E counts continued.
+ *
+ * A PP_E chunk's slots take 2 KB and its source sums 3 KB in FP32 and 20 KB in
+ * FP64 (the Jacobian's 6 and 40 KB), and where every pair is an Ewald pair the
+ * chunks grow with the square of the leaves.  So the leaves run in batches whose
+ * chunks fit EW_SCRATCH, each reduced before the next (leaf_batches), and where
+ * the source leaves' own sums do not fit it, they are made for a range of vectors
+ * at a time (k_ewald_tsum).  Neither changes the order of any sum.
  */
 #pragma once
 
@@ -31,6 +38,12 @@ __host__ __device__ __forceinline__ int32_t ew_kpp(int32_t len, bool fine) {
     return k < lo ? lo : (k > EW_KPP_MAX ? EW_KPP_MAX : k);
 }
 constexpr int EW_KPC = 64; /* PC_E source nodes per chunk */
+
+/* leaves [l0, l1) with their PP_E chunks [a0, a0 + na) and PC_E chunks [c0, c0 + nc),
+ * whose slots follow each other in that order */
+struct EwBatch {
+    int32_t l0, l1, a0, na, c0, nc;
+};
 
 /* one warp per leaf: chunk counts (zeros at li = nleaves, so that the scan ends
  * in the totals); with slot, marks the source leaves of the PP_E lists */
@@ -83,11 +96,42 @@ __device__ __forceinline__ int32_t ew_leaf(const int32_t *__restrict__ off, int3
     return lo;
 }
 
+/* the source sums of a chunk (rows of sf, one per source leaf, holding vectors [t0, t1)) into its row of tpart */
+template <class T, class S>
+__device__ __forceinline__ void ew_tsum(const int32_t *s_row, int n, int t0, int t1, int tid, const S *__restrict__ sf,
+                                        T m, S *__restrict__ out) {
+    for (int t = t0 + tid; t < t1; t += 64) {
+        S a = sep_zero<S>();
+#pragma unroll 8
+        for (int u = 0; u < n; u++) sep_madd(a, m, sf[(int64_t)s_row[u] * (t1 - t0) + t - t0]);
+        out[t] = a;
+    }
+}
+/* the same in a launch of its own, for the chunks from `first` on */
+template <class T, class S>
+__global__ void __launch_bounds__(64) k_ewald_tsum(T m, bool fine, const int32_t *__restrict__ leaves, int32_t nleaves,
+                                                   int32_t first, const int32_t *__restrict__ off, ListView LV,
+                                                   const int32_t *__restrict__ slot, int t0, int t1,
+                                                   const S *__restrict__ sf, S *__restrict__ tpart) {
+    __shared__ int32_t s_row[EW_KPP_MAX];
+    const int tid = threadIdx.x;
+    const int64_t c = (int64_t)first + blockIdx.x;
+    const int32_t li = ew_leaf(off, nleaves, c), k = (int32_t)(c - off[li]);
+    const int32_t leaf = leaves[li];
+    const int32_t *lst = LV.pool[TG_PP_E] + LV.off[TG_PP_E][leaf];
+    const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len, fine), e0 = k * kpp, e1 = min(len, e0 + kpp);
+    if (tid < e1 - e0) s_row[tid] = slot[lst[e0 + tid]];
+    __syncthreads();
+    ew_tsum<T, S>(s_row, e1 - e0, t0, t1, tid, sf, m, tpart + (int64_t)blockIdx.x * Sep<T>::N);
+}
+
 /* one chunk of a PP_E list: entries [k ew_kpp, ...) of its leaf.  The
- * real-space part per pair and the chunk's reciprocal source sums (tpart). */
+ * real-space part per pair and, with sf (all vectors), the chunk's reciprocal
+ * source sums (tpart).  Block b takes chunk first + b, its slot is b. */
 template <class T>
 __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
-    k_ewald_pp(GParams P, bool fine, const int32_t *__restrict__ leaves, int32_t nleaves, const int32_t *__restrict__ off,
+    k_ewald_pp(GParams P, bool fine, const int32_t *__restrict__ leaves, int32_t nleaves, int32_t first,
+               const int32_t *__restrict__ off,
                const int32_t *__restrict__ pb, const int32_t *__restrict__ pe, const int4 *__restrict__ pos, ListView LV,
                EwaldTables E, double *__restrict__ part, const int32_t *__restrict__ slot,
                const typename Sep<T>::T2 *__restrict__ sf, typename Sep<T>::T2 *__restrict__ tpart) {
@@ -95,7 +139,7 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
     __shared__ int4 sy[64];
     __shared__ int32_t s_row[EW_KPP_MAX];
     const int tid = threadIdx.x;
-    const int64_t c = blockIdx.x;
+    const int64_t c = (int64_t)first + blockIdx.x;
     const int32_t li = ew_leaf(off, nleaves, c), k = (int32_t)(c - off[li]);
     const int32_t leaf = leaves[li];
     const int32_t b = pb[leaf], cnt = pe[leaf] - b;
@@ -125,28 +169,19 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
             }
     }
     if (active) {
-        double *o = part + 4 * (c * 64 + tid);
+        double *o = part + 4 * ((int64_t)blockIdx.x * 64 + tid);
         o[0] = aphi.get();
         for (int d = 0; d < 3; d++) o[1 + d] = ag[d].get();
     }
     /* this chunk's reciprocal source sums, a thread per vector (s_row: written before the loop's barriers) */
-    for (int t = tid; t < Sep<T>::N; t += 64) {
-        T2 a;
-        a.x = a.y = T(0);
-#pragma unroll 8
-        for (int u = 0; u < e1 - e0; u++) {
-            const T2 f = sf[(int64_t)s_row[u] * Sep<T>::N + t];
-            a.x = fma(m, f.x, a.x);
-            a.y = fma(m, f.y, a.y);
-        }
-        tpart[c * Sep<T>::N + t] = a;
-    }
+    if (sf) ew_tsum<T, T2>(s_row, e1 - e0, 0, Sep<T>::N, tid, sf, m, tpart + (int64_t)blockIdx.x * Sep<T>::N);
 }
 
-/* one chunk of a PC_E list: chunk c counts on from the PP_E chunks (offp: its leaves' scan) */
+/* one chunk of a PC_E list: block b takes chunk first + b (offp: the PC_E part of the scan), its slot is slot0 + b */
 template <class T>
 __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 8 : 6)
-    k_ewald_pc(const int32_t *__restrict__ leaves, int32_t nleaves, int32_t first, const int32_t *__restrict__ offp,
+    k_ewald_pc(const int32_t *__restrict__ leaves, int32_t nleaves, int32_t first, int32_t slot0,
+               const int32_t *__restrict__ offp,
                const int32_t *__restrict__ pb, const int32_t *__restrict__ pe, const MSrc *__restrict__ ms,
                const int4 *__restrict__ pos, ListView LV, EwaldTables E, double *__restrict__ part) {
     const int tid = threadIdx.x;
@@ -175,17 +210,17 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 8 : 6)
         aphi.add(ph);
         for (int d = 0; d < 3; d++) ag[d].add(g[d]);
     }
-    double *o = part + 4 * (c * 64 + tid);
+    double *o = part + 4 * ((int64_t)(slot0 + blockIdx.x) * 64 + tid);
     o[0] = aphi.get();
     for (int d = 0; d < 3; d++) o[1 + d] = ag[d].get();
 }
 
 /* Add each leaf's chunk sums, in chunk order, to its FP64 accumulators, and
  * the reciprocal part from the PP_E chunks' source sums (in chunk
- * order).  One block per leaf; the four groups of 64 threads take a quarter
- * of the vectors each. */
+ * order).  One block per leaf of the batch; the four groups of 64 threads take a
+ * quarter of the vectors each. */
 template <class T>
-__global__ void __launch_bounds__(256) k_ewald_reduce(const int32_t *__restrict__ leaves, int32_t nleaves,
+__global__ void __launch_bounds__(256) k_ewald_reduce(EwBatch B, const int32_t *__restrict__ leaves, int32_t nleaves,
                                                       const int32_t *__restrict__ off, const int32_t *__restrict__ pb,
                                                       const int32_t *__restrict__ pe, const double *__restrict__ part,
                                                       double *__restrict__ acc,
@@ -193,10 +228,11 @@ __global__ void __launch_bounds__(256) k_ewald_reduce(const int32_t *__restrict_
                                                       const int4 *__restrict__ pos, EwaldTables E) {
     __shared__ double2 sT[Sep<T>::N];
     __shared__ double sv[4][64][4];
-    const int32_t li = blockIdx.x;
+    const int32_t li = B.l0 + blockIdx.x;
     const int tid = threadIdx.x, t = tid & 63, grp = tid >> 6;
     const int32_t *offp = off + nleaves + 1;
-    const int32_t a0 = off[li], a1 = off[li + 1], p0 = offp[li], p1 = offp[li + 1];
+    const int32_t a0 = off[li] - B.a0, a1 = off[li + 1] - B.a0; /* the leaf's slots */
+    const int32_t p0 = offp[li] - B.c0 + B.na, p1 = offp[li + 1] - B.c0 + B.na;
     if (a1 == a0 && p1 == p0) return; /* block-uniform */
     const int32_t leaf = leaves[li];
     const int32_t b = pb[leaf], cnt = pe[leaf] - b;

@@ -42,15 +42,25 @@ __device__ __forceinline__ typename Sep<T>::T2 sep_cs(int32_t x0, int32_t x1, in
     return cs;
 }
 
+/* source sums: zero, and a += m f */
+template <class S> __device__ __forceinline__ S sep_zero();
+template <> __device__ __forceinline__ float2 sep_zero<float2>() { return make_float2(0.0f, 0.0f); }
+template <> __device__ __forceinline__ double2 sep_zero<double2>() { return make_double2(0.0, 0.0); }
+template <class T, class S> __device__ __forceinline__ void sep_madd(S &a, T m, const S &f) {
+    a.x = fma(m, f.x, a.x);
+    a.y = fma(m, f.y, a.y);
+}
+
 /* One block per source leaf of some PP_E list: the sums of (cos, sin) over its
- * particles, a thread per vector */
+ * particles, a thread per vector of [t0, t1) */
 template <class T>
 __global__ void __launch_bounds__(128) k_ewald_sf(const int32_t *__restrict__ src, const int32_t *__restrict__ pb,
                                                   const int32_t *__restrict__ pe, const int4 *__restrict__ pos,
-                                                  EwaldTables E, typename Sep<T>::T2 *__restrict__ sf) {
+                                                  EwaldTables E, int t0, int t1,
+                                                  typename Sep<T>::T2 *__restrict__ sf) {
     const int32_t node = src[blockIdx.x];
     const int32_t b = pb[node], e = pe[node];
-    for (int t = threadIdx.x; t < Sep<T>::N; t += 128) {
+    for (int t = t0 + threadIdx.x; t < t1; t += 128) {
         const int4 h = __ldg(&E.sep_h[t]);
         typename Sep<T>::T2 a;
         a.x = a.y = T(0);
@@ -60,7 +70,7 @@ __global__ void __launch_bounds__(128) k_ewald_sf(const int32_t *__restrict__ sr
             a.x += q.x;
             a.y += q.y;
         }
-        sf[(int64_t)blockIdx.x * Sep<T>::N + t] = a;
+        sf[(int64_t)blockIdx.x * (t1 - t0) + t - t0] = a;
     }
 }
 

@@ -21,7 +21,9 @@
  * sums folded into Kahan-compensated accumulators) or T = double (the plain
  * FP64 port).  Expansions L are FP64 in both.
  */
+#include <memory>
 #include <mutex>
+#include <new>
 
 #include "tg_solver.cuh"
 
@@ -747,37 +749,88 @@ static int leaf_chunks(Solver &S, const ListView &LV, int32_t &npp, int32_t &tot
     return TG_OK;
 }
 
+/* The leaves in batches whose chunks fit the scratch: pp and pc bytes per PP_E and
+ * PC_E chunk.  All of them in one where they fit, else from the chunk offsets. */
+static int leaf_batches(Solver &S, int32_t npp, int32_t total, size_t pp, size_t pc, std::vector<EwBatch> &out,
+                        cudaStream_t st) {
+    const int32_t nleaves = (int32_t)S.st.leaves;
+    out.clear();
+    if ((size_t)npp * pp + (size_t)(total - npp) * pc <= S.ew_scratch) {
+        out.push_back({0, nleaves, 0, npp, npp, total - npp});
+        return TG_OK;
+    }
+    const size_t noff = 2 * ((size_t)nleaves + 1);
+    std::unique_ptr<int32_t[]> off(new (std::nothrow) int32_t[noff]);
+    if (!off) return TG_ERR_NOMEM;
+    TG_CUDA(cudaMemcpyAsync(off.get(), S.ew_off.p, noff * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    TG_CUDA(cudaStreamSynchronize(st));
+    const int32_t *offp = off.get() + nleaves + 1;
+    for (int32_t l0 = 0, l1; l0 < nleaves; l0 = l1) {
+        for (l1 = l0 + 1; l1 < nleaves; l1++) /* at least one leaf */
+            if ((size_t)(off[l1 + 1] - off[l0]) * pp + (size_t)(offp[l1 + 1] - offp[l0]) * pc > S.ew_scratch) break;
+        out.push_back({l0, l1, off[l0], off[l1] - off[l0], offp[l0], offp[l1] - offp[l0]});
+    }
+    return TG_OK;
+}
+/* vectors whose source sums (nsrc rows, `bytes` each) are held at a time, of N */
+static int ew_vectors(const Solver &S, int32_t nsrc, size_t bytes, int N) {
+    const size_t n = S.ew_scratch / (std::max(nsrc, 1) * bytes);
+    return n >= (size_t)N ? N : std::max(1, (int)n);
+}
+
 /* the leaf Ewald lists (PP_E, PC_E) of every leaf, in balanced chunks, added
  * to the FP64 accumulators accd (leaf_max <= 64) */
 template <class T>
 static int leaf_ewald(Solver &S, const GParams &P, const ListView &LV, const EwaldTables &E, cudaStream_t st) {
     typedef typename Sep<T>::T2 T2;
+    constexpr int N = Sep<T>::N;
     const int32_t nleaves = (int32_t)S.st.leaves;
     int32_t npp = 0, total = 0, nsrc = 0;
     TG_TRY(leaf_chunks(S, LV, npp, total, nsrc, st));
     if (total <= 0) return TG_OK;
-    TG_TRY(ensure(S.ew_part, (size_t)total * 64 * 4));
-    const int32_t *offp = S.ew_off.p + nleaves + 1;
-    T2 *tpart = nullptr;
+    std::vector<EwBatch> batches;
+    TG_TRY(leaf_batches(S, npp, total, (256 * sizeof(double)) + N * sizeof(T2), 256 * sizeof(double), batches, st));
+    size_t slots = 0, sums = 0;
+    for (const EwBatch &B : batches) {
+        slots = std::max(slots, (size_t)B.na + B.nc);
+        sums = std::max(sums, (size_t)B.na);
+    }
+    const int nv = ew_vectors(S, nsrc, sizeof(T2), N);
+    TG_TRY(ensure(S.ew_part, slots * 64 * 4));
     if (npp > 0) {
-        TG_TRY(ensure(S.ew_sf, (size_t)nsrc * Sep<T>::N * sizeof(T2)));
-        TG_TRY(ensure(S.ew_tpart, (size_t)npp * Sep<T>::N * sizeof(T2)));
-        T2 *sf = reinterpret_cast<T2 *>(S.ew_sf.p);
-        tpart = reinterpret_cast<T2 *>(S.ew_tpart.p);
-        k_ewald_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E, sf);
-        TG_TRY(launched(S));
-        k_ewald_pp<T><<<npp, 64, 0, st>>>(P, ew_fine(S), S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, LV, E,
-                                          S.ew_part.p, S.ew_slot.p, sf, tpart);
+        TG_TRY(ensure(S.ew_sf, (size_t)nsrc * nv * sizeof(T2)));
+        TG_TRY(ensure(S.ew_tpart, sums * N * sizeof(T2)));
+    }
+    T2 *sf = reinterpret_cast<T2 *>(S.ew_sf.p), *tpart = reinterpret_cast<T2 *>(S.ew_tpart.p);
+    const int32_t *offp = S.ew_off.p + nleaves + 1;
+    const bool fine = ew_fine(S);
+    if (npp > 0 && nv == N) {
+        k_ewald_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E, 0, N, sf);
         TG_TRY(launched(S));
     }
-    if (total > npp) {
-        k_ewald_pc<T><<<total - npp, 64, 0, st>>>(S.idx.p, nleaves, npp, offp, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p, S.pos.p,
-                                                  LV, E, S.ew_part.p);
+    for (const EwBatch &B : batches) {
+        if (B.na > 0) {
+            k_ewald_pp<T><<<B.na, 64, 0, st>>>(P, fine, S.idx.p, nleaves, B.a0, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p,
+                                               LV, E, S.ew_part.p, S.ew_slot.p, nv == N ? sf : nullptr, tpart);
+            TG_TRY(launched(S));
+        }
+        for (int t0 = 0; B.na > 0 && nv < N && t0 < N; t0 += nv) {
+            const int t1 = std::min(N, t0 + nv);
+            k_ewald_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E, t0, t1, sf);
+            TG_TRY(launched(S));
+            k_ewald_tsum<T, T2><<<B.na, 64, 0, st>>>(T(P.m_d), fine, S.idx.p, nleaves, B.a0, S.ew_off.p, LV, S.ew_slot.p,
+                                                     t0, t1, sf, tpart);
+            TG_TRY(launched(S));
+        }
+        if (B.nc > 0) {
+            k_ewald_pc<T><<<B.nc, 64, 0, st>>>(S.idx.p, nleaves, B.c0, B.na, offp, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p,
+                                               S.pos.p, LV, E, S.ew_part.p);
+            TG_TRY(launched(S));
+        }
+        k_ewald_reduce<T><<<B.l1 - B.l0, 256, 0, st>>>(B, S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.ew_part.p,
+                                                       S.accd.p, tpart, S.pos.p, E);
         TG_TRY(launched(S));
     }
-    k_ewald_reduce<T><<<nleaves, 256, 0, st>>>(S.idx.p, nleaves, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.ew_part.p, S.accd.p,
-                                               tpart, S.pos.p, E);
-    TG_TRY(launched(S));
     return TG_OK;
 }
 

@@ -66,6 +66,11 @@ struct DevBuf {
 
 constexpr int NLIST = 8;
 
+/* Bytes of each of the two scratch areas of the leaf Ewald sums: the chunks of one
+ * batch of leaves, and the source leaves' sums (tg_ewald_leaf.cuh).  128^3 at theta 0.2
+ * and smaller boxes run in one batch. */
+constexpr size_t EW_SCRATCH = 1ull << 30;
+
 struct Solver {
     tg_params prm{};
     int dev = 0;
@@ -152,6 +157,7 @@ struct Solver {
     DevBuf<int32_t> ew_slot, ew_src; /* per node: its row of ew_sf, or -1; the nodes of the rows, then their count */
     DevBuf<unsigned char> ew_sf;    /* per PP_E source leaf and h: (cos, sin) sums over its particles (Sep<T>::T2) */
     DevBuf<unsigned char> ew_tpart; /* per PP_E chunk and h: source sums (Sep<T>::T2) */
+    size_t ew_scratch = EW_SCRATCH;
     bool ew_use_tab = false;       /* a periodic solver of the FP32 path */
     const float *ew_tab = nullptr; /* the device's table of local expansions (FP32 path), shared by its solvers */
     bool have_tables = false;

@@ -131,6 +131,11 @@ class GravitySolver:
         check("tg_set_walk_capacity", lib.tg_set_walk_capacity(self.h, int(entries)))
         return self
 
+    def set_ewald_scratch(self, nbytes: int):
+        """Device bytes of each scratch area of the leaf Ewald sums (0: 1 GiB)."""
+        check("tg_set_ewald_scratch", lib.tg_set_ewald_scratch(self.h, int(nbytes)))
+        return self
+
     def forces(self, stream=None):
         check("tg_forces", lib.tg_forces(self.h, _stream(stream)))
         return self
