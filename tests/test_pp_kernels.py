@@ -75,3 +75,43 @@ def test_jacobian_fp32_against_fp64(n, theta, leaf, ewald):
             out[p] = s.tidal(u)
     rms = np.sqrt(np.mean(out["f64"] ** 2))
     assert np.sqrt(np.mean((out["f32"] - out["f64"]) ** 2)) <= 1e-5 * rms
+
+
+def _seam(x, src, precision, ewald, h, kind="direct"):
+    """(phi, g) of one sink group through the PP seam"""
+    import torch
+    from tigergrav_b200 import solver as tgs
+    p = tgs.make_params(soft_len=h, m=1.0 / len(src), ewald=ewald, precision=precision)
+    def off(n):
+        return torch.tensor([0, n], dtype=torch.int64, device="cuda")
+    f = torch.zeros((len(x), 4), dtype=torch.float64, device="cuda")
+    tgs.gravity_PP(kind, p, off(len(x)), torch.from_numpy(x).cuda(), off(len(src)), torch.from_numpy(src).cuda(), f)
+    return f.cpu().numpy()
+
+
+@pytest.mark.parametrize("kind,ewald", [("direct", True), ("direct", False), ("ewald", True)])
+@pytest.mark.parametrize("ns,ny", [(1, 1), (7, 128), (64, 1000), (130, 257)])
+def test_seam_fp32_against_fp64(ns, ny, kind, ewald):
+    """Sinks and sources up to a whole box apart (beyond the int32 range in free
+    space), FP32 terms in FP64 sums: a term carries a few 2^-24, an Ewald term a few
+    1e-7 of unit mass, so 2e-6 of the mean of the terms' sizes."""
+    from tigergrav_b200 import ics
+    rng = np.random.default_rng(ns + ny)
+    x = ics.double_to_pos(np.concatenate([np.full((1, 3), 1e-9), rng.random((ns, 3))])[:ns])
+    src = ics.double_to_pos(np.concatenate([np.full((1, 3), 1.0 - 1e-9), rng.random((ny, 3))])[:ny])
+    a, b = (_seam(x, src, p, ewald, 1e-3, kind) for p in ("f32", "f64"))
+    d = (x[:, None].astype(np.int64) - src[None].astype(np.int64)) / 4294967296.0
+    if ewald:
+        d -= np.round(d)
+    r = np.maximum(np.sqrt((d ** 2).sum(-1)), 5e-4)
+    size = 1.0 if kind == "ewald" else np.stack([(1 / r).mean(1)] + [(1 / r ** 2).mean(1)] * 3, 1)
+    assert np.all(np.abs(a - b) <= 2e-6 * size)
+
+
+def test_seam_infinite_term():
+    """A term beyond FP32 (coincident particles, 1 / h past its range) is an
+    infinite potential, not a NaN, and stays with its own sink."""
+    x = np.array([[5, 6, 7], [2 ** 30, 0, 0]], np.int32)
+    src = np.array([[2 ** 29, 1, 2], [5, 6, 7], [-2 ** 28, 8, 9]], np.int32)
+    f = _seam(x, src, "f32", True, 6.5e-39)
+    assert f[0, 0] == -np.inf and np.all(np.isfinite(f[1]))

@@ -124,6 +124,12 @@ template <> __device__ __forceinline__ double sep<double>(int32_t X, int32_t Y, 
     return periodic ? wrap_sep_d(X, Y) : free_sep_d(X, Y);
 }
 
+/* i as a double: 2^52 + 2^31 + i by its bits, less 2^52 + 2^31 (an addition on the FP64
+ * units for a conversion, which run at a quarter of their rate) */
+__device__ __forceinline__ double i2d(int32_t i) {
+    return __dadd_rn(__hiloint2double(0x43300000, i ^ (int32_t)0x80000000), -4503601774854144.0);
+}
+
 template <class T> __device__ __forceinline__ T wrap_sep_t(int32_t X, int32_t Y);
 template <> __device__ __forceinline__ float wrap_sep_t<float>(int32_t X, int32_t Y) { return wrap_sep_f(X, Y); }
 template <> __device__ __forceinline__ double wrap_sep_t<double>(int32_t X, int32_t Y) { return wrap_sep_d(X, Y); }

@@ -531,10 +531,11 @@ __device__ __forceinline__ int32_t rel_off(int32_t Y, int32_t Xr, bool per, uint
 /* PP seams: one block per sink group.  A pass takes up to SEAM_T sinks, ns of
  * them, in C = SEAM_T / ns copies (thread t: sink t % ns, copy t / ns); the
  * sources are staged SEAM_T at a time and copy p takes every C-th of a stage.
- * FP32 terms go to two-float (Kahan) sums, FP64 terms to doubles, and the copies
- * are added in order.  4096 groups of 64 sinks and 2048 sources, direct: 2.13 ms
- * with a thread per sink, sources read from global memory and four
- * float-to-double conversions per pair, 1.68 ms now. */
+ * All sums are FP64, the copies added in order; in FP32 the pair's factors are
+ * converted and multiplied by the separation's exact value, so a direct pair takes
+ * two conversions.  4096 groups of 64 sinks and 2048 sources, direct: 2.13 ms with a
+ * thread per sink, sources read from global memory and four float-to-double
+ * conversions per pair, 1.38 ms now (compensated FP32 sums: 1.68). */
 constexpr int SEAM_T = 128;
 template <class T, bool EWALD>
 __global__ void __launch_bounds__(SEAM_T) k_seam_pp(GParams P, int do_phi, int64_t ngroups,
@@ -554,9 +555,7 @@ __global__ void __launch_bounds__(SEAM_T) k_seam_pp(GParams P, int do_phi, int64
             const int C = SEAM_T / ns, phase = t / ns;
             const int64_t i = i0 + t % ns;
             const int32_t xi[3] = {sink_x[3 * i], sink_x[3 * i + 1], sink_x[3 * i + 2]};
-            Acc<T> o[4];
-#pragma unroll
-            for (int d = 0; d < 4; d++) o[d].init(0.0);
+            double o[4] = {0.0, 0.0, 0.0, 0.0};
             for (int64_t jb = j0; jb < j1; jb += SEAM_T) {
                 const int nt = (int)min((int64_t)SEAM_T, j1 - jb);
                 __syncthreads();
@@ -570,22 +569,27 @@ __global__ void __launch_bounds__(SEAM_T) k_seam_pp(GParams P, int do_phi, int64
                                              wrap_sep_t<T>(xi[2], y[2])};
                             T p, g3[3];
                             pp_ewald_pair<T>(E, dX, p, g3);
-                            o[0].add(p);
+                            o[0] += (double)p;
 #pragma unroll
-                            for (int d = 0; d < 3; d++) o[1 + d].add(g3[d]);
+                            for (int d = 0; d < 3; d++) o[1 + d] += (double)g3[d];
                         } else {
                             const T dX[3] = {sep<T>(xi[0], y[0], per), sep<T>(xi[1], y[1], per),
                                              sep<T>(xi[2], y[2], per)};
                             T fk, p;
                             pp_direct_pair<T>(P, dX, fk, p);
-                            o[0].add(-p);
+                            o[0] -= (double)p;
 #pragma unroll
-                            for (int d = 0; d < 3; d++) o[1 + d].add(-dX[d] * fk);
+                            for (int d = 0; d < 3; d++) {
+                                const double x = sizeof(T) == 8 ? (double)dX[d]
+                                                 : per ? i2d((int32_t)((uint32_t)xi[d] - (uint32_t)y[d]))
+                                                       : i2d(xi[d]) - i2d(y[d]);
+                                o[1 + d] = fma(-x, (double)fk, o[1 + d]);
+                            }
                         }
                     }
             }
 #pragma unroll
-            for (int d = 0; d < 4; d++) red[t][d] = o[d].get();
+            for (int d = 0; d < 4; d++) red[t][d] = o[d];
             __syncthreads();
             if (t < ns) {
                 double v[4] = {0.0, 0.0, 0.0, 0.0};
@@ -595,7 +599,8 @@ __global__ void __launch_bounds__(SEAM_T) k_seam_pp(GParams P, int do_phi, int64
                 if (EWALD || do_phi) f[4 * i] += P.m_d * v[0] - (EWALD ? 0.0 : P.phi_self);
                 else f[4 * i] -= P.phi_self;
 #pragma unroll
-                for (int d = 0; d < 3; d++) f[4 * i + 1 + d] += P.m_d * v[1 + d];
+                for (int d = 0; d < 3; d++)
+                    f[4 * i + 1 + d] += P.m_d * (EWALD || sizeof(T) == 8 ? v[1 + d] : v[1 + d] * POS_INV);
             }
             __syncthreads(); /* red is rewritten next */
         }
