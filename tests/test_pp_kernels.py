@@ -77,6 +77,31 @@ def test_jacobian_fp32_against_fp64(n, theta, leaf, ewald):
     assert np.sqrt(np.mean((out["f32"] - out["f64"]) ** 2)) <= 1e-5 * rms
 
 
+def test_jacobian_sums_keep_small_terms():
+    """Two sources at +-1/16 of a sink, upstream gradients +-2^14, first in the order
+    of the particles and in different copies of the sink: their terms (2^27 of unit
+    mass) cancel to the bit, and the other pairs' terms stay, since every pair goes to
+    a compensated sum of its copy: within 1e-5 of their sizes (their own rounding is a
+    few 2^-24)."""
+    import tigergrav_b200 as tg
+    n = 64
+    rng = np.random.default_rng(1)
+    x = rng.integers(-2 ** 31, 2 ** 31, (n, 3)).astype(np.int32)
+    x[4:, 0] &= 2 ** 31 - 1  # the upper half of the box: after the first four
+    u = rng.standard_normal((n, 3))
+    x[:4] = [[-2 ** 30, 0, 0], [-2 ** 30 + 2 ** 28, 0, 0], [-2 ** 30 - 2 ** 28, 0, 0], [-2 ** 30 + 2 ** 20, 0, 0]]
+    u[:4] = [[0, 0, 0], [2.0 ** 14, 0, 0], [-2.0 ** 14, 0, 0], [0, 0, 0]]
+    with tg.GravitySolver(n, theta=0.7, leaf_max=64, ewald=False, m=1.0 / n, soft_len=1e-3) as s:
+        s.set_particles(x).build().multipoles().walk()
+        got = s.tidal(u)[0]
+        at = np.argsort(s.perm())  # sorted position of each particle; copy = position mod 2
+    assert at[2] == 0 and at[1] == 3
+    d = (x[0].astype(np.int64) - x[4:]) / 4294967296.0
+    r = np.linalg.norm(d, axis=1)[:, None]
+    t = -(-u[4:] / r ** 3 - 3.0 * d * (d * -u[4:]).sum(1)[:, None] / r ** 5) / n
+    assert np.all(np.abs(got - t.sum(0)) <= 1e-5 * np.abs(t).sum(0))
+
+
 def _seam(x, src, precision, ewald, h, kind="direct"):
     """(phi, g) of one sink group through the PP seam"""
     import torch

@@ -321,10 +321,12 @@ __global__ void __launch_bounds__(BLOCK) k_tidal_leaf(GParams P, const int32_t *
 /*
  * PP direct: out_i += -sum_j m H(x_i - x_j) (u_i - u_j), H the Hessian of the
  * softened pair force (pp_pair_deriv).  One block per leaf of at most 64 sinks,
- * C = 128 / ns copies of them (copy p takes every C-th source of a stage), sums
- * over 8 pairs folded into the compensated totals, copies added in order.  In
- * k_tidal_leaf, at the registers of the PC tensors and with every pair folded,
- * this was 2.2 of 5 ms of a 64^3 Jacobian product.
+ * C = 128 / ns copies of them (copy p takes every C-th source of a stage), every
+ * pair folded into the compensated totals, copies added in FP64 in order.  In
+ * k_tidal_leaf, at the registers of the PC tensors, this was 2.2 of 5 ms of a 64^3
+ * Jacobian product.  Plain sums over 8 pairs before each fold take 0.2 ms less of the
+ * 15.8 ms of two steps forward and back there, and lose terms that are 2^-24 of
+ * another in their group.
  */
 template <class T>
 __global__ void __launch_bounds__(128) k_tidal_pp(GParams P, const int32_t *__restrict__ leaves,
@@ -370,20 +372,16 @@ __global__ void __launch_bounds__(128) k_tidal_pp(GParams P, const int32_t *__re
         if (nt == 0) break;
         __syncthreads();
         if (phase >= C) continue;
-        for (int32_t q0 = phase; q0 < nt; q0 += 8 * C) {
-            T s[3] = {T(0), T(0), T(0)};
-            const int32_t q1 = min(nt, q0 + 8 * C);
-            for (int32_t q = q0; q < q1; q += C) {
-                const int4 y = sy[q];
-                const T du[3] = {ui[0] - su[q][0], ui[1] - su[q][1], ui[2] - su[q][2]};
-                const T dX[3] = {sep<T>(xi.x, y.x, per), sep<T>(xi.y, y.y, per), sep<T>(xi.z, y.z, per)};
-                const T r2 = dX[0] * dX[0] + dX[1] * dX[1] + dX[2] * dX[2];
-                T f, fpr;
-                pp_pair_deriv<T>(P, r2, f, fpr);
-                const T w = (dX[0] * du[0] + dX[1] * du[1] + dX[2] * du[2]) * fpr;
-                for (int d = 0; d < 3; d++) s[d] += f * du[d] + dX[d] * w;
-            }
-            for (int d = 0; d < 3; d++) o[d].add(-m * s[d]);
+#pragma unroll 4
+        for (int32_t q = phase; q < nt; q += C) {
+            const int4 y = sy[q];
+            const T du[3] = {ui[0] - su[q][0], ui[1] - su[q][1], ui[2] - su[q][2]};
+            const T dX[3] = {sep<T>(xi.x, y.x, per), sep<T>(xi.y, y.y, per), sep<T>(xi.z, y.z, per)};
+            const T r2 = dX[0] * dX[0] + dX[1] * dX[1] + dX[2] * dX[2];
+            T f, fpr;
+            pp_pair_deriv<T>(P, r2, f, fpr);
+            const T w = (dX[0] * du[0] + dX[1] * du[1] + dX[2] * du[2]) * fpr;
+            for (int d = 0; d < 3; d++) o[d].add(-m * (f * du[d] + dX[d] * w));
         }
     }
     for (int d = 0; d < 3; d++) red[t][d] = phase < C ? o[d].get() : 0.0;

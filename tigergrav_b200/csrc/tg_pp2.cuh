@@ -248,37 +248,34 @@ __device__ __forceinline__ void ppb_near_run(const GParams &P, float h2, const S
     }
 }
 /* a sink against the wrap particles [q, q1) of a stage: the arithmetic of the near
- * form with the separation converted from the wrapped difference, one at a time */
+ * form with the separation converted from the wrapped difference, every pair folded */
 __device__ __forceinline__ void ppb_wrap_run(const GParams &P, float h2, const int4 *st, int q, int q1, int4 x,
                                              bool per, PPAcc &a) {
     const float u = 2.3283064365386963e-10f; /* 2^-32 */
-    while (q < q1) {
-        const int e1 = min(q1, q + 16);
-        for (; q < e1; q++) {
-            const int4 y = st[q];
-            float d[3];
-            if (per) {
-                d[0] = __int2float_rn((int32_t)((uint32_t)x.x - (uint32_t)y.x));
-                d[1] = __int2float_rn((int32_t)((uint32_t)x.y - (uint32_t)y.y));
-                d[2] = __int2float_rn((int32_t)((uint32_t)x.z - (uint32_t)y.z));
-            } else {
-                d[0] = __ll2float_rn((long long)x.x - y.x);
-                d[1] = __ll2float_rn((long long)x.y - y.y);
-                d[2] = __ll2float_rn((long long)x.z - y.z);
-            }
-            const float r2 = fmaf(d[0], d[0], fmaf(d[1], d[1], d[2] * d[2]));
-            float p = rsqrt_ftz(fmaxf(r2, h2)), f = p * p * p;
-            if (r2 <= h2) { /* softened, in box units */
-                const float b[3] = {d[0] * u, d[1] * u, d[2] * u};
-                pp_direct_pair<float>(P, b, f, p);
-                p *= u;
-                f *= u * u * u;
-            }
-            a.tp.x += p;
-            a.t0.x = fmaf(d[0], f, a.t0.x);
-            a.t1.x = fmaf(d[1], f, a.t1.x);
-            a.t2.x = fmaf(d[2], f, a.t2.x);
+    for (; q < q1; q++) {
+        const int4 y = st[q];
+        float d[3];
+        if (per) {
+            d[0] = __int2float_rn((int32_t)((uint32_t)x.x - (uint32_t)y.x));
+            d[1] = __int2float_rn((int32_t)((uint32_t)x.y - (uint32_t)y.y));
+            d[2] = __int2float_rn((int32_t)((uint32_t)x.z - (uint32_t)y.z));
+        } else {
+            d[0] = __ll2float_rn((long long)x.x - y.x);
+            d[1] = __ll2float_rn((long long)x.y - y.y);
+            d[2] = __ll2float_rn((long long)x.z - y.z);
         }
+        const float r2 = fmaf(d[0], d[0], fmaf(d[1], d[1], d[2] * d[2]));
+        float p = rsqrt_ftz(fmaxf(r2, h2)), f = p * p * p;
+        if (r2 <= h2) { /* softened, in box units */
+            const float b[3] = {d[0] * u, d[1] * u, d[2] * u};
+            pp_direct_pair<float>(P, b, f, p);
+            p *= u;
+            f *= u * u * u;
+        }
+        a.tp.x = p;
+        a.t0.x = d[0] * f;
+        a.t1.x = d[1] * f;
+        a.t2.x = d[2] * f;
         a.fold();
     }
 }
