@@ -1,5 +1,6 @@
 """The algebra behind the FP32 path's reciprocal-space sums per sink
-(tigergrav_b200/csrc/tg_ewald_sep.cuh, k_node_ewald_recip): for any
+(tigergrav_b200/csrc/tg_ewald_sep.cuh, which uses it for the particles of leaves;
+multipole sources, whose sums the expansion table took over, are the general case): for any
 coefficient table of the M2P / M2L contractions (src/gravity.cpp:26-169) and
 any set of sources, summing m_k cos/sin(2 pi h.X_j) per sink and evaluating
 the terms once at the sink equals contracting each source's multipole with

@@ -401,13 +401,16 @@ __global__ void __launch_bounds__(128) k_tidal_pp(GParams P, const int32_t *__re
  * of (h.u_j)(cos, sin) th_j; the real-space part is the Hessians of the nearest
  * image and its neighbours towards the near corner.  The whole green_ewald
  * per pair took 0.9 of a 64^3 Jacobian product (12e6 pairs).
+ *
+ * The reciprocal sums are FP64 in both paths: a sink takes (h.u_i) times one pair of
+ * sums less the other, and with FP32 sums a common part of u, which every
+ * u_i - u_j is free of, would leave its rounding.  In the FP32 path the nearest image
+ * is FP64 too, as in the force (sep_near), for the same cancellation, at alpha^3.
  */
-template <class T> struct Sep4 {
-    T c, s, uc, us;
+struct Sep4 {
+    double c, s, uc, us;
 };
-template <> __device__ __forceinline__ Sep4<float> sep_zero<Sep4<float>>() { return {0.0f, 0.0f, 0.0f, 0.0f}; }
-template <> __device__ __forceinline__ Sep4<double> sep_zero<Sep4<double>>() { return {0.0, 0.0, 0.0, 0.0}; }
-template <class T> __device__ __forceinline__ void sep_madd(Sep4<T> &a, T m, const Sep4<T> &f) {
+__device__ __forceinline__ void sep_madd(Sep4 &a, double m, const Sep4 &f) {
     a.c = fma(m, f.c, a.c);
     a.s = fma(m, f.s, a.s);
     a.uc = fma(m, f.uc, a.uc);
@@ -418,34 +421,64 @@ template <class T>
 __global__ void __launch_bounds__(128) k_tidal_sf(const int32_t *__restrict__ src, const int32_t *__restrict__ pb,
                                                   const int32_t *__restrict__ pe, const int4 *__restrict__ pos,
                                                   const double *__restrict__ u, EwaldTables E, int t0, int t1,
-                                                  Sep4<T> *__restrict__ sf) {
+                                                  Sep4 *__restrict__ sf) {
+    __shared__ SepTrig<T> trig;
     const int32_t node = src[blockIdx.x];
-    const int32_t b = pb[node], e = pe[node];
-    for (int t = t0 + threadIdx.x; t < t1; t += 128) {
-        const int4 h = __ldg(&E.sep_h[t]);
-        Sep4<T> a{T(0), T(0), T(0), T(0)};
-        for (int32_t j = b; j < e; j++) {
-            const int4 p = __ldg(&pos[j]);
-            const typename Sep<T>::T2 q = sep_cs<T>(p.x, p.y, p.z, h);
-            const T hu = T(h.x * u[3 * (int64_t)j] + h.y * u[3 * (int64_t)j + 1] + h.z * u[3 * (int64_t)j + 2]);
-            a.c += q.x;
-            a.s += q.y;
-            a.uc = fma(hu, q.x, a.uc);
-            a.us = fma(hu, q.y, a.us);
+    const int32_t b = pb[node], n = pe[node] - b;
+    sep_trig<T>(trig, pos + b, n);
+    Sep4 *const row = sf + (int64_t)blockIdx.x * (t1 - t0) - t0;
+    if constexpr (sizeof(T) == 4) { /* a thread per run, as k_ewald_sf */
+        for (int r = threadIdx.x; r < E.sep_nrun; r += 128) {
+            const int4 run = __ldg(&E.sep_run[r]);
+            const int t = run.w >> 8, len = run.w & 255;
+            if (t >= t1 || t + len <= t0) continue;
+            Sep4 a[SEP_RUN] = {};
+            for (int32_t j = 0; j < n; j++) {
+                double2 e = trig.first(j, run);
+                const double2 z = trig.step(j);
+                const double *uj = u + 3 * (int64_t)(b + j);
+                double hu = run.x * uj[0] + run.y * uj[1] + run.z * uj[2];
+#pragma unroll
+                for (int k = 0; k < SEP_RUN; k++) {
+                    a[k].c += e.x;
+                    a[k].s += e.y;
+                    a[k].uc = fma(hu, e.x, a[k].uc);
+                    a[k].us = fma(hu, e.y, a[k].us);
+                    hu += uj[2];
+                    e = trig.mul(e, z);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < SEP_RUN; k++)
+                if (k < len && t + k >= t0 && t + k < t1) row[t + k] = a[k];
         }
-        sf[(int64_t)blockIdx.x * (t1 - t0) + t - t0] = a;
+    } else {
+        for (int t = t0 + threadIdx.x; t < t1; t += 128) {
+            const int4 h = __ldg(&E.sep_h[t]);
+            Sep4 a{};
+            for (int32_t j = 0; j < n; j++) {
+                const double2 q = trig.at(j, pos + b, h);
+                const double *uj = u + 3 * (int64_t)(b + j);
+                const double hu = h.x * uj[0] + h.y * uj[1] + h.z * uj[2];
+                a.c += q.x;
+                a.s += q.y;
+                a.uc = fma(hu, q.x, a.uc);
+                a.us = fma(hu, q.y, a.us);
+            }
+            row[t] = a;
+        }
     }
 }
 
-/* r += (d1 + d2 x x^T) du for one image at displacement x */
+/* r += (d1 + d2 x x^T) du for one image at displacement x.  With the exact erfc: the
+ * reference's, good to 1.5e-7, would put 3 / r^3 of that into the Hessian. */
 template <class T>
 __device__ __forceinline__ void tidal_image(T x0, T x1, T x2, T r2, const T *du, T *r) {
     const T alpha = T(Sep<T>::ALPHA);
     const T rinv = t_rsqrt(r2), r2inv = rinv * rinv, rr = r2 * rinv;
-    T e;
-    const T erfc = t_erfcexp(alpha * rr, &e);
+    const T e = exp(-(alpha * rr) * (alpha * rr)), ec = erfc(alpha * rr);
     const T ce = T(Sep<T>::ALPHA * 1.1283791670955126) * e; /* 2 alpha / sqrt(pi) e^(-alpha^2 r^2) */
-    const T d1 = fma(ce, rr, erfc) * rinv * r2inv;
+    const T d1 = fma(ce, rr, ec) * rinv * r2inv;
     const T d2 = -fma(T(3), d1, T(2) * alpha * alpha * ce) * r2inv;
     const T s = (x0 * du[0] + x1 * du[1] + x2 * du[2]) * d2;
     r[0] = fma(x0, s, fma(d1, du[0], r[0]));
@@ -453,59 +486,119 @@ __device__ __forceinline__ void tidal_image(T x0, T x1, T x2, T r2, const T *du,
     r[2] = fma(x2, s, fma(d1, du[2], r[2]));
 }
 
-/* the real-space part of D2(x) du; nothing (with the leaf sums' reciprocal part
- * taken back) for r <= 1e-6 */
+/* the mirror images of a pair at |x| = a, in the octant of |x|: r += D2 w */
 template <class T>
-__device__ __forceinline__ void tidal_ewald_pair(const EwaldTables &E, const T *x, const T *du, T *r) {
-    r[0] = r[1] = r[2] = T(0);
-    const T r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-    if (!(r2 > T(1.0e-12))) {
-        for (int d = 0; d < 3; d++) r[d] = -T(E.sep_r2) * du[d];
-        return;
-    }
-    T a[3], b[3], u[3], v[3], w[3], q[3] = {T(0), T(0), T(0)};
+__device__ __forceinline__ void tidal_images(const T *a, const T *w, T *r) {
+    T b[3], u[3], v[3];
 #pragma unroll
-    for (int d = 0; d < 3; d++) { /* in the octant of |x| */
-        a[d] = fabs(x[d]);
+    for (int d = 0; d < 3; d++) {
         b[d] = a[d] - T(1);
         u[d] = a[d] * a[d];
         v[d] = b[d] * b[d];
-        w[d] = copysign(T(1), x[d]) * du[d];
     }
 #pragma unroll
     for (int k = 1; k < 8; k++) {
         const T s = (k & 1 ? v[0] : u[0]) + (k & 2 ? v[1] : u[1]) + (k & 4 ? v[2] : u[2]);
-        if (s < T(1)) tidal_image<T>(k & 1 ? b[0] : a[0], k & 2 ? b[1] : a[1], k & 4 ? b[2] : a[2], s, w, q);
+        if (s < T(1)) tidal_image<T>(k & 1 ? b[0] : a[0], k & 2 ? b[1] : a[1], k & 4 ? b[2] : a[2], s, w, r);
     }
-    /* nearest image with the direct 1/r removed: d1 = -f0, d2 = (3 f0 - 2 alpha^2 c e) / r^2, or the
-     * derivative of f0's series (ewald_nearest) for alpha r < 1/2, where the two cancel */
-    const T alpha = T(Sep<T>::ALPHA);
-    const T rinv = t_rsqrt(r2), rr = r2 * rinv, y = alpha * alpha * r2;
-    T p0, f0, d2;
-    ewald_nearest<T>(alpha, rr, rinv, p0, f0);
-    if (y < T(0.25)) {
-        T s = T(0);
-        if constexpr (sizeof(T) == 8) {
-            s = T(10.0 / 41731200.0);
-            s = fma(s, y, T(-9.0 / 3810240.0));
-            s = fma(s, y, T(8.0 / 383040.0));
-        }
-        s = fma(s, y, T(-7.0 / 42840.0));
-        s = fma(s, y, T(6.0 / 5400.0));
-        s = fma(s, y, T(-5.0 / 780.0));
-        s = fma(s, y, T(4.0 / 132.0));
-        s = fma(s, y, T(-3.0 / 27.0));
-        s = fma(s, y, T(2.0 / 7.0));
-        s = fma(s, y, T(-0.4));
-        d2 = T(-2.0 * 1.1283791670955126) * (alpha * alpha * alpha * alpha * alpha) * s;
-    } else {
-        const T ce = T(Sep<T>::ALPHA * 1.1283791670955126) * exp(-y);
-        d2 = (T(3) * f0 - T(2) * alpha * alpha * ce) * rinv * rinv;
-    }
-    const T s = (a[0] * w[0] + a[1] * w[1] + a[2] * w[2]) * d2;
-#pragma unroll
-    for (int d = 0; d < 3; d++) r[d] = copysign(T(1), x[d]) * (q[d] + a[d] * s - f0 * w[d]);
 }
+
+/* the sums of one sink over the real-space parts D2(x) (u_i - u_j) of its pairs,
+ * times -m; a pair with r <= 1e-6 has none, and takes back what the leaf sums add */
+template <class T> struct TidalPairs;
+template <> struct TidalPairs<double> {
+    double o[3], ui[3];
+    __device__ __forceinline__ void init(const double *u) {
+        for (int d = 0; d < 3; d++) o[d] = 0.0, ui[d] = u[d];
+    }
+    __device__ __forceinline__ void add(const EwaldTables &E, const SepNear &, double m, int4 xi, int4 yj, const double *uj) {
+        const double x[3] = {wrap_sep_d(xi.x, yj.x), wrap_sep_d(xi.y, yj.y), wrap_sep_d(xi.z, yj.z)};
+        const double du[3] = {ui[0] - uj[0], ui[1] - uj[1], ui[2] - uj[2]};
+        const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
+        if (!(r2 > 1.0e-12)) {
+            for (int d = 0; d < 3; d++) o[d] += -m * (-E.sep_r2 * du[d]);
+            return;
+        }
+        double a[3], w[3], q[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            a[d] = fabs(x[d]);
+            w[d] = copysign(1.0, x[d]) * du[d];
+        }
+        tidal_images<double>(a, w, q);
+        /* nearest image with the direct 1/r removed: d1 = -f0, d2 = (3 f0 - 2 alpha^2 c e) / r^2, or the
+         * derivative of f0's series (ewald_nearest) for alpha r < 1/2, where the two cancel */
+        const double alpha = Sep<double>::ALPHA;
+        const double rinv = t_rsqrt(r2), rr = r2 * rinv, y = alpha * alpha * r2;
+        double p0, f0, d2;
+        ewald_nearest<double>(alpha, rr, rinv, p0, f0);
+        if (y < 0.25) {
+            double s = 10.0 / 41731200.0;
+            s = fma(s, y, -9.0 / 3810240.0);
+            s = fma(s, y, 8.0 / 383040.0);
+            s = fma(s, y, -7.0 / 42840.0);
+            s = fma(s, y, 6.0 / 5400.0);
+            s = fma(s, y, -5.0 / 780.0);
+            s = fma(s, y, 4.0 / 132.0);
+            s = fma(s, y, -3.0 / 27.0);
+            s = fma(s, y, 2.0 / 7.0);
+            s = fma(s, y, -0.4);
+            d2 = -2.0 * 1.1283791670955126 * (alpha * alpha * alpha * alpha * alpha) * s;
+        } else {
+            const double ce = Sep<double>::ALPHA * 1.1283791670955126 * exp(-y);
+            d2 = (3.0 * f0 - 2.0 * alpha * alpha * ce) * rinv * rinv;
+        }
+        const double s = (a[0] * w[0] + a[1] * w[1] + a[2] * w[2]) * d2;
+#pragma unroll
+        for (int d = 0; d < 3; d++) o[d] += -m * (copysign(1.0, x[d]) * (q[d] + a[d] * s - f0 * w[d]));
+    }
+    __device__ __forceinline__ double get(int d, double) const { return o[d]; }
+};
+/* FP32: the nearest image in FP64, d1 = -f0 and d2 = -2 df0/dr^2; the mirror images
+ * in FP32 with compensated sums */
+template <> struct TidalPairs<float> {
+    double o[3], ui[3];
+    Acc<float> i[3];
+    __device__ __forceinline__ void init(const double *u) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            o[d] = 0.0, ui[d] = u[d];
+            i[d].init(0.0);
+        }
+    }
+    __device__ __forceinline__ void add(const EwaldTables &E, const SepNear &K, double, int4 xi, int4 yj, const double *uj) {
+        const int32_t n[3] = {(int32_t)((uint32_t)xi.x - (uint32_t)yj.x), (int32_t)((uint32_t)xi.y - (uint32_t)yj.y),
+                              (int32_t)((uint32_t)xi.z - (uint32_t)yj.z)};
+        float x[3], a[3], w[3], q[3] = {0.0f, 0.0f, 0.0f};
+        double X[3], du[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            x[d] = __int2float_rn(n[d]) * 2.3283064365386963e-10f;
+            X[d] = i2d(n[d]);
+            du[d] = ui[d] - uj[d];
+            a[d] = fabsf(x[d]);
+            w[d] = copysignf(1.0f, x[d]) * (float)du[d];
+        }
+        if (!(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] > 1.0e-12f)) {
+            for (int d = 0; d < 3; d++) o[d] -= E.sep_r2 * du[d];
+            return;
+        }
+        tidal_images<float>(a, w, q);
+#pragma unroll
+        for (int d = 0; d < 3; d++) i[d].add(copysignf(1.0f, x[d]) * q[d]);
+        const double t = fma(fma(X[0], X[0], fma(X[1], X[1], X[2] * X[2])), 8.0 / 3.0 * POS_INV * POS_INV, -1.0);
+        double f = K.f[SEP_DF], df = 0.0; /* f0 and its derivative by t */
+#pragma unroll
+        for (int k = SEP_DF - 1; k >= 0; k--) {
+            df = fma(df, t, f);
+            f = fma(f, t, K.f[k]);
+        }
+        const double s = fma(X[0], du[0], fma(X[1], du[1], X[2] * du[2])) * (-16.0 / 3.0 * POS_INV * POS_INV * df);
+#pragma unroll
+        for (int d = 0; d < 3; d++) o[d] += fma(X[d], s, -f * du[d]);
+    }
+    __device__ __forceinline__ double get(int d, double m) const { return -m * (o[d] + i[d].get()); }
+};
 
 /* one chunk of a PP_E list (as k_ewald_pp): the real-space part per pair into
  * part (3 per sink) and, with sf, the reciprocal source sums into tpart */
@@ -513,11 +606,11 @@ template <class T>
 __global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, bool fine, const int32_t *__restrict__ leaves, int32_t nleaves,
                                                        int32_t first, const int32_t *__restrict__ off, const int32_t *__restrict__ pb,
                                                        const int32_t *__restrict__ pe, const int4 *__restrict__ pos,
-                                                       ListView LV, EwaldTables E, const double *__restrict__ u,
+                                                       ListView LV, EwaldTables E, SepNear K, const double *__restrict__ u,
                                                        double *__restrict__ part, const int32_t *__restrict__ slot,
-                                                       const Sep4<T> *__restrict__ sf, Sep4<T> *__restrict__ tpart) {
+                                                       const Sep4 *__restrict__ sf, Sep4 *__restrict__ tpart) {
     __shared__ int4 sy[64];
-    __shared__ T su[64][3];
+    __shared__ double su[64][3];
     __shared__ int32_t s_row[EW_KPP_MAX];
     const int tid = threadIdx.x;
     const int64_t c = (int64_t)first + blockIdx.x;
@@ -526,12 +619,10 @@ __global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, bool fine, con
     const int32_t b = pb[leaf], cnt = pe[leaf] - b;
     const int64_t i = b + (tid < cnt ? tid : 0);
     const int4 xi = pos[i];
-    const T ui[3] = {T(u[3 * i]), T(u[3 * i + 1]), T(u[3 * i + 2])};
-    Acc<T> o[3];
-    for (int d = 0; d < 3; d++) o[d].init(0.0);
+    TidalPairs<T> o;
+    o.init(u + 3 * i);
     const int32_t *lst = LV.pool[TG_PP_E] + LV.off[TG_PP_E][leaf];
     const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len, fine), e0 = k * kpp, e1 = min(len, e0 + kpp);
-    const T m = T(P.m_d);
     if (tid < e1 - e0) s_row[tid] = slot[lst[e0 + tid]];
     for (int32_t e = e0; e < e1; e++) {
         const int32_t src = lst[e];
@@ -540,22 +631,15 @@ __global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, bool fine, con
         if (tid < sn) {
             const int64_t q = sb + tid;
             sy[tid] = pos[q];
-            for (int d = 0; d < 3; d++) su[tid][d] = T(u[3 * q + d]);
+            for (int d = 0; d < 3; d++) su[tid][d] = u[3 * q + d];
         }
         __syncthreads();
         if (tid < ((cnt + 31) & ~31))
-            for (int32_t q = 0; q < sn; q++) {
-                const int4 y = sy[q];
-                const T dX[3] = {wrap_sep_t<T>(xi.x, y.x), wrap_sep_t<T>(xi.y, y.y), wrap_sep_t<T>(xi.z, y.z)};
-                const T du[3] = {ui[0] - su[q][0], ui[1] - su[q][1], ui[2] - su[q][2]};
-                T r[3];
-                tidal_ewald_pair<T>(E, dX, du, r);
-                for (int d = 0; d < 3; d++) o[d].add(-m * r[d]);
-            }
+            for (int32_t q = 0; q < sn; q++) o.add(E, K, P.m_d, xi, sy[q], su[q]);
     }
     if (tid < cnt)
-        for (int d = 0; d < 3; d++) part[3 * ((int64_t)blockIdx.x * 64 + tid) + d] = o[d].get();
-    if (sf) ew_tsum<T, Sep4<T>>(s_row, e1 - e0, 0, Sep<T>::N, tid, sf, m, tpart + (int64_t)blockIdx.x * Sep<T>::N);
+        for (int d = 0; d < 3; d++) part[3 * ((int64_t)blockIdx.x * 64 + tid) + d] = o.get(d, P.m_d);
+    if (sf) ew_tsum<Sep4>(s_row, e1 - e0, 0, Sep<T>::N, tid, sf, P.m_d, tpart + (int64_t)blockIdx.x * Sep<T>::N);
 }
 
 /* out += the chunk sums of each leaf, in chunk order, and the reciprocal part
@@ -567,8 +651,9 @@ __global__ void __launch_bounds__(256) k_tidal_ewald_reduce(EwBatch B, const int
                                                             const int32_t *__restrict__ pb, const int32_t *__restrict__ pe,
                                                             const int4 *__restrict__ pos, EwaldTables E,
                                                             const double *__restrict__ u, const double *__restrict__ part,
-                                                            const Sep4<T> *__restrict__ tpart, double *__restrict__ out) {
-    constexpr int TILE = 384; /* vectors whose sums are held at a time */
+                                                            const Sep4 *__restrict__ tpart, double *__restrict__ out) {
+    constexpr int TILE = sizeof(T) == 4 ? Sep<float>::N : 384; /* vectors whose sums are held at a time */
+    __shared__ SepTrig<T> trig;
     __shared__ double4 sT[TILE];
     __shared__ double sv[4][64][3];
     const int32_t li = B.l0 + blockIdx.x;
@@ -578,8 +663,8 @@ __global__ void __launch_bounds__(256) k_tidal_ewald_reduce(EwBatch B, const int
     const int32_t leaf = leaves[li];
     const int32_t b = pb[leaf], cnt = pe[leaf] - b;
     const int64_t i = b + (t < cnt ? t : 0);
-    const int4 p = pos[i];
     const double ui[3] = {u[3 * i], u[3 * i + 1], u[3 * i + 2]};
+    sep_trig<T>(trig, pos + b, cnt);
     double v[3] = {0.0, 0.0, 0.0};
     for (int t0 = 0; t0 < Sep<T>::N; t0 += TILE) {
         const int nt = min(TILE, Sep<T>::N - t0);
@@ -587,19 +672,39 @@ __global__ void __launch_bounds__(256) k_tidal_ewald_reduce(EwBatch B, const int
         for (int q = tid; q < nt; q += 256) {
             double4 s = make_double4(0.0, 0.0, 0.0, 0.0);
             for (int64_t c = a0; c < a1; c++) {
-                const Sep4<T> f = tpart[c * Sep<T>::N + t0 + q];
-                s.x += (double)f.c;
-                s.y += (double)f.s;
-                s.z += (double)f.uc;
-                s.w += (double)f.us;
+                const Sep4 f = tpart[c * Sep<T>::N + t0 + q];
+                s.x += f.c;
+                s.y += f.s;
+                s.z += f.uc;
+                s.w += f.us;
             }
             sT[q] = s;
         }
         __syncthreads();
-        if (t < cnt)
+        if (t >= cnt) continue;
+        if constexpr (sizeof(T) == 4) {
+            const double2 z = trig.step(t);
+            for (int r = grp; r < E.sep_nrun; r += 4) {
+                const int4 run = __ldg(&E.sep_run[r]);
+                const int q0 = run.w >> 8, len = run.w & 255;
+                double2 e = trig.first(t, run);
+                double hu = run.x * ui[0] + run.y * ui[1] + run.z * ui[2], h = run.z, sum = 0.0;
+                for (int k = 0; k < len; k++) {
+                    const double4 s = sT[q0 + k];
+                    const double f = __ldg(&E.sep_w[q0 + k]) * (hu * (e.x * s.x + e.y * s.y) - (e.x * s.z + e.y * s.w));
+                    sum += f;
+                    v[2] = fma(f, h, v[2]);
+                    h += 1.0;
+                    hu += ui[2];
+                    e = trig.mul(e, z);
+                }
+                v[0] = fma(sum, (double)run.x, v[0]);
+                v[1] = fma(sum, (double)run.y, v[1]);
+            }
+        } else {
             for (int q = grp; q < nt; q += 4) {
                 const int4 h = __ldg(&E.sep_h[t0 + q]);
-                const typename Sep<T>::T2 cs = sep_cs<T>(p.x, p.y, p.z, h);
+                const double2 cs = trig.at(t, pos + b, h);
                 const double4 s = sT[q];
                 const double hu = h.x * ui[0] + h.y * ui[1] + h.z * ui[2];
                 const double C = cs.x, Sn = cs.y;
@@ -608,6 +713,7 @@ __global__ void __launch_bounds__(256) k_tidal_ewald_reduce(EwBatch B, const int
                 v[1] += f * h.y;
                 v[2] += f * h.z;
             }
+        }
     }
     for (int d = 0; d < 3; d++) sv[grp][t][d] = v[d];
     __syncthreads();
@@ -620,6 +726,9 @@ __global__ void __launch_bounds__(256) k_tidal_ewald_reduce(EwBatch B, const int
     }
 }
 
+/* bytes of a PP_E chunk of a Jacobian product */
+constexpr size_t tidal_chunk_bytes(int N) { return 64 * 3 * sizeof(double) + N * sizeof(Sep4); }
+
 /* the PP_E lists' part of J u, added to tid_o (leaf_max <= 64) */
 template <class T>
 static int tidal_ewald(Solver &S, const GParams &P, const ListView &LV, const EwaldTables &E, cudaStream_t st) {
@@ -627,17 +736,16 @@ static int tidal_ewald(Solver &S, const GParams &P, const ListView &LV, const Ew
     int32_t npp = 0, total = 0, nsrc = 0;
     TG_TRY(leaf_chunks(S, LV, npp, total, nsrc, st));
     if (npp <= 0) return TG_OK;
-    typedef Sep4<T> T4;
     constexpr int N = Sep<T>::N;
     std::vector<EwBatch> batches;
-    TG_TRY(leaf_batches(S, npp, npp, 192 * sizeof(double) + N * sizeof(T4), 0, batches, st));
+    TG_TRY(leaf_batches(S, npp, npp, tidal_chunk_bytes(N), 0, batches, st));
     size_t slots = 0;
     for (const EwBatch &B : batches) slots = std::max(slots, (size_t)B.na);
-    const int nv = ew_vectors(S, nsrc, sizeof(T4), N);
+    const int nv = ew_vectors(S, nsrc, sizeof(Sep4), N);
     TG_TRY(ensure(S.ew_part, slots * 64 * 3));
-    TG_TRY(ensure(S.ew_sf, (size_t)nsrc * nv * sizeof(T4)));
-    TG_TRY(ensure(S.ew_tpart, slots * N * sizeof(T4)));
-    T4 *sf = reinterpret_cast<T4 *>(S.ew_sf.p), *tpart = reinterpret_cast<T4 *>(S.ew_tpart.p);
+    TG_TRY(ensure(S.ew_sf, (size_t)nsrc * nv * sizeof(Sep4)));
+    TG_TRY(ensure(S.ew_tpart, slots * N * sizeof(Sep4)));
+    Sep4 *sf = reinterpret_cast<Sep4 *>(S.ew_sf.p), *tpart = reinterpret_cast<Sep4 *>(S.ew_tpart.p);
     const bool fine = ew_fine(S);
     if (nv == N) {
         k_tidal_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, S.tid_u.p, E, 0, N, sf);
@@ -646,14 +754,14 @@ static int tidal_ewald(Solver &S, const GParams &P, const ListView &LV, const Ew
     for (const EwBatch &B : batches) {
         if (B.na == 0) continue;
         k_tidal_ewald_pp<T><<<B.na, 64, 0, st>>>(P, fine, S.idx.p, nleaves, B.a0, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p,
-                                                 LV, E, S.tid_u.p, S.ew_part.p, S.ew_slot.p, nv == N ? sf : nullptr, tpart);
+                                                 LV, E, S.ew_near, S.tid_u.p, S.ew_part.p, S.ew_slot.p, nv == N ? sf : nullptr, tpart);
         TG_TRY(launched(S));
         for (int t0 = 0; nv < N && t0 < N; t0 += nv) {
             const int t1 = std::min(N, t0 + nv);
             k_tidal_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, S.tid_u.p, E, t0, t1, sf);
             TG_TRY(launched(S));
-            k_ewald_tsum<T, T4><<<B.na, 64, 0, st>>>(T(P.m_d), fine, S.idx.p, nleaves, B.a0, S.ew_off.p, LV, S.ew_slot.p,
-                                                     t0, t1, sf, tpart);
+            k_ewald_tsum<Sep4><<<B.na, 64, 0, st>>>(N, P.m_d, fine, S.idx.p, nleaves, B.a0, S.ew_off.p, LV, S.ew_slot.p, t0,
+                                                    t1, sf, tpart);
             TG_TRY(launched(S));
         }
         k_tidal_ewald_reduce<T><<<B.l1 - B.l0, 256, 0, st>>>(B, S.idx.p, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E,

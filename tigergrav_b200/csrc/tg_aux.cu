@@ -102,6 +102,45 @@ __global__ void k_periodic_parts(const float4 *four, int nf, double scale, doubl
     Pd[2 * t + 1] = make_double2(Hd[HS * t + E1(1)], Hd[HS * t + E1(2)]);
 }
 
+/* monomial coefficients m[0..n] in t of the Chebyshev interpolation of fn(r^2), r^2 = 3/8 (t + 1) */
+template <class F> static void sep_fit(F fn, int n, double *m) {
+    const double pi = 3.141592653589793;
+    std::vector<double> c(n + 1, 0.0), a(n + 1, 0.0), b(n + 1, 0.0), sum(n + 1, 0.0);
+    for (int j = 0; j <= n; j++) {
+        const double th = pi * (j + 0.5) / (n + 1), v = fn(0.375 * (std::cos(th) + 1.0));
+        for (int k = 0; k <= n; k++) c[k] += (k ? 2.0 : 1.0) / (n + 1) * v * std::cos(k * th);
+    }
+    a[0] = 1.0; /* T_k, and T_k+1 in b */
+    b[1] = 1.0;
+    for (int k = 0; k <= n; k++) {
+        for (int i = 0; i <= n; i++) sum[i] += c[k] * a[i];
+        for (int i = n; i >= 0; i--) a[i] = (i ? 2.0 * b[i - 1] : 0.0) - a[i]; /* T_k+2 = 2 t T_k+1 - T_k */
+        std::swap(a, b);
+    }
+    for (int i = 0; i <= n; i++) m[i] = (double)sum[i];
+}
+
+/* SepNear: interpolation errors 3e-9 of the potential, 1e-9 of the force and 2e-7 of the Jacobian (f0' r^2),
+ * against ~1 */
+static void sep_near(double alpha, SepNear &K) {
+    const double al = alpha, ispi = 1.1283791670955126; /* 2 / sqrt(pi) */
+    sep_fit([&](double y) { return std::erf(al * std::sqrt(y)) / std::sqrt(y); }, SEP_DP, K.p);
+    K.p[0] += 3.141592653589793 / (alpha * alpha) + SEP_OFFSET;
+    sep_fit(
+        [&](double y) {
+            const double x = al * std::sqrt(y);
+            if (x > 1.0) return (std::erf(x) - ispi * x * std::exp(-x * x)) / (y * std::sqrt(y));
+            double s = 0.0, t = 1.0; /* ewald_nearest's series; t = (-x^2)^(k-1) / k! */
+            for (int k = 1; k < 30; k++) {
+                t /= k;
+                s += 2 * k * t / (2 * k + 1);
+                t *= -x * x;
+            }
+            return al * al * al * ispi * s;
+        },
+        SEP_DF, K.f);
+}
+
 int ewald_tables(Solver &S, cudaStream_t st) {
     if (S.have_tables) return TG_OK;
     const auto real = lattice(17), four = lattice(9);
@@ -130,14 +169,15 @@ int ewald_tables(Solver &S, cudaStream_t st) {
     k_periodic_parts<<<(NFOUR_HALF + 63) / 64, 64, 0, st>>>(S.ew_four.p, NFOUR_HALF, 2.0, S.ew_Hd.p, S.ew_Hf.p, S.ew_Pf.p,
                                                             S.ew_Pd.p);
     TG_TRY(launched(S));
-    /* the PP Ewald split: vectors in increasing |h|^2 */
-    std::vector<int4> sh;
+    /* the PP Ewald split: vectors in increasing |h|^2 (FP64) or in lexicographic order with their runs (FP32) */
+    std::vector<int4> sh, runs;
     std::vector<double> sw;
     double r0 = 0.0, r2 = 0.0;
     const bool f64 = S.prm.precision == TG_PREC_F64;
     const double alpha = f64 ? Sep<double>::ALPHA : Sep<float>::ALPHA;
     const size_t nsep = f64 ? Sep<double>::N : Sep<float>::N;
-    const auto rec = lattice(f64 ? Sep<double>::H2MAX : Sep<float>::H2MAX);
+    auto rec = lattice(f64 ? Sep<double>::H2MAX : Sep<float>::H2MAX);
+    if (!f64) std::sort(rec.rbegin(), rec.rend()); /* along z, for the runs */
     for (auto v = rec.rbegin(); v != rec.rend(); ++v) {
         const int lead = (*v)[0] != 0 ? (*v)[0] : ((*v)[1] != 0 ? (*v)[1] : (*v)[2]);
         if (lead <= 0) continue;
@@ -146,15 +186,27 @@ int ewald_tables(Solver &S, cudaStream_t st) {
         const double w = 2.0 * std::exp(-pi * pi * h2 / (alpha * alpha)) / h2;
         sh.push_back(make_int4((*v)[0], (*v)[1], (*v)[2], 0));
         sw.push_back(w);
+        if (!f64) {
+            const int t = (int)sh.size() - 1;
+            int4 *q = runs.empty() ? nullptr : &runs.back();
+            if (q && q->x == (*v)[0] && q->y == (*v)[1] && (q->w & 255) < SEP_RUN && q->z + (q->w & 255) == (*v)[2]) q->w++;
+            else runs.push_back(make_int4((*v)[0], (*v)[1], (*v)[2], t << 8 | 1));
+        }
         r0 -= w / pi;
         r2 += 4.0 * pi / 3.0 * w * h2;
     }
     if (sh.size() != nsep) return TG_ERR_STATE;
-    S.ew_sep_k = 3.141592653589793 / (alpha * alpha) + (S.prm.precision == TG_PREC_F32 ? SEP_OFFSET : 0.0);
+    if (!f64) sep_near(alpha, S.ew_near);
+    S.ew_sep_k = 3.141592653589793 / (alpha * alpha);
     S.ew_sep_r0 = r0;
     S.ew_sep_r2 = r2;
     TG_TRY(ensure(S.ew_sep_h, nsep));
     TG_TRY(ensure(S.ew_sep_w, nsep));
+    if (!f64) {
+        S.ew_sep_nrun = (int)runs.size();
+        TG_TRY(ensure(S.ew_sep_run, runs.size()));
+        TG_CUDA(cudaMemcpyAsync(S.ew_sep_run.p, runs.data(), sizeof(int4) * runs.size(), cudaMemcpyHostToDevice, st));
+    }
     TG_CUDA(cudaMemcpyAsync(S.ew_sep_h.p, sh.data(), sizeof(int4) * nsep, cudaMemcpyHostToDevice, st));
     TG_CUDA(cudaMemcpyAsync(S.ew_sep_w.p, sw.data(), sizeof(double) * nsep, cudaMemcpyHostToDevice, st));
     if (S.ew_use_tab && !S.ew_tab) TG_TRY(ewald_table_acquire(S.dev, S.ew_real.p, S.ew_four.p, &S.ew_tab, st));

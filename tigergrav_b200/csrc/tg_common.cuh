@@ -29,22 +29,30 @@ constexpr float EWALD_RCUT = 1.0e-6f;
 constexpr float EWALD_PHI0 = 2.8372975f; /* r -> 0 limit (tigergrav/green.hpp:272) */
 
 /* The split of the PP Ewald sums (tg_ewald_sep.cuh): alpha, the largest |h|^2 of
- * the reciprocal vectors, and their number (one of each pair +-h) */
+ * the reciprocal vectors (FP32: and the largest |h_d|), and their number (one of
+ * each pair +-h) */
 /* The FP32 pair's potential keeps the mean by which the FP32 sums of the reference's
- * split (alpha = 2, Abramowitz & Stegun 7.1.26 for erfc) lie below FP64: -4.4e-7 to
- * -6.6e-7 per pair of unit mass over uniform boxes of 1000 to 6000 particles.  A
- * larger alpha has less of it, and potentials near zero would show the difference. */
+ * split (alpha = 2, Abramowitz & Stegun 7.1.26 for erfc) lie below FP64: -5.3e-7 per
+ * pair of unit mass over the cube of separations (-6.9e-7 for |x_d| < 1/4, -9e-7
+ * below 1/20).  The same erfc at alpha = 4.5 leaves -3e-8 of it; this is the rest.
+ * Without it the potentials of small boxes, which cancel to a few 1e-2, differ from
+ * the reference's FP32 ones by 2e-5 of their size. */
 constexpr double SEP_OFFSET = -4.8e-7;
 template <class T> struct Sep;
 template <> struct Sep<float> {
-    static constexpr double ALPHA = 4.2;
-    static constexpr int H2MAX = 30, N = 369;
-    typedef float2 T2;
+    static constexpr double ALPHA = 4.5;
+    static constexpr int H2MAX = 41, HMAX = 6, N = 570;
 };
 template <> struct Sep<double> {
     static constexpr double ALPHA = 5.2;
     static constexpr int H2MAX = 70, N = 1258;
-    typedef double2 T2;
+};
+/* the FP32 pair's nearest image in FP64 (sep_near): erf(alpha r)/r + pi / alpha^2 and
+ * its force factor as polynomials in t = 8/3 r^2 - 1 */
+constexpr int SEP_RUN = 7; /* vectors of a run, at most (SepTrig) */
+constexpr int SEP_DP = 17, SEP_DF = 20;
+struct SepNear {
+    double p[SEP_DP + 1], f[SEP_DF + 1];
 };
 
 /* ---- symmetric index arithmetic (constant-folded after unrolling) ---- */
@@ -278,8 +286,10 @@ struct EwaldTables {
     const float4 *Pf;   /* NFOUR_HALF x (H0, Hx, Hy, Hz): the potential and force terms, float */
     const double2 *Pd;  /* NFOUR_HALF x 2, double */
     const int4 *sep_h;  /* reciprocal vectors of the PP Ewald split (tg_ewald_sep.cuh; Sep<T>::N of them) */
+    const int4 *sep_run; /* FP32: runs of vectors along z (SepTrig): hx, hy, the first hz, first vector << 8 | vectors */
+    int sep_nrun;
     const double *sep_w; /* their weights 2 exp(-pi^2 h^2 / alpha^2) / h^2 */
-    double sep_k, sep_r0, sep_r2; /* pi / alpha^2 (and SEP_OFFSET); the reciprocal part near r = 0: phi = r0, g = -r2 x */
+    double sep_k, sep_r0, sep_r2; /* pi / alpha^2 (FP64 pairs); the reciprocal part near r = 0: phi = r0, g = -r2 x */
     const float *tab;   /* local expansions of green_ewald (tg_ewald_table.cuh); solvers of the FP32 path only */
 };
 

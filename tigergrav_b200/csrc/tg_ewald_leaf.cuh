@@ -17,8 +17,8 @@
  * the scan of the leaves' PP_E chunk counts, off[nleaves + 1, 2 nleaves + 1]
  * that of their PC_E counts continued.
  *
- * A PP_E chunk's slots take 2 KB and its source sums 3 KB in FP32 and 20 KB in
- * FP64 (the Jacobian's 6 and 40 KB), and where every pair is an Ewald pair the
+ * A PP_E chunk's slots take 2 KB and its source sums 9 KB in FP32 and 20 KB in
+ * FP64 (the Jacobian's 18 and 40 KB), and where every pair is an Ewald pair the
  * chunks grow with the square of the leaves.  So the leaves run in batches whose
  * chunks fit EW_SCRATCH, each reduced before the next (leaf_batches), and where
  * the source leaves' own sums do not fit it, they are made for a range of vectors
@@ -38,6 +38,9 @@ __host__ __device__ __forceinline__ int32_t ew_kpp(int32_t len, bool fine) {
     return k < lo ? lo : (k > EW_KPP_MAX ? EW_KPP_MAX : k);
 }
 constexpr int EW_KPC = 64; /* PC_E source nodes per chunk */
+#ifndef EW_MINB_F
+#define EW_MINB_F 16 /* resident 64-thread blocks per SM that the FP32 pair kernel is compiled for */
+#endif
 
 /* leaves [l0, l1) with their PP_E chunks [a0, a0 + na) and PC_E chunks [c0, c0 + nc),
  * whose slots follow each other in that order */
@@ -97,21 +100,21 @@ __device__ __forceinline__ int32_t ew_leaf(const int32_t *__restrict__ off, int3
 }
 
 /* the source sums of a chunk (rows of sf, one per source leaf, holding vectors [t0, t1)) into its row of tpart */
-template <class T, class S>
+template <class S>
 __device__ __forceinline__ void ew_tsum(const int32_t *s_row, int n, int t0, int t1, int tid, const S *__restrict__ sf,
-                                        T m, S *__restrict__ out) {
+                                        double m, S *__restrict__ out) {
     for (int t = t0 + tid; t < t1; t += 64) {
-        S a = sep_zero<S>();
+        S a{};
 #pragma unroll 8
         for (int u = 0; u < n; u++) sep_madd(a, m, sf[(int64_t)s_row[u] * (t1 - t0) + t - t0]);
         out[t] = a;
     }
 }
-/* the same in a launch of its own, for the chunks from `first` on */
-template <class T, class S>
-__global__ void __launch_bounds__(64) k_ewald_tsum(T m, bool fine, const int32_t *__restrict__ leaves, int32_t nleaves,
-                                                   int32_t first, const int32_t *__restrict__ off, ListView LV,
-                                                   const int32_t *__restrict__ slot, int t0, int t1,
+/* the same in a launch of its own, for the chunks from `first` on, rows of N vectors */
+template <class S>
+__global__ void __launch_bounds__(64) k_ewald_tsum(int N, double m, bool fine, const int32_t *__restrict__ leaves,
+                                                   int32_t nleaves, int32_t first, const int32_t *__restrict__ off,
+                                                   ListView LV, const int32_t *__restrict__ slot, int t0, int t1,
                                                    const S *__restrict__ sf, S *__restrict__ tpart) {
     __shared__ int32_t s_row[EW_KPP_MAX];
     const int tid = threadIdx.x;
@@ -122,20 +125,18 @@ __global__ void __launch_bounds__(64) k_ewald_tsum(T m, bool fine, const int32_t
     const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len, fine), e0 = k * kpp, e1 = min(len, e0 + kpp);
     if (tid < e1 - e0) s_row[tid] = slot[lst[e0 + tid]];
     __syncthreads();
-    ew_tsum<T, S>(s_row, e1 - e0, t0, t1, tid, sf, m, tpart + (int64_t)blockIdx.x * Sep<T>::N);
+    ew_tsum<S>(s_row, e1 - e0, t0, t1, tid, sf, m, tpart + (int64_t)blockIdx.x * N);
 }
 
 /* one chunk of a PP_E list: entries [k ew_kpp, ...) of its leaf.  The
  * real-space part per pair and, with sf (all vectors), the chunk's reciprocal
  * source sums (tpart).  Block b takes chunk first + b, its slot is b. */
 template <class T>
-__global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
+__global__ void __launch_bounds__(64, sizeof(T) == 4 ? EW_MINB_F : 12)
     k_ewald_pp(GParams P, bool fine, const int32_t *__restrict__ leaves, int32_t nleaves, int32_t first,
-               const int32_t *__restrict__ off,
-               const int32_t *__restrict__ pb, const int32_t *__restrict__ pe, const int4 *__restrict__ pos, ListView LV,
-               EwaldTables E, double *__restrict__ part, const int32_t *__restrict__ slot,
-               const typename Sep<T>::T2 *__restrict__ sf, typename Sep<T>::T2 *__restrict__ tpart) {
-    typedef typename Sep<T>::T2 T2;
+               const int32_t *__restrict__ off, const int32_t *__restrict__ pb, const int32_t *__restrict__ pe,
+               const int4 *__restrict__ pos, ListView LV, EwaldTables E, SepNear K, double *__restrict__ part,
+               const int32_t *__restrict__ slot, const double2 *__restrict__ sf, double2 *__restrict__ tpart) {
     __shared__ int4 sy[64];
     __shared__ int32_t s_row[EW_KPP_MAX];
     const int tid = threadIdx.x;
@@ -145,12 +146,10 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
     const int32_t b = pb[leaf], cnt = pe[leaf] - b;
     const bool active = tid < cnt;
     const int4 xi = pos[b + (active ? tid : 0)];
-    Acc<T> aphi, ag[3];
-    aphi.init(0.0);
-    for (int d = 0; d < 3; d++) ag[d].init(0.0);
+    SepPairs<T> s;
+    s.init();
     const int32_t *lst = LV.pool[TG_PP_E] + LV.off[TG_PP_E][leaf];
     const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len, fine), e0 = k * kpp, e1 = min(len, e0 + kpp);
-    const T m = T(P.m_d);
     if (tid < e1 - e0) s_row[tid] = slot[lst[e0 + tid]];
     for (int32_t e = e0; e < e1; e++) {
         const int32_t src = lst[e];
@@ -159,22 +158,12 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
         if (tid < sn) sy[tid] = pos[sb + tid];
         __syncthreads();
         if (tid < ((cnt + 31) & ~31)) /* a warp without sinks only stages */
-            for (int32_t q = 0; q < sn; q++) {
-                const int4 y = sy[q];
-                const T dX[3] = {wrap_sep_t<T>(xi.x, y.x), wrap_sep_t<T>(xi.y, y.y), wrap_sep_t<T>(xi.z, y.z)};
-                T ph, g[3];
-                pp_ewald_pair_sep<T>(E, dX, ph, g);
-                aphi.add(m * ph);
-                for (int d = 0; d < 3; d++) ag[d].add(m * g[d]);
-            }
+            for (int32_t q = 0; q < sn; q++) s.add(E, K, P.m_d, xi, sy[q]);
     }
-    if (active) {
-        double *o = part + 4 * ((int64_t)blockIdx.x * 64 + tid);
-        o[0] = aphi.get();
-        for (int d = 0; d < 3; d++) o[1 + d] = ag[d].get();
-    }
+    if (active)
+        for (int q = 0; q < 4; q++) part[4 * ((int64_t)blockIdx.x * 64 + tid) + q] = s.get(q, P.m_d);
     /* this chunk's reciprocal source sums, a thread per vector (s_row: written before the loop's barriers) */
-    if (sf) ew_tsum<T, T2>(s_row, e1 - e0, 0, Sep<T>::N, tid, sf, m, tpart + (int64_t)blockIdx.x * Sep<T>::N);
+    if (sf) ew_tsum<double2>(s_row, e1 - e0, 0, Sep<T>::N, tid, sf, P.m_d, tpart + (int64_t)blockIdx.x * Sep<T>::N);
 }
 
 /* one chunk of a PC_E list: block b takes chunk first + b (offp: the PC_E part of the scan), its slot is slot0 + b */
@@ -223,9 +212,9 @@ template <class T>
 __global__ void __launch_bounds__(256) k_ewald_reduce(EwBatch B, const int32_t *__restrict__ leaves, int32_t nleaves,
                                                       const int32_t *__restrict__ off, const int32_t *__restrict__ pb,
                                                       const int32_t *__restrict__ pe, const double *__restrict__ part,
-                                                      double *__restrict__ acc,
-                                                      const typename Sep<T>::T2 *__restrict__ tpart,
+                                                      double *__restrict__ acc, const double2 *__restrict__ tpart,
                                                       const int4 *__restrict__ pos, EwaldTables E) {
+    __shared__ SepTrig<T> trig;
     __shared__ double2 sT[Sep<T>::N];
     __shared__ double sv[4][64][4];
     const int32_t li = B.l0 + blockIdx.x;
@@ -241,14 +230,16 @@ __global__ void __launch_bounds__(256) k_ewald_reduce(EwBatch B, const int32_t *
         for (int i = tid; i < Sep<T>::N; i += 256) {
             double sx = 0.0, sy = 0.0;
             for (int64_t c = a0; c < a1; c++) {
-                const typename Sep<T>::T2 f = tpart[c * Sep<T>::N + i];
-                sx += (double)f.x;
-                sy += (double)f.y;
+                const double2 f = tpart[c * Sep<T>::N + i];
+                sx += f.x;
+                sy += f.y;
             }
-            sT[i] = make_double2(sx, sy);
+            const double w = sizeof(T) == 4 ? __ldg(&E.sep_w[i]) : 1.0; /* FP32: the weight here */
+            sT[i] = make_double2(w * sx, w * sy);
         }
+        sep_trig<T>(trig, pos + b, cnt);
         __syncthreads();
-        if (t < cnt) sep_eval<T>(E, sT, grp, 4, pos[b + t], v[0], v + 1);
+        if (t < cnt) sep_eval<T>(E, trig, sT, grp, t, pos + b, v[0], v + 1);
     }
 #pragma unroll
     for (int q = 0; q < 4; q++) sv[grp][t][q] = v[q];

@@ -669,7 +669,7 @@ __global__ void k_seam_node(GParams P, int kind_ewald, int is_cc, int64_t ngroup
 
 static EwaldTables tables(Solver &S) {
     return EwaldTables{S.ew_real.p,  S.ew_four.p, S.ew_Hf.p,  S.ew_Hd.p,  S.ew_Pf.p, S.ew_Pd.p,
-                       S.ew_sep_h.p, S.ew_sep_w.p, S.ew_sep_k, S.ew_sep_r0, S.ew_sep_r2, S.ew_tab};
+                       S.ew_sep_h.p, S.ew_sep_run.p, S.ew_sep_nrun, S.ew_sep_w.p, S.ew_sep_k, S.ew_sep_r0, S.ew_sep_r2, S.ew_tab};
 }
 
 static ListView listview(Solver &S) {
@@ -787,26 +787,25 @@ static int ew_vectors(const Solver &S, int32_t nsrc, size_t bytes, int N) {
  * to the FP64 accumulators accd (leaf_max <= 64) */
 template <class T>
 static int leaf_ewald(Solver &S, const GParams &P, const ListView &LV, const EwaldTables &E, cudaStream_t st) {
-    typedef typename Sep<T>::T2 T2;
     constexpr int N = Sep<T>::N;
     const int32_t nleaves = (int32_t)S.st.leaves;
     int32_t npp = 0, total = 0, nsrc = 0;
     TG_TRY(leaf_chunks(S, LV, npp, total, nsrc, st));
     if (total <= 0) return TG_OK;
     std::vector<EwBatch> batches;
-    TG_TRY(leaf_batches(S, npp, total, (256 * sizeof(double)) + N * sizeof(T2), 256 * sizeof(double), batches, st));
+    TG_TRY(leaf_batches(S, npp, total, (256 * sizeof(double)) + N * sizeof(double2), 256 * sizeof(double), batches, st));
     size_t slots = 0, sums = 0;
     for (const EwBatch &B : batches) {
         slots = std::max(slots, (size_t)B.na + B.nc);
         sums = std::max(sums, (size_t)B.na);
     }
-    const int nv = ew_vectors(S, nsrc, sizeof(T2), N);
+    const int nv = ew_vectors(S, nsrc, sizeof(double2), N);
     TG_TRY(ensure(S.ew_part, slots * 64 * 4));
     if (npp > 0) {
-        TG_TRY(ensure(S.ew_sf, (size_t)nsrc * nv * sizeof(T2)));
-        TG_TRY(ensure(S.ew_tpart, sums * N * sizeof(T2)));
+        TG_TRY(ensure(S.ew_sf, (size_t)nsrc * nv * sizeof(double2)));
+        TG_TRY(ensure(S.ew_tpart, sums * N * sizeof(double2)));
     }
-    T2 *sf = reinterpret_cast<T2 *>(S.ew_sf.p), *tpart = reinterpret_cast<T2 *>(S.ew_tpart.p);
+    double2 *sf = reinterpret_cast<double2 *>(S.ew_sf.p), *tpart = reinterpret_cast<double2 *>(S.ew_tpart.p);
     const int32_t *offp = S.ew_off.p + nleaves + 1;
     const bool fine = ew_fine(S);
     if (npp > 0 && nv == N) {
@@ -816,15 +815,15 @@ static int leaf_ewald(Solver &S, const GParams &P, const ListView &LV, const Ewa
     for (const EwBatch &B : batches) {
         if (B.na > 0) {
             k_ewald_pp<T><<<B.na, 64, 0, st>>>(P, fine, S.idx.p, nleaves, B.a0, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p,
-                                               LV, E, S.ew_part.p, S.ew_slot.p, nv == N ? sf : nullptr, tpart);
+                                               LV, E, S.ew_near, S.ew_part.p, S.ew_slot.p, nv == N ? sf : nullptr, tpart);
             TG_TRY(launched(S));
         }
         for (int t0 = 0; B.na > 0 && nv < N && t0 < N; t0 += nv) {
             const int t1 = std::min(N, t0 + nv);
             k_ewald_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E, t0, t1, sf);
             TG_TRY(launched(S));
-            k_ewald_tsum<T, T2><<<B.na, 64, 0, st>>>(T(P.m_d), fine, S.idx.p, nleaves, B.a0, S.ew_off.p, LV, S.ew_slot.p,
-                                                     t0, t1, sf, tpart);
+            k_ewald_tsum<double2><<<B.na, 64, 0, st>>>(N, P.m_d, fine, S.idx.p, nleaves, B.a0, S.ew_off.p, LV, S.ew_slot.p,
+                                                       t0, t1, sf, tpart);
             TG_TRY(launched(S));
         }
         if (B.nc > 0) {

@@ -153,10 +153,13 @@ struct Solver {
     DevBuf<double2> ew_Pd;
     DevBuf<int4> ew_sep_h;       /* PP Ewald split: reciprocal vectors and weights */
     DevBuf<double> ew_sep_w;
+    DevBuf<int4> ew_sep_run; /* FP32: runs of the vectors */
+    int ew_sep_nrun = 0;
     double ew_sep_k = 0.0, ew_sep_r0 = 0.0, ew_sep_r2 = 0.0;
+    SepNear ew_near{}; /* FP32 path */
     DevBuf<int32_t> ew_slot, ew_src; /* per node: its row of ew_sf, or -1; the nodes of the rows, then their count */
-    DevBuf<unsigned char> ew_sf;    /* per PP_E source leaf and h: (cos, sin) sums over its particles (Sep<T>::T2) */
-    DevBuf<unsigned char> ew_tpart; /* per PP_E chunk and h: source sums (Sep<T>::T2) */
+    DevBuf<unsigned char> ew_sf;    /* per PP_E source leaf and h: (cos, sin) sums over its particles (double2) */
+    DevBuf<unsigned char> ew_tpart; /* per PP_E chunk and h: source sums (double2) */
     size_t ew_scratch = EW_SCRATCH;
     bool ew_use_tab = false;       /* a periodic solver of the FP32 path */
     const float *ew_tab = nullptr; /* the device's table of local expansions (FP32 path), shared by its solvers */
