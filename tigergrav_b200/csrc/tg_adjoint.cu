@@ -796,8 +796,12 @@ __global__ void k_axpy3(int64_t n, double c, const double *__restrict__ x, doubl
     y[i] += c * x[i];
 }
 
-/* the buffers and kernels of tidal_apply, taken ahead of the first backward pass */
+/* The buffers and kernels of tidal_apply, taken ahead of the first backward pass: an
+ * allocation waits for the device, and took 0.2 to 0.7 s on some machines.  The Ewald
+ * scratch is sized by the largest lists of the solver's force evaluations, which are
+ * those of the checkpoints. */
 int tidal_reserve(Solver &S) {
+    const bool f64 = S.prm.precision == TG_PREC_F64, small = S.prm.leaf_max <= 64;
     TG_TRY(ensure(S.adj_x, 3 * S.n));
     TG_TRY(ensure(S.adj_v, 3 * S.n));
     TG_TRY(ensure(S.tid_u, 3 * S.n));
@@ -805,13 +809,23 @@ int tidal_reserve(Solver &S) {
     TG_TRY(ensure(S.tid_U, 3 * S.nnodes));
     TG_TRY(ensure(S.tid_V, 6 * S.nnodes));
     TG_TRY(ensure(S.tid_tile, 3 * ((S.n + USUM_TILE - 1) / USUM_TILE)));
-    const bool f64 = S.prm.precision == TG_PREC_F64;
-    const void *k[] = {f64 ? (const void *)k_vfield_node<double> : (const void *)k_vfield_node<float>,
-                       f64 ? (const void *)k_tidal_leaf<double, 64, false> : (const void *)k_tidal_leaf<float, 64, false>,
+    if (S.ew_max_npp > 0) { /* as tidal_ewald */
+        const int N = f64 ? Sep<double>::N : Sep<float>::N;
+        const size_t slots = std::min<size_t>(S.ew_max_npp, S.ew_scratch / tidal_chunk_bytes(N) + 1);
+        TG_TRY(ensure(S.ew_part, slots * 64 * 3));
+        TG_TRY(ensure(S.ew_tpart, slots * N * sizeof(Sep4)));
+        TG_TRY(ensure(S.ew_sf, (size_t)S.ew_max_nsrc * ew_vectors(S, S.ew_max_nsrc, sizeof(Sep4), N) * sizeof(Sep4)));
+    }
+    const void *leaf = small ? (f64 ? (const void *)k_tidal_leaf<double, 64, false> : (const void *)k_tidal_leaf<float, 64, false>)
+                             : (f64 ? (const void *)k_tidal_leaf<double, 128, true> : (const void *)k_tidal_leaf<float, 128, true>);
+    const void *k[] = {leaf,
+                       f64 ? (const void *)k_vfield_node<double> : (const void *)k_vfield_node<float>,
                        f64 ? (const void *)k_tidal_pp<double> : (const void *)k_tidal_pp<float>,
                        f64 ? (const void *)k_tidal_sf<double> : (const void *)k_tidal_sf<float>,
                        f64 ? (const void *)k_tidal_ewald_pp<double> : (const void *)k_tidal_ewald_pp<float>,
-                       f64 ? (const void *)k_tidal_ewald_reduce<double> : (const void *)k_tidal_ewald_reduce<float>};
+                       f64 ? (const void *)k_tidal_ewald_reduce<double> : (const void *)k_tidal_ewald_reduce<float>,
+                       (const void *)k_gather3, (const void *)k_tile_usum, (const void *)k_node_usum,
+                       (const void *)k_vfield_down, (const void *)k_scatter_axpy3, (const void *)k_axpy3};
     cudaFuncAttributes a;
     for (const void *f : k) TG_CUDA(cudaFuncGetAttributes(&a, f)); /* loads the kernel's code */
     return TG_OK;

@@ -574,7 +574,6 @@ int tg_forward(tg_solver *s, double dt, int n_steps, void *stream) {
     TG_TRY(ensure(S.ck_v, (size_t)3 * n * (n_steps + 1)));
     S.ck_steps = -1;
     if (!S.have_forces) TG_TRY(tg_solve_gravity(s, stream));
-    TG_TRY(tidal_reserve(S));
     const int gn = (int)((n + 255) / 256);
     k_unpack<<<gn, 256, 0, st>>>(n, S.pos.p, S.vel.p, S.ck_x.p, S.ck_v.p);
     TG_TRY(launched(S));
@@ -587,6 +586,7 @@ int tg_forward(tg_solver *s, double dt, int n_steps, void *stream) {
                                      S.ck_v.p + (size_t)3 * n * (k + 1));
         TG_TRY(launched(S));
     }
+    TG_TRY(tidal_reserve(S));
     S.ck_steps = n_steps;
     S.ck_dt = dt;
     return TG_OK;

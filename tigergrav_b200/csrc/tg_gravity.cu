@@ -751,6 +751,8 @@ static int leaf_chunks(Solver &S, const ListView &LV, int32_t &npp, int32_t &tot
     int32_t tot[3];
     std::memcpy(tot, S.h_small + 2048, sizeof(tot));
     npp = tot[0], total = tot[1], nsrc = tot[2];
+    S.ew_max_npp = std::max(S.ew_max_npp, npp);
+    S.ew_max_nsrc = std::max(S.ew_max_nsrc, nsrc);
     return TG_OK;
 }
 

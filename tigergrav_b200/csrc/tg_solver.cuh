@@ -161,6 +161,7 @@ struct Solver {
     DevBuf<unsigned char> ew_sf;    /* per PP_E source leaf and h: (cos, sin) sums over its particles (double2) */
     DevBuf<unsigned char> ew_tpart; /* per PP_E chunk and h: source sums (double2) */
     size_t ew_scratch = EW_SCRATCH;
+    int32_t ew_max_npp = 0, ew_max_nsrc = 0; /* most PP_E chunks and source leaves of any evaluation */
     bool ew_use_tab = false;       /* a periodic solver of the FP32 path */
     const float *ew_tab = nullptr; /* the device's table of local expansions (FP32 path), shared by its solvers */
     bool have_tables = false;
