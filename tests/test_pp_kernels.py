@@ -33,10 +33,10 @@ CASES = {
     "short_48": (lambda: _uniform(20000, 4), 0.7, 48, True, None),
     "short_leaf7": (lambda: _uniform(6000, 5), 0.6, 7, True, None),
     "short_free_soft": (lambda: _clumps(9000, 6), 0.6, 32, False, 2e-3),
-    "long_leaf1": (lambda: _uniform(2000, 7), 0.3, 1, True, None),
-    "long_leaf12": (lambda: _uniform(9000, 8), 0.3, 12, True, None),
-    "long_leaf26": (lambda: _uniform(17000, 9), 0.3, 26, False, None),
-    "long_clumps_58": (lambda: _clumps(40000, 10), 0.3, 58, False, 1e-3),
+    "long_leaf1": (lambda: _uniform(2000, 7), 0.25, 1, True, None),
+    "long_leaf12": (lambda: _uniform(9000, 8), 0.25, 12, True, None),
+    "long_leaf26": (lambda: _uniform(17000, 9), 0.25, 26, False, None),
+    "long_clumps_58": (lambda: _clumps(40000, 10), 0.25, 58, False, 1e-3),
 }
 
 

@@ -870,14 +870,20 @@ static int node_stage(Solver &S, const GParams &P, const ListView &LV, const Ewa
 /* PP direct of the FP32 path (leaf_max <= 64): far + PP_direct - phi_self into acc.
  * A list holds about 17 / theta^3 source leaves (leaves within (r_a + r_b) / theta,
  * at most all of them).  From PPB_LONG on, or with fewer leaves than SMs,
- * k_pp_long is the faster one: ms with k_pp_short / k_pp_long at 40 leaves per
- * list (128^3, theta 0.7) 4.2 / 4.6, 95 (101^3, theta 0.5) 2.9 / 3.4, 1800 (128^3,
- * theta 0.2) 112 / 102, 2100 (256^3, theta 0.19) 731 / 662; 92 leaves with 92 each
- * (4096 uniform) 0.175 / 0.050 in quarters.  Fewer leaves than one wave of blocks:
+ * k_pp_long is the faster one.  ms with k_pp_short / k_pp_long by that length:
+ *   128^3 clustered, leaf 64   50: 4.08 / 4.57   266: 20.8 / 23.1   397: 29.4 / 32.2
+ *                             630: 40.4 / 40.4   967: 55.3 / 52.5  2125: 107 / 98
+ *   101^3 clustered, leaf 32  397: 7.56 / 8.74   864: 13.0 / 13.1  1597: 21.3 / 20.4
+ *   101^3 uniform, leaf 48    266: 7.89 / 8.85   630: 16.9 / 18.2  1230: 27.1 / 25.7
+ *   64^3 clustered, leaf 64   397: 4.18 / 4.48   774: 6.81 / 6.47
+ *   64^3 clustered, leaf 16   397: 1.60 / 1.73   774: 2.67 / 2.70  1597: 4.99 / 4.71
+ *   64^3 halos (free), leaf 32  266: 1.65 / 1.78  630: 2.84 / 2.93  1088: 4.06 / 3.94
+ * and 256^3, leaf 48, 2480: 731 / 662.  92 leaves with 92 each (4096 uniform) 0.175 /
+ * 0.050 in quarters.  Fewer leaves than one wave of blocks:
  * the lists are cut into shares so that the wave is full (4096 uniform: 0.79 ms
  * without).  The choice depends on the tree alone, not on which leaves are
  * active, so a rung step's forces equal a full solve's bit for bit. */
-constexpr int PPB_LONG = 512;
+constexpr int PPB_LONG = 800;
 static int pp_direct(Solver &S, const GParams &P, const ListView &LV, cudaStream_t st) {
     const int64_t n = S.n, nn = S.nnodes;
     const int32_t nleaves = (int32_t)S.st.leaves;
