@@ -1,7 +1,7 @@
 """PP direct and the pair part of the Jacobian product at the edges of the CUDA
 kernels' ranges: sink leaves of 1 to 64 particles (every cut into lanes and
-copies), lists below and above the length where the kernel changes, fewer
-leaves than SMs (list shares, quarters of leaves), sources about half a box
+copies), lists below and above the length where the kernel changes, lists
+of a large part of the tree (shares, quarters of leaves), sources about half a box
 away (offsets beyond the int32 range), softened pairs."""
 import numpy as np
 import pytest
@@ -30,9 +30,13 @@ CASES = {
     "few_leaves_64": (lambda: _uniform(4096, 1), 0.7, 64, True, None),
     "few_leaves_one": (lambda: _uniform(61, 2), 0.7, 64, True, None),
     "few_free_33": (lambda: _uniform(1500, 3), 0.5, 33, False, None),
-    "short_48": (lambda: _uniform(20000, 4), 0.7, 48, True, None),
-    "short_leaf7": (lambda: _uniform(6000, 5), 0.6, 7, True, None),
-    "short_free_soft": (lambda: _clumps(9000, 6), 0.6, 32, False, 2e-3),
+    "wide_48": (lambda: _uniform(20000, 4), 0.7, 48, True, None),
+    "wide_leaf7": (lambda: _uniform(6000, 5), 0.6, 7, True, None),
+    "wide_free_soft": (lambda: _clumps(9000, 6), 0.6, 32, False, 2e-3),
+    "short_24": (lambda: _uniform(20000, 4), 0.7, 24, True, None),
+    "short_leaf7": (lambda: _uniform(6000, 5), 0.7, 7, True, None),
+    "short_free_soft": (lambda: _clumps(12000, 6), 0.7, 16, False, 2e-3),
+    "short_free_60": (lambda: _clumps(60000, 7), 0.8, 60, False, 1e-3),
     "long_leaf1": (lambda: _uniform(2000, 7), 0.25, 1, True, None),
     "long_leaf12": (lambda: _uniform(9000, 8), 0.25, 12, True, None),
     "long_leaf26": (lambda: _uniform(17000, 9), 0.25, 26, False, None),

@@ -869,8 +869,10 @@ static int node_stage(Solver &S, const GParams &P, const ListView &LV, const Ewa
 
 /* PP direct of the FP32 path (leaf_max <= 64): far + PP_direct - phi_self into acc.
  * A list holds about 17 / theta^3 source leaves (leaves within (r_a + r_b) / theta,
- * at most all of them).  From PPB_LONG on, or with fewer leaves than SMs,
- * k_pp_long is the faster one.  ms with k_pp_short / k_pp_long by that length:
+ * at most all of them).
+ *
+ * From PPB_LONG on k_pp_long (whole leaves per warp) is the faster one of the two.
+ * ms with k_pp_short / k_pp_long by that length:
  *   128^3 clustered, leaf 64   50: 4.08 / 4.57   266: 20.8 / 23.1   397: 29.4 / 32.2
  *                             630: 40.4 / 40.4   967: 55.3 / 52.5  2125: 107 / 98
  *   101^3 clustered, leaf 32  397: 7.56 / 8.74   864: 13.0 / 13.1  1597: 21.3 / 20.4
@@ -878,12 +880,24 @@ static int node_stage(Solver &S, const GParams &P, const ListView &LV, const Ewa
  *   64^3 clustered, leaf 64   397: 4.18 / 4.48   774: 6.81 / 6.47
  *   64^3 clustered, leaf 16   397: 1.60 / 1.73   774: 2.67 / 2.70  1597: 4.99 / 4.71
  *   64^3 halos (free), leaf 32  266: 1.65 / 1.78  630: 2.84 / 2.93  1088: 4.06 / 3.94
- * and 256^3, leaf 48, 2480: 731 / 662.  92 leaves with 92 each (4096 uniform) 0.175 /
- * 0.050 in quarters.  Fewer leaves than one wave of blocks:
- * the lists are cut into shares so that the wave is full (4096 uniform: 0.79 ms
- * without).  The choice depends on the tree alone, not on which leaves are
- * active, so a rung step's forces equal a full solve's bit for bit. */
-constexpr int PPB_LONG = 800;
+ * and 256^3, leaf 48, 2480: 731 / 662 (703 in quarters).
+ *
+ * A list of at least 1 / PPB_WIDE of the tree's leaves reaches half a box, where
+ * k_pp_short takes whole stages pair by pair; below PPB_LONG k_pp_long in quarters
+ * of leaves takes those.  ms with k_pp_short / k_pp_long in quarters by the share:
+ *   leaf 64, uniform   0.54: 0.165 / 0.052 (4096)     0.17: 0.581 / 0.108 (14000)
+ *     0.13: 2.43 / 2.23 (1e5)  0.10: 0.325 / 0.087 (20000)  0.07: 0.122 / 0.124 (32768)
+ *     0.06: 2.44 / 2.48 (2e5)  0.05: 0.208 / 0.220 (50000)  0.03: 1.26 / 1.27 (2e5)
+ *   leaf 32, clustered 0.22: 0.458 / 0.112  0.09: 0.243 / 0.220  0.05: 0.302 / 0.312
+ *   leaf 16, uniform   0.13: 0.400 / 0.151  0.07: 0.063 / 0.040  0.05: 0.218 / 0.243
+ *   leaf 32, halos (free)  0.12: 0.355 / 0.083  0.06: 0.435 / 0.112  0.05: 1.32 / 0.79
+ *                          0.03: 0.189 / 0.196
+ *
+ * Fewer leaves than one wave of blocks: the lists are cut into shares so that the
+ * wave is full (4096 uniform: 0.79 ms without).  The choices depend on the tree alone,
+ * not on which leaves are active, so a rung step's forces equal a full solve's bit
+ * for bit. */
+constexpr int PPB_LONG = 800, PPB_WIDE = 20;
 static int pp_direct(Solver &S, const GParams &P, const ListView &LV, cudaStream_t st) {
     const int64_t n = S.n, nn = S.nnodes;
     const int32_t nleaves = (int32_t)S.st.leaves;
@@ -893,7 +907,7 @@ static int pp_direct(Solver &S, const GParams &P, const ListView &LV, cudaStream
     TG_TRY(launched(S));
     const int64_t tree = tree_leaves(S);
     const double list = std::min(17.0 / (S.prm.theta * S.prm.theta * S.prm.theta), (double)tree);
-    const bool few = tree < S.num_sms, longl = few || list >= PPB_LONG;
+    const bool whole = list >= PPB_LONG, quarter = !whole && list * PPB_WIDE >= (double)tree, longl = whole || quarter;
     const int wave = S.num_sms * (longl ? PPL_MINB : PPS_MINB);
     const int shares = tree >= wave ? 1 : (int)std::min<int64_t>((wave + tree - 1) / tree, PPB_SHARES);
     double *part = nullptr;
@@ -902,7 +916,7 @@ static int pp_direct(Solver &S, const GParams &P, const ListView &LV, cudaStream
         part = S.pp_part.p;
     }
     const dim3 g(nleaves, shares);
-    if (few)
+    if (quarter)
         k_pp_long<true><<<g, PPB_T, 0, st>>>(P, S.idx.p, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p, rec, S.pos.p, LV, S.accd.p,
                                              S.acc.p, part, n);
     else if (longl)
