@@ -603,7 +603,7 @@ template <> struct TidalPairs<float> {
 /* one chunk of a PP_E list (as k_ewald_pp): the real-space part per pair into
  * part (3 per sink) and, with sf, the reciprocal source sums into tpart */
 template <class T>
-__global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, bool fine, const int32_t *__restrict__ leaves, int32_t nleaves,
+__global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, const int32_t *__restrict__ leaves, int32_t nleaves,
                                                        int32_t first, const int32_t *__restrict__ off, const int32_t *__restrict__ pb,
                                                        const int32_t *__restrict__ pe, const int4 *__restrict__ pos,
                                                        ListView LV, EwaldTables E, SepNear K, const double *__restrict__ u,
@@ -622,7 +622,7 @@ __global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, bool fine, con
     TidalPairs<T> o;
     o.init(u + 3 * i);
     const int32_t *lst = LV.pool[TG_PP_E] + LV.off[TG_PP_E][leaf];
-    const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len, fine), e0 = k * kpp, e1 = min(len, e0 + kpp);
+    const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len), e0 = k * kpp, e1 = min(len, e0 + kpp);
     if (tid < e1 - e0) s_row[tid] = slot[lst[e0 + tid]];
     for (int32_t e = e0; e < e1; e++) {
         const int32_t src = lst[e];
@@ -746,21 +746,20 @@ static int tidal_ewald(Solver &S, const GParams &P, const ListView &LV, const Ew
     TG_TRY(ensure(S.ew_sf, (size_t)nsrc * nv * sizeof(Sep4)));
     TG_TRY(ensure(S.ew_tpart, slots * N * sizeof(Sep4)));
     Sep4 *sf = reinterpret_cast<Sep4 *>(S.ew_sf.p), *tpart = reinterpret_cast<Sep4 *>(S.ew_tpart.p);
-    const bool fine = ew_fine(S);
     if (nv == N) {
         k_tidal_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, S.tid_u.p, E, 0, N, sf);
         TG_TRY(launched(S));
     }
     for (const EwBatch &B : batches) {
         if (B.na == 0) continue;
-        k_tidal_ewald_pp<T><<<B.na, 64, 0, st>>>(P, fine, S.idx.p, nleaves, B.a0, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p,
+        k_tidal_ewald_pp<T><<<B.na, 64, 0, st>>>(P, S.idx.p, nleaves, B.a0, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p,
                                                  LV, E, S.ew_near, S.tid_u.p, S.ew_part.p, S.ew_slot.p, nv == N ? sf : nullptr, tpart);
         TG_TRY(launched(S));
         for (int t0 = 0; nv < N && t0 < N; t0 += nv) {
             const int t1 = std::min(N, t0 + nv);
             k_tidal_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, S.tid_u.p, E, t0, t1, sf);
             TG_TRY(launched(S));
-            k_ewald_tsum<Sep4><<<B.na, 64, 0, st>>>(N, P.m_d, fine, S.idx.p, nleaves, B.a0, S.ew_off.p, LV, S.ew_slot.p, t0,
+            k_ewald_tsum<Sep4><<<B.na, 64, 0, st>>>(N, P.m_d, S.idx.p, nleaves, B.a0, S.ew_off.p, LV, S.ew_slot.p, t0,
                                                     t1, sf, tpart);
             TG_TRY(launched(S));
         }

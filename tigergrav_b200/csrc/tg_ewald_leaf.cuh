@@ -27,15 +27,15 @@
 #pragma once
 
 constexpr int EW_KPP_MAX = 32;
-/* PP_E source leaves per chunk: 16 chunks of a list, of 8 to 32 leaves (at most
- * 32 * 64 * 64 pairs).  Each chunk's slots take 5 KB in FP32, so chunks of 8
- * throughout hold 225 MB for 32768 particles where these hold 60 MB.  fine (a tree
- * with fewer leaves than twice the SMs): up to 24 chunks, of 4 leaves on, which
- * fill the GPU (4096 particles: leaf Ewald and L2P 0.41 -> 0.33 ms).  By the list and the tree alone, so the order of the sums does not
- * depend on which leaves are active. */
-__host__ __device__ __forceinline__ int32_t ew_kpp(int32_t len, bool fine) {
-    const int32_t k = fine ? (len + 23) / 24 : (len + 15) >> 4, lo = fine ? 4 : 8;
-    return k < lo ? lo : (k > EW_KPP_MAX ? EW_KPP_MAX : k);
+/* PP_E source leaves per chunk: 24 chunks of a list, of 4 to 32 leaves (at most
+ * 32 * 64 * 64 pairs), so that small trees fill the GPU.  Leaf Ewald and L2P in ms
+ * with 16 chunks of 8 leaves on / with 24 of 4 on (theta 0.7, leaf 64): 4096 uniform
+ * 0.40 / 0.31, 20000 0.77 / 0.72, 32768 0.92 / 0.84, 50000 0.61 / 0.53, 1e5 and more,
+ * and theta 0.25 to 0.5, the same.  By the list alone, so the order of the sums does
+ * not depend on which leaves are active. */
+__host__ __device__ __forceinline__ int32_t ew_kpp(int32_t len) {
+    const int32_t k = (len + 23) / 24;
+    return k < 4 ? 4 : (k > EW_KPP_MAX ? EW_KPP_MAX : k);
 }
 constexpr int EW_KPC = 64; /* PC_E source nodes per chunk */
 #ifndef EW_MINB_F
@@ -51,7 +51,7 @@ struct EwBatch {
 /* one warp per leaf: chunk counts (zeros at li = nleaves, so that the scan ends
  * in the totals); with slot, marks the source leaves of the PP_E lists */
 __global__ void k_ewald_count(const int32_t *__restrict__ leaves, int32_t nleaves, ListView LV,
-                              int32_t *__restrict__ cnt, int32_t *__restrict__ slot, bool fine) {
+                              int32_t *__restrict__ cnt, int32_t *__restrict__ slot) {
     const int32_t li = (int32_t)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (li > nleaves) return;
@@ -65,7 +65,7 @@ __global__ void k_ewald_count(const int32_t *__restrict__ leaves, int32_t nleave
         }
     }
     if (lane == 0) {
-        cnt[li] = (npp + ew_kpp(npp, fine) - 1) / ew_kpp(npp, fine);
+        cnt[li] = (npp + ew_kpp(npp) - 1) / ew_kpp(npp);
         cnt[nleaves + 1 + li] = (npc + EW_KPC - 1) / EW_KPC;
     }
 }
@@ -112,7 +112,7 @@ __device__ __forceinline__ void ew_tsum(const int32_t *s_row, int n, int t0, int
 }
 /* the same in a launch of its own, for the chunks from `first` on, rows of N vectors */
 template <class S>
-__global__ void __launch_bounds__(64) k_ewald_tsum(int N, double m, bool fine, const int32_t *__restrict__ leaves,
+__global__ void __launch_bounds__(64) k_ewald_tsum(int N, double m, const int32_t *__restrict__ leaves,
                                                    int32_t nleaves, int32_t first, const int32_t *__restrict__ off,
                                                    ListView LV, const int32_t *__restrict__ slot, int t0, int t1,
                                                    const S *__restrict__ sf, S *__restrict__ tpart) {
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(64) k_ewald_tsum(int N, double m, bool fine, c
     const int32_t li = ew_leaf(off, nleaves, c), k = (int32_t)(c - off[li]);
     const int32_t leaf = leaves[li];
     const int32_t *lst = LV.pool[TG_PP_E] + LV.off[TG_PP_E][leaf];
-    const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len, fine), e0 = k * kpp, e1 = min(len, e0 + kpp);
+    const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len), e0 = k * kpp, e1 = min(len, e0 + kpp);
     if (tid < e1 - e0) s_row[tid] = slot[lst[e0 + tid]];
     __syncthreads();
     ew_tsum<S>(s_row, e1 - e0, t0, t1, tid, sf, m, tpart + (int64_t)blockIdx.x * N);
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(64) k_ewald_tsum(int N, double m, bool fine, c
  * source sums (tpart).  Block b takes chunk first + b, its slot is b. */
 template <class T>
 __global__ void __launch_bounds__(64, sizeof(T) == 4 ? EW_MINB_F : 12)
-    k_ewald_pp(GParams P, bool fine, const int32_t *__restrict__ leaves, int32_t nleaves, int32_t first,
+    k_ewald_pp(GParams P, const int32_t *__restrict__ leaves, int32_t nleaves, int32_t first,
                const int32_t *__restrict__ off, const int32_t *__restrict__ pb, const int32_t *__restrict__ pe,
                const int4 *__restrict__ pos, ListView LV, EwaldTables E, SepNear K, double *__restrict__ part,
                const int32_t *__restrict__ slot, const double2 *__restrict__ sf, double2 *__restrict__ tpart) {
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? EW_MINB_F : 12)
     SepPairs<T> s;
     s.init();
     const int32_t *lst = LV.pool[TG_PP_E] + LV.off[TG_PP_E][leaf];
-    const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len, fine), e0 = k * kpp, e1 = min(len, e0 + kpp);
+    const int32_t len = LV.len[TG_PP_E][leaf], kpp = ew_kpp(len), e0 = k * kpp, e1 = min(len, e0 + kpp);
     if (tid < e1 - e0) s_row[tid] = slot[lst[e0 + tid]];
     for (int32_t e = e0; e < e1; e++) {
         const int32_t src = lst[e];

@@ -718,8 +718,6 @@ static int64_t tree_leaves(const Solver &S) {
     for (int64_t l : S.level_leaves) n += l;
     return n;
 }
-/* whether the PP_E chunks are the fine ones (ew_kpp) */
-static bool ew_fine(const Solver &S) { return tree_leaves(S) < 2 * S.num_sms; }
 
 /* The leaf Ewald lists cut into chunks (tg_ewald_leaf.cuh): their offsets in
  * ew_off, the PP_E source leaves in ew_src with their rows in ew_slot, and the
@@ -736,7 +734,7 @@ static int leaf_chunks(Solver &S, const ListView &LV, int32_t &npp, int32_t &tot
     TG_CUDA(cudaMemsetAsync(slot, 0xff, sizeof(int32_t) * nn, st));
     TG_CUDA(cudaMemsetAsync(nsrc_d, 0, sizeof(int32_t), st));
     k_ewald_count<<<(int)(((int64_t)(nleaves + 1) * 32 + 127) / 128), 128, 0, st>>>(S.idx.p, nleaves, LV, S.ew_cnt.p,
-                                                                                  slot, ew_fine(S));
+                                                                                  slot);
     TG_TRY(launched(S));
     k_ewald_slots<<<(int)((nn + 255) / 256), 256, 0, st>>>(nn, slot, S.ew_src.p, nsrc_d);
     TG_TRY(launched(S));
@@ -809,14 +807,13 @@ static int leaf_ewald(Solver &S, const GParams &P, const ListView &LV, const Ewa
     }
     double2 *sf = reinterpret_cast<double2 *>(S.ew_sf.p), *tpart = reinterpret_cast<double2 *>(S.ew_tpart.p);
     const int32_t *offp = S.ew_off.p + nleaves + 1;
-    const bool fine = ew_fine(S);
     if (npp > 0 && nv == N) {
         k_ewald_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E, 0, N, sf);
         TG_TRY(launched(S));
     }
     for (const EwBatch &B : batches) {
         if (B.na > 0) {
-            k_ewald_pp<T><<<B.na, 64, 0, st>>>(P, fine, S.idx.p, nleaves, B.a0, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p,
+            k_ewald_pp<T><<<B.na, 64, 0, st>>>(P, S.idx.p, nleaves, B.a0, S.ew_off.p, S.nd_pb.p, S.nd_pe.p, S.pos.p,
                                                LV, E, S.ew_near, S.ew_part.p, S.ew_slot.p, nv == N ? sf : nullptr, tpart);
             TG_TRY(launched(S));
         }
@@ -824,7 +821,7 @@ static int leaf_ewald(Solver &S, const GParams &P, const ListView &LV, const Ewa
             const int t1 = std::min(N, t0 + nv);
             k_ewald_sf<T><<<nsrc, 128, 0, st>>>(S.ew_src.p, S.nd_pb.p, S.nd_pe.p, S.pos.p, E, t0, t1, sf);
             TG_TRY(launched(S));
-            k_ewald_tsum<double2><<<B.na, 64, 0, st>>>(N, P.m_d, fine, S.idx.p, nleaves, B.a0, S.ew_off.p, LV, S.ew_slot.p,
+            k_ewald_tsum<double2><<<B.na, 64, 0, st>>>(N, P.m_d, S.idx.p, nleaves, B.a0, S.ew_off.p, LV, S.ew_slot.p,
                                                        t0, t1, sf, tpart);
             TG_TRY(launched(S));
         }
