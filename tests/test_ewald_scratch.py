@@ -17,7 +17,7 @@ def _run(x, u, precision, leaf, theta, scratch):
 
 # one leaf and one vector at a time; batches of a few leaves, ranges of vectors; several batches, all vectors
 @pytest.mark.parametrize("precision,n,leaf,scratch", [("f32", 400, 16, 1), ("f64", 300, 16, 1),
-                                                      ("f32", 5000, 16, 400_000), ("f64", 3000, 16, 1_500_000),
+                                                      ("f32", 5000, 16, 1_000_000), ("f64", 3000, 16, 1_500_000),
                                                       ("f32", 20000, 64, 1_000_000), ("f64", 9000, 40, 4_000_000)])
 def test_same_bits_within_the_bytes(precision, n, leaf, scratch):
     from tigergrav_b200 import ics
@@ -28,7 +28,8 @@ def test_same_bits_within_the_bytes(precision, n, leaf, scratch):
     assert np.array_equal(p0, p1) and np.array_equal(g0, g1) and np.array_equal(j0, j1)
     if scratch == 1:
         return
-    # a buffer holds at most the bytes, and a quarter more by its slack (ew_part is the nodes' too)
+    # a buffer holds at most the bytes (at least one leaf, whose 24 chunks fit here), and a quarter more by its slack
+    # (ew_part is the nodes' too)
     for full, small in ((r0, r1), (t0, t1)):
         for buf in ("ew_tpart", "ew_sf"):
             assert small[buf] <= 1.25 * scratch + 4096 < full[buf], buf

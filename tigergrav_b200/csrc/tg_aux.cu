@@ -146,7 +146,7 @@ int ewald_tables(Solver &S, cudaStream_t st) {
     const auto real = lattice(17), four = lattice(9);
     if ((int)real.size() != NREAL || (int)four.size() != NFOUR) return TG_ERR_STATE;
     std::vector<float4> r4(NREAL), f4;
-    /* device order: increasing |n|^2, so the first NREAL_F32 are the candidates of the FP32 cut */
+    /* device order: increasing |n|^2 */
     for (int i = 0; i < NREAL; i++) {
         const auto &v = real[NREAL - 1 - i];
         r4[i] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]));

@@ -21,7 +21,6 @@ constexpr int LP = 35;
 constexpr double POS_MAX = 4294967296.0;
 constexpr double POS_INV = 1.0 / 4294967296.0;
 constexpr int NREAL = 305;  /* |n|^2 <= 17 (tigergrav/green.hpp:3,8-28) */
-constexpr int NREAL_F32 = 123; /* |n|^2 <= 9: every n that can lie within the FP32 cut 2.1 of |X| <= sqrt(3)/2 */
 constexpr int NFOUR = 123;  /* |h|^2 <= 9 */
 constexpr int NFOUR_HALF = 61; /* one of each pair +-h (h != 0) */
 constexpr int HS = 36;         /* row stride of the coefficient tables (16-byte rows) */

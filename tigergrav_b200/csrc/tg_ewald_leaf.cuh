@@ -38,9 +38,6 @@ __host__ __device__ __forceinline__ int32_t ew_kpp(int32_t len) {
     return k < 4 ? 4 : (k > EW_KPP_MAX ? EW_KPP_MAX : k);
 }
 constexpr int EW_KPC = 64; /* PC_E source nodes per chunk */
-#ifndef EW_MINB_F
-#define EW_MINB_F 16 /* resident 64-thread blocks per SM that the FP32 pair kernel is compiled for */
-#endif
 
 /* leaves [l0, l1) with their PP_E chunks [a0, a0 + na) and PC_E chunks [c0, c0 + nc),
  * whose slots follow each other in that order */
@@ -130,9 +127,13 @@ __global__ void __launch_bounds__(64) k_ewald_tsum(int N, double m, const int32_
 
 /* one chunk of a PP_E list: entries [k ew_kpp, ...) of its leaf.  The
  * real-space part per pair and, with sf (all vectors), the chunk's reciprocal
- * source sums (tpart).  Block b takes chunk first + b, its slot is b. */
+ * source sums (tpart).  Block b takes chunk first + b, its slot is b.
+ *
+ * What bounds it: latency of the image and polynomial chains at 16 blocks per SM in
+ * FP32 (63 registers, issue 66 %, FP64 pipe 27 %): 0.69 ms at 32768 uniform (12 blocks
+ * 0.73, 14: 0.69; polynomials in even and odd halves 0.69). */
 template <class T>
-__global__ void __launch_bounds__(64, sizeof(T) == 4 ? EW_MINB_F : 12)
+__global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
     k_ewald_pp(GParams P, const int32_t *__restrict__ leaves, int32_t nleaves, int32_t first,
                const int32_t *__restrict__ off, const int32_t *__restrict__ pb, const int32_t *__restrict__ pe,
                const int4 *__restrict__ pos, ListView LV, EwaldTables E, SepNear K, double *__restrict__ part,

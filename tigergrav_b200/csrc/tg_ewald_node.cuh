@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? EN_MINB : EN_MINB_D)
                 }
 #pragma unroll
                 for (int q = 0; q < MP; q++) M[q] = T(s.m[q]);
-                green_ewald_warp<T>(E, dX, D, lane);
+                green_ewald_warp(E, dX, D, lane);
                 contract_M2L<T, T>(L, M, D);
             }
         }

@@ -235,43 +235,28 @@ __device__ __forceinline__ void green_ewald_full(const EwaldTables &E, const T *
     else ewald_finish<T, T>(D, X);
 }
 
-/* green_ewald(dX) split over a warp: this lane's share of the real-space
- * candidates (every n that can fall inside the cut) and of the reciprocal
- * terms, plus, on lane 0, the final assembly.  The sum of the 32 partial
- * results is green_ewald; the M2L / P2L contractions are linear, so each lane
- * contracts its own part.  X must not be 0 (the caller handles r <= 1e-6). */
-template <class T>
-__device__ __forceinline__ void green_ewald_warp(const EwaldTables &E, const T *X, T *D, int lane) {
+/* FP64: green_ewald(dX) split over a warp: this lane's share of the real-space
+ * candidates and of the reciprocal terms, plus, on lane 0, the final assembly.
+ * The sum of the 32 partial results is green_ewald; the M2L contractions are linear,
+ * so each lane contracts its own part.  X must not be 0 (the caller handles
+ * r <= 1e-6). */
+__device__ __forceinline__ void green_ewald_warp(const EwaldTables &E, const double *X, double *D, int lane) {
 #pragma unroll
-    for (int k = 0; k < LP; k++) D[k] = T(0);
-    const int ncand = sizeof(T) == 4 ? NREAL_F32 : NREAL;
-    EwaldMom<T> mom;
+    for (int k = 0; k < LP; k++) D[k] = 0.0;
+    EwaldMom<double> mom;
     mom.init();
-    for (int t = lane; t < ncand; t += 32) {
+    for (int t = lane; t < NREAL; t += 32) {
         const float4 n = __ldg(&E.real[t]);
-        const T dx[3] = {X[0] - T(n.x), X[1] - T(n.y), X[2] - T(n.z)};
-        const T r2 = dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2];
-        if (r2 < ewald_rcut2<T>() && n.w <= 17.0f) {
-            if constexpr (sizeof(T) == 4) {
-                if (n.w == 0.0f) ewald_origin_add(D, mom, dx, r2);
-                else ewald_real_image<T>(D, mom, dx, r2);
-            } else {
-                ewald_real_image<T>(D, mom, dx, r2);
-            }
-        }
+        const double dx[3] = {X[0] - n.x, X[1] - n.y, X[2] - n.z};
+        const double r2 = dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2];
+        if (r2 < ewald_rcut2<double>()) ewald_real_image<double>(D, mom, dx, r2);
     }
-    ewald_mom_finish<T>(D, mom);
-    for (int t = lane; t < NFOUR_HALF; t += 32) {
-        const T *H = (sizeof(T) == 4) ? (const T *)(E.Hf + HS * t) : (const T *)(E.Hd + HS * t);
-        ewald_four_term<T>(D, X, __ldg(&E.four[t]), H);
-    }
-    if (lane == 0) {
-        if constexpr (sizeof(T) == 4) D[E0()] += T(0.78539816339744831);
-        else ewald_finish<T, T>(D, X);
-    }
+    ewald_mom_finish<double>(D, mom);
+    for (int t = lane; t < NFOUR_HALF; t += 32) ewald_four_term<double>(D, X, __ldg(&E.four[t]), E.Hd + HS * t);
+    if (lane == 0) ewald_finish<double, double>(D, X);
 }
 
-/* CC/CP Ewald lists shorter than this are evaluated one source at a time by
+/* FP64: CC Ewald lists shorter than this are evaluated one source at a time by
  * the whole warp (green_ewald_warp); longer ones one source per lane */
 constexpr int EWALD_WARP_LIST = 12;
 
@@ -291,8 +276,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 template <class T>
 __global__ void __launch_bounds__(128) k_node(GParams P, int64_t nn, const int32_t *__restrict__ pb,
                                               const int32_t *__restrict__ pe, const MSrc *__restrict__ ms,
-                                              const int4 *__restrict__ pos, ListView LV, EwaldTables E,
-                                              double *__restrict__ Lloc) {
+                                              const int4 *__restrict__ pos, ListView LV, double *__restrict__ Lloc) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nn; i += warps) {
@@ -848,9 +832,9 @@ static int node_stage(Solver &S, const GParams &P, const ListView &LV, const Ewa
         const int64_t want = (nn * 32 + TPB - 1) / TPB;
         const int g = (int)(want < 65535 * 8 ? want : 65535 * 8);
         if (f64)
-            k_node<double><<<g, TPB, 0, st>>>(P, nn, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p, S.pos.p, LV, E, S.nd_Lloc.p);
+            k_node<double><<<g, TPB, 0, st>>>(P, nn, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p, S.pos.p, LV, S.nd_Lloc.p);
         else
-            k_node<float><<<g, TPB, 0, st>>>(P, nn, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p, S.pos.p, LV, E, S.nd_Lloc.p);
+            k_node<float><<<g, TPB, 0, st>>>(P, nn, S.nd_pb.p, S.nd_pe.p, S.nd_ms.p, S.pos.p, LV, S.nd_Lloc.p);
         TG_TRY(launched(S));
     }
     if (S.prm.ewald) TG_TRY(node_ewald(S, P, LV, E, f64, st));
