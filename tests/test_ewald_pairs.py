@@ -3,7 +3,7 @@ close ones are not a multipole either, with a softening so long (8) that the dir
 force is below 0.03 and its rounding below 4e-9.  The FP32
 path against the FP64 path over separations |x_d| <= lim, the bounds from the FP32
 rounding of the outputs (|g| <= 1.5, |phi| <= 4: 4e-8 and 1e-7 rms) and of the mirror
-images (at most 0.13 each, with an erfc good to 1.5e-7: 1.2e-7 in the force)."""
+images (at most 0.13 each; an erfc good to 1.5e-7 would add 1.2e-7 to the force)."""
 import numpy as np
 import pytest
 
@@ -34,7 +34,7 @@ def test_force_and_potential(lim):
     dg = np.array([a[1] - b[1] for a, b in zip(f32, f64)])
     dphi = np.array([a[0] - b[0] for a, b in zip(f32, f64)])
     assert np.sqrt((dg ** 2).sum(-1).mean()) <= 2.5e-7
-    # the mean that is kept on purpose: -4.8e-7, and -4e-8 from the erfc of the mirror images
+    # the mean that is kept on purpose, -4.8e-7
     assert abs(dphi.mean() + 5.0e-7) <= 1e-7
     assert dphi.std() <= 2e-7
 

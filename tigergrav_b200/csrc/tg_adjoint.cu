@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(128) k_tidal_pp(GParams P, const int32_t *__re
                                                   const int4 *__restrict__ pos, ListView LV,
                                                   const double *__restrict__ u, double *__restrict__ out) {
     __shared__ int4 sy[128];
-    __shared__ T su[128][3];
+    __shared__ __align__(4 * sizeof(T)) T su[128][4]; /* x, y, z: one load */
     __shared__ double red[128][3];
     const int t = threadIdx.x;
     const bool per = P.ewald != 0;
@@ -375,7 +375,13 @@ __global__ void __launch_bounds__(128) k_tidal_pp(GParams P, const int32_t *__re
 #pragma unroll 4
         for (int32_t q = phase; q < nt; q += C) {
             const int4 y = sy[q];
-            const T du[3] = {ui[0] - su[q][0], ui[1] - su[q][1], ui[2] - su[q][2]};
+            T du[3];
+            if constexpr (sizeof(T) == 4) {
+                const float4 uj = *reinterpret_cast<const float4 *>(su[q]);
+                du[0] = ui[0] - uj.x, du[1] = ui[1] - uj.y, du[2] = ui[2] - uj.z;
+            } else {
+                for (int d = 0; d < 3; d++) du[d] = ui[d] - su[q][d];
+            }
             const T dX[3] = {sep<T>(xi.x, y.x, per), sep<T>(xi.y, y.y, per), sep<T>(xi.z, y.z, per)};
             const T r2 = dX[0] * dX[0] + dX[1] * dX[1] + dX[2] * dX[2];
             T f, fpr;
@@ -470,13 +476,13 @@ __global__ void __launch_bounds__(128) k_tidal_sf(const int32_t *__restrict__ sr
     }
 }
 
-/* r += (d1 + d2 x x^T) du for one image at displacement x.  With the exact erfc: the
- * reference's, good to 1.5e-7, would put 3 / r^3 of that into the Hessian. */
+/* r += (d1 + d2 x x^T) du for one image at displacement x */
 template <class T>
-__device__ __forceinline__ void tidal_image(T x0, T x1, T x2, T r2, const T *du, T *r) {
+__device__ __forceinline__ void tidal_image(const SepNear &K, T x0, T x1, T x2, T r2, const T *du, T *r) {
     const T alpha = T(Sep<T>::ALPHA);
     const T rinv = t_rsqrt(r2), r2inv = rinv * rinv, rr = r2 * rinv;
-    const T e = exp(-(alpha * rr) * (alpha * rr)), ec = erfc(alpha * rr);
+    T e;
+    const T ec = sep_erfc(K, r2, rinv, e);
     const T ce = T(Sep<T>::ALPHA * 1.1283791670955126) * e; /* 2 alpha / sqrt(pi) e^(-alpha^2 r^2) */
     const T d1 = fma(ce, rr, ec) * rinv * r2inv;
     const T d2 = -fma(T(3), d1, T(2) * alpha * alpha * ce) * r2inv;
@@ -488,7 +494,7 @@ __device__ __forceinline__ void tidal_image(T x0, T x1, T x2, T r2, const T *du,
 
 /* the mirror images of a pair at |x| = a, in the octant of |x|: r += D2 w */
 template <class T>
-__device__ __forceinline__ void tidal_images(const T *a, const T *w, T *r) {
+__device__ __forceinline__ void tidal_images(const SepNear &K, const T *a, const T *w, T *r) {
     T b[3], u[3], v[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
@@ -499,7 +505,7 @@ __device__ __forceinline__ void tidal_images(const T *a, const T *w, T *r) {
 #pragma unroll
     for (int k = 1; k < 8; k++) {
         const T s = (k & 1 ? v[0] : u[0]) + (k & 2 ? v[1] : u[1]) + (k & 4 ? v[2] : u[2]);
-        if (s < T(1)) tidal_image<T>(k & 1 ? b[0] : a[0], k & 2 ? b[1] : a[1], k & 4 ? b[2] : a[2], s, w, r);
+        if (s < T(1)) tidal_image<T>(K, k & 1 ? b[0] : a[0], k & 2 ? b[1] : a[1], k & 4 ? b[2] : a[2], s, w, r);
     }
 }
 
@@ -511,7 +517,7 @@ template <> struct TidalPairs<double> {
     __device__ __forceinline__ void init(const double *u) {
         for (int d = 0; d < 3; d++) o[d] = 0.0, ui[d] = u[d];
     }
-    __device__ __forceinline__ void add(const EwaldTables &E, const SepNear &, double m, int4 xi, int4 yj, const double *uj) {
+    __device__ __forceinline__ void add(const EwaldTables &E, const SepNear &K, double m, int4 xi, int4 yj, const double *uj) {
         const double x[3] = {wrap_sep_d(xi.x, yj.x), wrap_sep_d(xi.y, yj.y), wrap_sep_d(xi.z, yj.z)};
         const double du[3] = {ui[0] - uj[0], ui[1] - uj[1], ui[2] - uj[2]};
         const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
@@ -525,7 +531,7 @@ template <> struct TidalPairs<double> {
             a[d] = fabs(x[d]);
             w[d] = copysign(1.0, x[d]) * du[d];
         }
-        tidal_images<double>(a, w, q);
+        tidal_images<double>(K, a, w, q);
         /* nearest image with the direct 1/r removed: d1 = -f0, d2 = (3 f0 - 2 alpha^2 c e) / r^2, or the
          * derivative of f0's series (ewald_nearest) for alpha r < 1/2, where the two cancel */
         const double alpha = Sep<double>::ALPHA;
@@ -583,7 +589,7 @@ template <> struct TidalPairs<float> {
             for (int d = 0; d < 3; d++) o[d] -= E.sep_r2 * du[d];
             return;
         }
-        tidal_images<float>(a, w, q);
+        tidal_images<float>(K, a, w, q);
 #pragma unroll
         for (int d = 0; d < 3; d++) i[d].add(copysignf(1.0f, x[d]) * q[d]);
         const double t = fma(fma(X[0], X[0], fma(X[1], X[1], X[2] * X[2])), 8.0 / 3.0 * POS_INV * POS_INV, -1.0);

@@ -102,12 +102,12 @@ __global__ void k_periodic_parts(const float4 *four, int nf, double scale, doubl
     Pd[2 * t + 1] = make_double2(Hd[HS * t + E1(1)], Hd[HS * t + E1(2)]);
 }
 
-/* monomial coefficients m[0..n] in t of the Chebyshev interpolation of fn(r^2), r^2 = 3/8 (t + 1) */
-template <class F> static void sep_fit(F fn, int n, double *m) {
+/* monomial coefficients m[0..n] of the Chebyshev interpolation of fn(t), |t| <= 1 */
+template <class F, class M> static void sep_fit(F fn, int n, M *m) {
     const double pi = 3.141592653589793;
     std::vector<double> c(n + 1, 0.0), a(n + 1, 0.0), b(n + 1, 0.0), sum(n + 1, 0.0);
     for (int j = 0; j <= n; j++) {
-        const double th = pi * (j + 0.5) / (n + 1), v = fn(0.375 * (std::cos(th) + 1.0));
+        const double th = pi * (j + 0.5) / (n + 1), v = fn(std::cos(th));
         for (int k = 0; k <= n; k++) c[k] += (k ? 2.0 : 1.0) / (n + 1) * v * std::cos(k * th);
     }
     a[0] = 1.0; /* T_k, and T_k+1 in b */
@@ -117,28 +117,30 @@ template <class F> static void sep_fit(F fn, int n, double *m) {
         for (int i = n; i >= 0; i--) a[i] = (i ? 2.0 * b[i - 1] : 0.0) - a[i]; /* T_k+2 = 2 t T_k+1 - T_k */
         std::swap(a, b);
     }
-    for (int i = 0; i <= n; i++) m[i] = (double)sum[i];
+    for (int i = 0; i <= n; i++) m[i] = (M)sum[i];
 }
 
 /* SepNear: interpolation errors 3e-9 of the potential, 1e-9 of the force and 2e-7 of the Jacobian (f0' r^2),
  * against ~1 */
 static void sep_near(double alpha, SepNear &K) {
     const double al = alpha, ispi = 1.1283791670955126; /* 2 / sqrt(pi) */
-    sep_fit([&](double y) { return std::erf(al * std::sqrt(y)) / std::sqrt(y); }, SEP_DP, K.p);
+    const auto r2 = [](double t) { return 0.375 * (t + 1.0); };
+    sep_fit([&](double t) { return std::erf(al * std::sqrt(r2(t))) / std::sqrt(r2(t)); }, SEP_DP, K.p);
     K.p[0] += 3.141592653589793 / (alpha * alpha) + SEP_OFFSET;
     sep_fit(
-        [&](double y) {
-            const double x = al * std::sqrt(y);
+        [&](double t) {
+            const double y = r2(t), x = al * std::sqrt(y);
             if (x > 1.0) return (std::erf(x) - ispi * x * std::exp(-x * x)) / (y * std::sqrt(y));
-            double s = 0.0, t = 1.0; /* ewald_nearest's series; t = (-x^2)^(k-1) / k! */
+            double s = 0.0, w = 1.0; /* ewald_nearest's series; w = (-x^2)^(k-1) / k! */
             for (int k = 1; k < 30; k++) {
-                t /= k;
-                s += 2 * k * t / (2 * k + 1);
-                t *= -x * x;
+                w /= k;
+                s += 2 * k * w / (2 * k + 1);
+                w *= -x * x;
             }
             return al * al * al * ispi * s;
         },
         SEP_DF, K.f);
+    sep_fit([&](double t) { const double x = 2.0 * al / (t + 3.0); return std::erfc(x) * std::exp(x * x); }, SEP_DQ, K.q);
 }
 
 int ewald_tables(Solver &S, cudaStream_t st) {

@@ -31,9 +31,9 @@ constexpr float EWALD_PHI0 = 2.8372975f; /* r -> 0 limit (tigergrav/green.hpp:27
  * the reciprocal vectors (FP32: and the largest |h_d|), and their number (one of
  * each pair +-h) */
 /* The FP32 pair's potential keeps the mean by which the FP32 sums of the reference's
- * split (alpha = 2, Abramowitz & Stegun 7.1.26 for erfc) lie below FP64: -5.3e-7 per
- * pair of unit mass over the cube of separations (-6.9e-7 for |x_d| < 1/4, -9e-7
- * below 1/20).  The same erfc at alpha = 4.5 leaves -3e-8 of it; this is the rest.
+ * split (alpha = 2, Abramowitz & Stegun 7.1.26 for erfc) lie below FP64: -4.7e-7 to
+ * -5.3e-7 per pair of unit mass over the cube of separations (-6.9e-7 for |x_d| < 1/4,
+ * -9e-7 below 1/20).
  * Without it the potentials of small boxes, which cancel to a few 1e-2, differ from
  * the reference's FP32 ones by 2e-5 of their size. */
 constexpr double SEP_OFFSET = -4.8e-7;
@@ -47,11 +47,13 @@ template <> struct Sep<double> {
     static constexpr int H2MAX = 70, N = 1258;
 };
 /* the FP32 pair's nearest image in FP64 (sep_near): erf(alpha r)/r + pi / alpha^2 and
- * its force factor as polynomials in t = 8/3 r^2 - 1 */
+ * its force factor as polynomials in t = 8/3 r^2 - 1; and the mirror images' erfc:
+ * e^(x^2) erfc(x), x = alpha r, as one in 2/r - 3 (1/2 <= r < 1; to 2e-9) */
 constexpr int SEP_RUN = 7; /* vectors of a run, at most (SepTrig) */
-constexpr int SEP_DP = 17, SEP_DF = 20;
+constexpr int SEP_DP = 17, SEP_DF = 20, SEP_DQ = 5;
 struct SepNear {
     double p[SEP_DP + 1], f[SEP_DF + 1];
+    float q[SEP_DQ + 1];
 };
 
 /* ---- symmetric index arithmetic (constant-folded after unrolling) ---- */

@@ -130,8 +130,9 @@ __global__ void __launch_bounds__(64) k_ewald_tsum(int N, double m, const int32_
  * source sums (tpart).  Block b takes chunk first + b, its slot is b.
  *
  * What bounds it: latency of the image and polynomial chains at 16 blocks per SM in
- * FP32 (63 registers, issue 66 %, FP64 pipe 27 %): 0.69 ms at 32768 uniform (12 blocks
- * 0.73, 14: 0.69; polynomials in even and odd halves 0.69). */
+ * FP32 (63 registers, issue 66 %, FP64 pipe 27 %): 0.62 ms at 32768 uniform.  With the
+ * erfc of 7.1.26 0.69 (12 blocks 0.73, 14: 0.69; the polynomials in even and odd
+ * halves 0.69). */
 template <class T>
 __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
     k_ewald_pp(GParams P, const int32_t *__restrict__ leaves, int32_t nleaves, int32_t first,

@@ -27,12 +27,14 @@
  * much as at alpha = 2.  Both are FP64 in the FP32 path: the nearest image as two
  * polynomials in r^2 of the exact separation (SepNear), phases and source sums from
  * FP64 powers of e^(2 pi i x_d) (SepTrig); only the mirror images, at most 0.13
- * each, are FP32.  Measured error of a pair against FP64, rms over |x_d| < 1/2, 1/4,
+ * each, are FP32, their erfc from a polynomial good to 2e-9 (SepNear; a third of the
+ * cost of erfc and expf, and two instructions fewer than the reference's 7.1.26 form,
+ * whose 1.5e-7 showed: force 1.1e-7 over the cube).  Measured error of a pair against FP64, rms over |x_d| < 1/2, 1/4,
  * 1/10, 1/20, with the FP32 output's own rounding:
- *   force     1.1e-7, 2.5e-8, 1.6e-8, 2.1e-8
+ *   force     4.6e-8, 2.5e-8, 1.6e-8, 2.1e-8
  *     the FP32 sums at alpha = 2: 5.4e-7, 5.2e-7, 1.7e-7, 2.0e-7
  *     FP32 throughout at alpha = 4.2: 9.4e-7, 2.1e-6, 1.3e-6, 3.6e-7
- *   Jacobian product (of ~10)  6.1e-7, 4.7e-7, 8.6e-7, 7.6e-7
+ *   Jacobian product (of ~10)  5.0e-7, 4.7e-7, 8.6e-7, 7.6e-7
  *     the FP32 sums at alpha = 2: 5.8e-6, 4.2e-6, 3.8e-6, 3.4e-6
  *     FP32 throughout at alpha = 4.2: 2.2e-5, 5.3e-5, 4.8e-5, 1.5e-5
  *
@@ -155,13 +157,25 @@ __global__ void __launch_bounds__(128) k_ewald_sf(const int32_t *__restrict__ sr
     }
 }
 
+/* erfc(alpha r) and e^(-alpha^2 r^2) of a mirror image, 1/2 <= r < 1 */
+__device__ __forceinline__ float sep_erfc(const SepNear &K, float r2, float rinv, float &e) {
+    e = ex2_ftz(r2 * (float)(-Sep<float>::ALPHA * Sep<float>::ALPHA * 1.4426950408889634));
+    const float w = fmaf(2.0f, rinv, -3.0f);
+    float p = K.q[SEP_DQ];
+#pragma unroll
+    for (int k = SEP_DQ - 1; k >= 0; k--) p = fmaf(p, w, K.q[k]);
+    return p * e;
+}
+__device__ __forceinline__ double sep_erfc(const SepNear &, double r2, double rinv, double &e) {
+    return t_erfcexp(Sep<double>::ALPHA * (r2 * rinv), &e);
+}
 /* one image at the displacement d (r2 = |d|^2 < 1): -erfc(alpha r)/r and its force */
 template <class T>
-__device__ __forceinline__ void sep_image(T d0, T d1, T d2, T r2, T &ph, T &gx, T &gy, T &gz) {
+__device__ __forceinline__ void sep_image(const SepNear &K, T d0, T d1, T d2, T r2, T &ph, T &gx, T &gy, T &gz) {
     const T rinv = t_rsqrt(r2);
     const T r = r2 * rinv;
     T expfac;
-    const T erfc = t_erfcexp(T(Sep<T>::ALPHA) * r, &expfac);
+    const T erfc = sep_erfc(K, r2, rinv, expfac);
     const T expfactor = T(Sep<T>::ALPHA * 1.1283791670955126) * r * expfac; /* 2 alpha / sqrt(pi) */
     const T f = (expfactor + erfc) * rinv * rinv * rinv;
     ph -= erfc * rinv;
@@ -172,24 +186,24 @@ __device__ __forceinline__ void sep_image(T d0, T d1, T d2, T r2, T &ph, T &gx, 
 
 /* the mirror images inside r < 1 of a pair, in the octant of |x|: u = x^2 per axis */
 template <class T>
-__device__ __forceinline__ void sep_images(T a0, T a1, T a2, T u0, T u1, T u2, T &ph, T &gx, T &gy, T &gz) {
+__device__ __forceinline__ void sep_images(const SepNear &K, T a0, T a1, T a2, T u0, T u1, T u2, T &ph, T &gx, T &gy, T &gz) {
     const T b0 = T(1) - a0, b1 = T(1) - a1, b2 = T(1) - a2;
     const T v0 = b0 * b0, v1 = b1 * b1, v2 = b2 * b2;
     T q;
     q = v0 + u1 + u2;
-    if (q < T(1)) sep_image<T>(-b0, a1, a2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, -b0, a1, a2, q, ph, gx, gy, gz);
     q = u0 + v1 + u2;
-    if (q < T(1)) sep_image<T>(a0, -b1, a2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, a0, -b1, a2, q, ph, gx, gy, gz);
     q = u0 + u1 + v2;
-    if (q < T(1)) sep_image<T>(a0, a1, -b2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, a0, a1, -b2, q, ph, gx, gy, gz);
     q = v0 + v1 + u2;
-    if (q < T(1)) sep_image<T>(-b0, -b1, a2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, -b0, -b1, a2, q, ph, gx, gy, gz);
     q = v0 + u1 + v2;
-    if (q < T(1)) sep_image<T>(-b0, a1, -b2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, -b0, a1, -b2, q, ph, gx, gy, gz);
     q = u0 + v1 + v2;
-    if (q < T(1)) sep_image<T>(a0, -b1, -b2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, a0, -b1, -b2, q, ph, gx, gy, gz);
     q = v0 + v1 + v2;
-    if (q < T(1)) sep_image<T>(-b0, -b1, -b2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, -b0, -b1, -b2, q, ph, gx, gy, gz);
 }
 
 /* the sums of one sink over the real-space parts of its PP_E pairs, times m */
@@ -197,7 +211,7 @@ template <class T> struct SepPairs;
 template <> struct SepPairs<double> {
     double s[4];
     __device__ __forceinline__ void init() { s[0] = s[1] = s[2] = s[3] = 0.0; }
-    __device__ __forceinline__ void add(const EwaldTables &E, const SepNear &, double m, int4 xi, int4 y) {
+    __device__ __forceinline__ void add(const EwaldTables &E, const SepNear &K, double m, int4 xi, int4 y) {
         const double x[3] = {wrap_sep_d(xi.x, y.x), wrap_sep_d(xi.y, y.y), wrap_sep_d(xi.z, y.z)};
         const double a0 = fabs(x[0]), a1 = fabs(x[1]), a2 = fabs(x[2]);
         const double u0 = a0 * a0, u1 = a1 * a1, u2 = a2 * a2, r2 = u0 + u1 + u2;
@@ -207,7 +221,7 @@ template <> struct SepPairs<double> {
             return;
         }
         double ph = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
-        sep_images<double>(a0, a1, a2, u0, u1, u2, ph, gx, gy, gz);
+        sep_images<double>(K, a0, a1, a2, u0, u1, u2, ph, gx, gy, gz);
         const double rinv = t_rsqrt(r2);
         double p0, f0;
         ewald_nearest<double>(Sep<double>::ALPHA, r2 * rinv, rinv, p0, f0);
@@ -246,7 +260,7 @@ template <> struct SepPairs<float> {
             return;
         }
         float ph = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f;
-        sep_images<float>(a0, a1, a2, u0, u1, u2, ph, gx, gy, gz);
+        sep_images<float>(K, a0, a1, a2, u0, u1, u2, ph, gx, gy, gz);
         i[0].add(ph);
         i[1].add(copysignf(1.0f, x0) * gx);
         i[2].add(copysignf(1.0f, x1) * gy);
