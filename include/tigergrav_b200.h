@@ -123,7 +123,8 @@ int tg_walk(tg_solver *s, void *stream);
  * counterpart in the reference (its lists are std::vectors). */
 int tg_set_walk_capacity(tg_solver *s, int64_t entries);
 /* Device bytes of each of the two scratch areas of the leaf Ewald sums (partial
- * sums of the sink leaves; sums of the source leaves), 0 = 1 GiB (the default).
+ * sums of the sink leaves; sums of the source leaves), 0 = the larger of 1 GiB and 256
+ * bytes per particle (the default).
  * Leaves that do not fit run in batches of at least one; the forces are the same to
  * the bit. */
 int tg_set_ewald_scratch(tg_solver *s, int64_t bytes);

@@ -816,7 +816,7 @@ int tidal_reserve(Solver &S) {
     TG_TRY(ensure(S.tid_tile, 3 * ((S.n + USUM_TILE - 1) / USUM_TILE)));
     if (S.ew_max_npp > 0) { /* as tidal_ewald */
         const int N = f64 ? Sep<double>::N : Sep<float>::N;
-        const size_t slots = std::min<size_t>(S.ew_max_npp, S.ew_scratch / tidal_chunk_bytes(N) + 1);
+        const size_t slots = std::min<size_t>(S.ew_max_npp, S.ew_scratch() / tidal_chunk_bytes(N) + 1);
         TG_TRY(ensure(S.ew_part, slots * 64 * 3));
         TG_TRY(ensure(S.ew_tpart, slots * N * sizeof(Sep4)));
         TG_TRY(ensure(S.ew_sf, (size_t)S.ew_max_nsrc * ew_vectors(S, S.ew_max_nsrc, sizeof(Sep4), N) * sizeof(Sep4)));

@@ -461,7 +461,7 @@ int tg_set_walk_capacity(tg_solver *s, int64_t entries) {
 int tg_set_ewald_scratch(tg_solver *s, int64_t bytes) {
     CHECK_HANDLE(s);
     if (bytes < 0) return TG_ERR_ARG;
-    s->S.ew_scratch = bytes > 0 ? (size_t)bytes : tg::EW_SCRATCH;
+    s->S.ew_scratch_set = (size_t)bytes;
     return TG_OK;
 }
 

@@ -20,7 +20,7 @@
  * A PP_E chunk's slots take 2 KB and its source sums 9 KB in FP32 and 20 KB in
  * FP64 (the Jacobian's 18 and 40 KB), and where every pair is an Ewald pair the
  * chunks grow with the square of the leaves.  So the leaves run in batches whose
- * chunks fit EW_SCRATCH, each reduced before the next (leaf_batches), and where
+ * chunks fit the scratch (EW_SCRATCH), each reduced before the next (leaf_batches), and where
  * the source leaves' own sums do not fit it, they are made for a range of vectors
  * at a time (k_ewald_tsum).  Neither changes the order of any sum.
  */

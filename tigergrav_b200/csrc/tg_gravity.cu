@@ -744,7 +744,7 @@ static int leaf_batches(Solver &S, int32_t npp, int32_t total, size_t pp, size_t
                         cudaStream_t st) {
     const int32_t nleaves = (int32_t)S.st.leaves;
     out.clear();
-    if ((size_t)npp * pp + (size_t)(total - npp) * pc <= S.ew_scratch) {
+    if ((size_t)npp * pp + (size_t)(total - npp) * pc <= S.ew_scratch()) {
         out.push_back({0, nleaves, 0, npp, npp, total - npp});
         return TG_OK;
     }
@@ -756,14 +756,14 @@ static int leaf_batches(Solver &S, int32_t npp, int32_t total, size_t pp, size_t
     const int32_t *offp = off.get() + nleaves + 1;
     for (int32_t l0 = 0, l1; l0 < nleaves; l0 = l1) {
         for (l1 = l0 + 1; l1 < nleaves; l1++) /* at least one leaf */
-            if ((size_t)(off[l1 + 1] - off[l0]) * pp + (size_t)(offp[l1 + 1] - offp[l0]) * pc > S.ew_scratch) break;
+            if ((size_t)(off[l1 + 1] - off[l0]) * pp + (size_t)(offp[l1 + 1] - offp[l0]) * pc > S.ew_scratch()) break;
         out.push_back({l0, l1, off[l0], off[l1] - off[l0], offp[l0], offp[l1] - offp[l0]});
     }
     return TG_OK;
 }
 /* vectors whose source sums (nsrc rows, `bytes` each) are held at a time, of N */
 static int ew_vectors(const Solver &S, int32_t nsrc, size_t bytes, int N) {
-    const size_t n = S.ew_scratch / (std::max(nsrc, 1) * bytes);
+    const size_t n = S.ew_scratch() / (std::max(nsrc, 1) * bytes);
     return n >= (size_t)N ? N : std::max(1, (int)n);
 }
 

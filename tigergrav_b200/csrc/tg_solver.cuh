@@ -18,6 +18,7 @@
  */
 #pragma once
 
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <vector>
@@ -66,10 +67,13 @@ struct DevBuf {
 
 constexpr int NLIST = 8;
 
-/* Bytes of each of the two scratch areas of the leaf Ewald sums: the chunks of one
- * batch of leaves, and the source leaves' sums (tg_ewald_leaf.cuh).  128^3 at theta 0.2
- * and smaller boxes run in one batch. */
-constexpr size_t EW_SCRATCH = 1ull << 30;
+/* Bytes of each of the two scratch areas of the leaf Ewald sums, the chunks of one
+ * batch of leaves and the source leaves' sums (tg_ewald_leaf.cuh): EW_SCRATCH, or
+ * EW_SCRATCH_N per particle where that is more.  The source leaves' sums take 9 KB
+ * per leaf in FP32, 256 B per particle at 36 particles a leaf; 256^3 at theta 0.19
+ * (2.1 GB of them) runs in one batch like smaller boxes, where 1 GiB gave two batches
+ * and two ranges of vectors and 4 ms of 878 more. */
+constexpr size_t EW_SCRATCH = 1ull << 30, EW_SCRATCH_N = 256;
 
 struct Solver {
     tg_params prm{};
@@ -160,7 +164,10 @@ struct Solver {
     DevBuf<int32_t> ew_slot, ew_src; /* per node: its row of ew_sf, or -1; the nodes of the rows, then their count */
     DevBuf<unsigned char> ew_sf;    /* per PP_E source leaf and h: (cos, sin) sums over its particles (double2) */
     DevBuf<unsigned char> ew_tpart; /* per PP_E chunk and h: source sums (double2) */
-    size_t ew_scratch = EW_SCRATCH;
+    size_t ew_scratch_set = 0; /* tg_set_ewald_scratch; 0: by EW_SCRATCH */
+    size_t ew_scratch() const {
+        return ew_scratch_set ? ew_scratch_set : std::max(EW_SCRATCH, EW_SCRATCH_N * (size_t)n);
+    }
     int32_t ew_max_npp = 0, ew_max_nsrc = 0; /* most PP_E chunks and source leaves of any evaluation */
     bool ew_use_tab = false;       /* a periodic solver of the FP32 path */
     const float *ew_tab = nullptr; /* the device's table of local expansions (FP32 path), shared by its solvers */

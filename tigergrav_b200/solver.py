@@ -132,7 +132,7 @@ class GravitySolver:
         return self
 
     def set_ewald_scratch(self, nbytes: int):
-        """Device bytes of each scratch area of the leaf Ewald sums (0: 1 GiB)."""
+        """Device bytes of each scratch area of the leaf Ewald sums (0: 1 GiB or 256 per particle)."""
         check("tg_set_ewald_scratch", lib.tg_set_ewald_scratch(self.h, int(nbytes)))
         return self
 
