@@ -492,20 +492,20 @@ __device__ __forceinline__ void tidal_image(const SepNear &K, T x0, T x1, T x2, 
     r[2] = fma(x2, s, fma(d1, du[2], r[2]));
 }
 
-/* the mirror images of a pair at |x| = a, in the octant of |x|: r += D2 w */
+/* the mirror images of a pair at x: r += D2 du */
 template <class T>
-__device__ __forceinline__ void tidal_images(const SepNear &K, const T *a, const T *w, T *r) {
-    T b[3], u[3], v[3];
+__device__ __forceinline__ void tidal_images(const SepNear &K, const T *x, const T *du, T *r) {
+    T c[3], u[3], v[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        b[d] = a[d] - T(1);
-        u[d] = a[d] * a[d];
-        v[d] = b[d] * b[d];
+        c[d] = x[d] - copysign(T(1), x[d]);
+        u[d] = x[d] * x[d];
+        v[d] = c[d] * c[d];
     }
 #pragma unroll
     for (int k = 1; k < 8; k++) {
         const T s = (k & 1 ? v[0] : u[0]) + (k & 2 ? v[1] : u[1]) + (k & 4 ? v[2] : u[2]);
-        if (s < T(1)) tidal_image<T>(K, k & 1 ? b[0] : a[0], k & 2 ? b[1] : a[1], k & 4 ? b[2] : a[2], s, w, r);
+        if (s < T(1)) tidal_image<T>(K, k & 1 ? c[0] : x[0], k & 2 ? c[1] : x[1], k & 4 ? c[2] : x[2], s, du, r);
     }
 }
 
@@ -525,13 +525,8 @@ template <> struct TidalPairs<double> {
             for (int d = 0; d < 3; d++) o[d] += -m * (-E.sep_r2 * du[d]);
             return;
         }
-        double a[3], w[3], q[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            a[d] = fabs(x[d]);
-            w[d] = copysign(1.0, x[d]) * du[d];
-        }
-        tidal_images<double>(K, a, w, q);
+        double q[3] = {0.0, 0.0, 0.0};
+        tidal_images<double>(K, x, du, q);
         /* nearest image with the direct 1/r removed: d1 = -f0, d2 = (3 f0 - 2 alpha^2 c e) / r^2, or the
          * derivative of f0's series (ewald_nearest) for alpha r < 1/2, where the two cancel */
         const double alpha = Sep<double>::ALPHA;
@@ -554,44 +549,50 @@ template <> struct TidalPairs<double> {
             const double ce = Sep<double>::ALPHA * 1.1283791670955126 * exp(-y);
             d2 = (3.0 * f0 - 2.0 * alpha * alpha * ce) * rinv * rinv;
         }
-        const double s = (a[0] * w[0] + a[1] * w[1] + a[2] * w[2]) * d2;
+        const double s = (x[0] * du[0] + x[1] * du[1] + x[2] * du[2]) * d2;
 #pragma unroll
-        for (int d = 0; d < 3; d++) o[d] += -m * (copysign(1.0, x[d]) * (q[d] + a[d] * s - f0 * w[d]));
+        for (int d = 0; d < 3; d++) o[d] += -m * (q[d] + x[d] * s - f0 * du[d]);
     }
+    __device__ __forceinline__ void fold() {}
     __device__ __forceinline__ double get(int d, double) const { return o[d]; }
 };
 /* FP32: the nearest image in FP64, d1 = -f0 and d2 = -2 df0/dr^2; the mirror images
- * in FP32 with compensated sums */
+ * in FP32, summed as in SepPairs */
 template <> struct TidalPairs<float> {
     double o[3], ui[3];
+    float a[3];
     Acc<float> i[3];
     __device__ __forceinline__ void init(const double *u) {
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            o[d] = 0.0, ui[d] = u[d];
+            o[d] = 0.0, ui[d] = u[d], a[d] = 0.0f;
             i[d].init(0.0);
+        }
+    }
+    __device__ __forceinline__ void fold() {
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            i[d].add(a[d]);
+            a[d] = 0.0f;
         }
     }
     __device__ __forceinline__ void add(const EwaldTables &E, const SepNear &K, double, int4 xi, int4 yj, const double *uj) {
         const int32_t n[3] = {(int32_t)((uint32_t)xi.x - (uint32_t)yj.x), (int32_t)((uint32_t)xi.y - (uint32_t)yj.y),
                               (int32_t)((uint32_t)xi.z - (uint32_t)yj.z)};
-        float x[3], a[3], w[3], q[3] = {0.0f, 0.0f, 0.0f};
+        float x[3], w[3];
         double X[3], du[3];
 #pragma unroll
         for (int d = 0; d < 3; d++) {
             x[d] = __int2float_rn(n[d]) * 2.3283064365386963e-10f;
             X[d] = i2d(n[d]);
             du[d] = ui[d] - uj[d];
-            a[d] = fabsf(x[d]);
-            w[d] = copysignf(1.0f, x[d]) * (float)du[d];
+            w[d] = (float)du[d];
         }
         if (!(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] > 1.0e-12f)) {
             for (int d = 0; d < 3; d++) o[d] -= E.sep_r2 * du[d];
             return;
         }
-        tidal_images<float>(K, a, w, q);
-#pragma unroll
-        for (int d = 0; d < 3; d++) i[d].add(copysignf(1.0f, x[d]) * q[d]);
+        tidal_images<float>(K, x, w, a);
         const double t = fma(fma(X[0], X[0], fma(X[1], X[1], X[2] * X[2])), 8.0 / 3.0 * POS_INV * POS_INV, -1.0);
         double f = K.f[SEP_DF], df = 0.0; /* f0 and its derivative by t */
 #pragma unroll
@@ -641,7 +642,11 @@ __global__ void __launch_bounds__(64) k_tidal_ewald_pp(GParams P, const int32_t 
         }
         __syncthreads();
         if (tid < ((cnt + 31) & ~31))
-            for (int32_t q = 0; q < sn; q++) o.add(E, K, P.m_d, xi, sy[q], su[q]);
+            for (int32_t q = 0; q < sn;) {
+                const int32_t q1 = min(sn, q + SEP_FOLD);
+                for (; q < q1; q++) o.add(E, K, P.m_d, xi, sy[q], su[q]);
+                o.fold();
+            }
     }
     if (tid < cnt)
         for (int d = 0; d < 3; d++) part[3 * ((int64_t)blockIdx.x * 64 + tid) + d] = o.get(d, P.m_d);

@@ -50,7 +50,8 @@ template <> struct Sep<double> {
  * its force factor as polynomials in t = 8/3 r^2 - 1; and the mirror images' erfc:
  * e^(x^2) erfc(x), x = alpha r, as one in 2/r - 3 (1/2 <= r < 1; to 2e-9) */
 constexpr int SEP_RUN = 7; /* vectors of a run, at most (SepTrig) */
-constexpr int SEP_DP = 17, SEP_DF = 20, SEP_DQ = 5;
+constexpr int SEP_DP = 16, SEP_DF = 19, SEP_DQ = 5;
+constexpr int SEP_FOLD = 4; /* pairs between folds of the mirror images' FP32 sums */
 struct SepNear {
     double p[SEP_DP + 1], f[SEP_DF + 1];
     float q[SEP_DQ + 1];

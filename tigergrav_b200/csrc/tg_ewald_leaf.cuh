@@ -130,9 +130,10 @@ __global__ void __launch_bounds__(64) k_ewald_tsum(int N, double m, const int32_
  * source sums (tpart).  Block b takes chunk first + b, its slot is b.
  *
  * What bounds it: latency of the image and polynomial chains at 16 blocks per SM in
- * FP32 (63 registers, issue 66 %, FP64 pipe 27 %): 0.62 ms at 32768 uniform.  With the
- * erfc of 7.1.26 0.69 (12 blocks 0.73, 14: 0.69; the polynomials in even and odd
- * halves 0.69). */
+ * FP32 (64 registers, issue 66 to 78 %, FP64 pipe 27 to 34 %): 64^3 clustered, theta 0.25,
+ * 9.4e10 pairs/s (8.8e10 with every pair's images folded by itself).  Measured and
+ * not kept: 12 or 14 blocks, the polynomials in even and odd halves, the erfc of
+ * 7.1.26 (0.69 ms for 0.62 at 32768 uniform). */
 template <class T>
 __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
     k_ewald_pp(GParams P, const int32_t *__restrict__ leaves, int32_t nleaves, int32_t first,
@@ -160,7 +161,11 @@ __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 16 : 12)
         if (tid < sn) sy[tid] = pos[sb + tid];
         __syncthreads();
         if (tid < ((cnt + 31) & ~31)) /* a warp without sinks only stages */
-            for (int32_t q = 0; q < sn; q++) s.add(E, K, P.m_d, xi, sy[q]);
+            for (int32_t q = 0; q < sn;) {
+                const int32_t q1 = min(sn, q + SEP_FOLD);
+                for (; q < q1; q++) s.add(E, K, P.m_d, xi, sy[q]);
+                s.fold();
+            }
     }
     if (active)
         for (int q = 0; q < 4; q++) part[4 * ((int64_t)blockIdx.x * 64 + tid) + q] = s.get(q, P.m_d);

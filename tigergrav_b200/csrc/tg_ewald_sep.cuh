@@ -184,26 +184,27 @@ __device__ __forceinline__ void sep_image(const SepNear &K, T d0, T d1, T d2, T 
     gz = fma(-d2, f, gz);
 }
 
-/* the mirror images inside r < 1 of a pair, in the octant of |x|: u = x^2 per axis */
+/* the mirror images inside r < 1 of a pair at x, u = x^2 per axis, added to ph and g */
 template <class T>
-__device__ __forceinline__ void sep_images(const SepNear &K, T a0, T a1, T a2, T u0, T u1, T u2, T &ph, T &gx, T &gy, T &gz) {
-    const T b0 = T(1) - a0, b1 = T(1) - a1, b2 = T(1) - a2;
-    const T v0 = b0 * b0, v1 = b1 * b1, v2 = b2 * b2;
+__device__ __forceinline__ void sep_images(const SepNear &K, T x0, T x1, T x2, T u0, T u1, T u2, T &ph, T &gx, T &gy,
+                                           T &gz) {
+    const T c0 = x0 - copysign(T(1), x0), c1 = x1 - copysign(T(1), x1), c2 = x2 - copysign(T(1), x2);
+    const T v0 = c0 * c0, v1 = c1 * c1, v2 = c2 * c2;
     T q;
     q = v0 + u1 + u2;
-    if (q < T(1)) sep_image<T>(K, -b0, a1, a2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, c0, x1, x2, q, ph, gx, gy, gz);
     q = u0 + v1 + u2;
-    if (q < T(1)) sep_image<T>(K, a0, -b1, a2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, x0, c1, x2, q, ph, gx, gy, gz);
     q = u0 + u1 + v2;
-    if (q < T(1)) sep_image<T>(K, a0, a1, -b2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, x0, x1, c2, q, ph, gx, gy, gz);
     q = v0 + v1 + u2;
-    if (q < T(1)) sep_image<T>(K, -b0, -b1, a2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, c0, c1, x2, q, ph, gx, gy, gz);
     q = v0 + u1 + v2;
-    if (q < T(1)) sep_image<T>(K, -b0, a1, -b2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, c0, x1, c2, q, ph, gx, gy, gz);
     q = u0 + v1 + v2;
-    if (q < T(1)) sep_image<T>(K, a0, -b1, -b2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, x0, c1, c2, q, ph, gx, gy, gz);
     q = v0 + v1 + v2;
-    if (q < T(1)) sep_image<T>(K, -b0, -b1, -b2, q, ph, gx, gy, gz);
+    if (q < T(1)) sep_image<T>(K, c0, c1, c2, q, ph, gx, gy, gz);
 }
 
 /* the sums of one sink over the real-space parts of its PP_E pairs, times m */
@@ -213,35 +214,46 @@ template <> struct SepPairs<double> {
     __device__ __forceinline__ void init() { s[0] = s[1] = s[2] = s[3] = 0.0; }
     __device__ __forceinline__ void add(const EwaldTables &E, const SepNear &K, double m, int4 xi, int4 y) {
         const double x[3] = {wrap_sep_d(xi.x, y.x), wrap_sep_d(xi.y, y.y), wrap_sep_d(xi.z, y.z)};
-        const double a0 = fabs(x[0]), a1 = fabs(x[1]), a2 = fabs(x[2]);
-        const double u0 = a0 * a0, u1 = a1 * a1, u2 = a2 * a2, r2 = u0 + u1 + u2;
+        const double u0 = x[0] * x[0], u1 = x[1] * x[1], u2 = x[2] * x[2], r2 = u0 + u1 + u2;
         if (!(r2 > 1.0e-12)) { /* phi0 alone: take back the reciprocal terms, R0 + R2 r^2 / 2 */
             s[0] += m * ((double)EWALD_PHI0 - E.sep_r0);
             for (int d = 0; d < 3; d++) s[1 + d] += m * (E.sep_r2 * x[d]);
             return;
         }
         double ph = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
-        sep_images<double>(K, a0, a1, a2, u0, u1, u2, ph, gx, gy, gz);
+        sep_images<double>(K, x[0], x[1], x[2], u0, u1, u2, ph, gx, gy, gz);
         const double rinv = t_rsqrt(r2);
         double p0, f0;
         ewald_nearest<double>(Sep<double>::ALPHA, r2 * rinv, rinv, p0, f0);
         s[0] += m * (ph + (E.sep_k + p0)); /* sep_k = pi / alpha^2 */
-        s[1] += m * fma(x[0], f0, copysign(1.0, x[0]) * gx);
-        s[2] += m * fma(x[1], f0, copysign(1.0, x[1]) * gy);
-        s[3] += m * fma(x[2], f0, copysign(1.0, x[2]) * gz);
+        s[1] += m * fma(x[0], f0, gx);
+        s[2] += m * fma(x[1], f0, gy);
+        s[3] += m * fma(x[2], f0, gz);
     }
+    __device__ __forceinline__ void fold() {}
     __device__ __forceinline__ double get(int q, double) const { return s[q]; }
 };
 /* FP32: the nearest image in FP64 (plain sums, the force in units of 2^-32), the
- * mirror images in FP32 (compensated sums) */
+ * mirror images in FP32: plain sums over the pairs between two folds (SEP_FOLD,
+ * with at most 0.13 per image a rounding of 2e-8, below a pair's own), then
+ * compensated ones */
 template <> struct SepPairs<float> {
     double s[4];
+    float a[4];
     Acc<float> i[4];
     __device__ __forceinline__ void init() {
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             s[q] = 0.0;
+            a[q] = 0.0f;
             i[q].init(0.0);
+        }
+    }
+    __device__ __forceinline__ void fold() {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            i[q].add(a[q]);
+            a[q] = 0.0f;
         }
     }
     __device__ __forceinline__ void add(const EwaldTables &E, const SepNear &K, double, int4 xi, int4 y) {
@@ -249,8 +261,7 @@ template <> struct SepPairs<float> {
                       d2 = (int32_t)((uint32_t)xi.z - (uint32_t)y.z);
         const float w = 2.3283064365386963e-10f; /* 2^-32 */
         const float x0 = __int2float_rn(d0) * w, x1 = __int2float_rn(d1) * w, x2 = __int2float_rn(d2) * w;
-        const float a0 = fabsf(x0), a1 = fabsf(x1), a2 = fabsf(x2);
-        const float u0 = a0 * a0, u1 = a1 * a1, u2 = a2 * a2;
+        const float u0 = x0 * x0, u1 = x1 * x1, u2 = x2 * x2;
         const double X0 = i2d(d0), X1 = i2d(d1), X2 = i2d(d2);
         if (!(u0 + u1 + u2 > 1.0e-12f)) { /* phi0 alone, as above */
             s[0] += (double)EWALD_PHI0 - E.sep_r0;
@@ -259,12 +270,7 @@ template <> struct SepPairs<float> {
             s[3] = fma(E.sep_r2, X2, s[3]);
             return;
         }
-        float ph = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f;
-        sep_images<float>(K, a0, a1, a2, u0, u1, u2, ph, gx, gy, gz);
-        i[0].add(ph);
-        i[1].add(copysignf(1.0f, x0) * gx);
-        i[2].add(copysignf(1.0f, x1) * gy);
-        i[3].add(copysignf(1.0f, x2) * gz);
+        sep_images<float>(K, x0, x1, x2, u0, u1, u2, a[0], a[1], a[2], a[3]);
         /* t = 8/3 r^2 - 1, r^2 in units of 2^-64 */
         const double t = fma(fma(X0, X0, fma(X1, X1, X2 * X2)), 8.0 / 3.0 * POS_INV * POS_INV, -1.0);
         double p = K.p[SEP_DP], f = K.f[SEP_DF];
