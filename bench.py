@@ -95,18 +95,17 @@ PP_FLOPS = 18
 # from the source the same way.  A derivative tensor from the expansion table
 # (tg_ewald_table.cuh): ~510 instructions, mostly FMAs -> 950; contractions: M2L
 # 858, M2P 414, P2L 70 (direct kernels: the reference's constants).  PP_E pair
-# (tg_ewald_sep.cuh): squares 14, the nearest image 40, 3 of its 7 mirror
-# neighbours on average at 45 -> 190; the reciprocal terms are summed per source
-# leaf and evaluated per sink particle (not counted).
+# (tg_ewald_sep.cuh): squares 14, 3 of the 7 mirror images on average at 45 -> 150;
+# its nearest image (about 90 FP64 operations) and the reciprocal terms, summed per
+# source leaf and evaluated per sink particle in FP64, are not counted.
 NODE_FLOPS = {"CC_D": 1025, "CP_D": 455, "CC_E": 1810, "CP_E": 1020}
-LEAF_FLOPS = {"PC_D": 581, "PC_E": 1360, "PP_E": 190}
+LEAF_FLOPS = {"PC_D": 581, "PC_E": 1360, "PP_E": 150}
 # DRAM bytes per interaction of each kernel group, from ncu captures
 # (dram__bytes_read.sum + dram__bytes_write.sum over the capture's
 # interactions) on the 72^3 clustered box at theta 0.19, leaf 48 (the
-# clustered72 workload); PP: an earlier kernel of the same reads (148 MB for
-# 3.2e10 pairs), leaf: k_ewald_pp.  Scaled by this run's counts on the assumption
+# clustered72 workload); PP: k_pp_long, leaf: k_ewald_pp.  Scaled by this run's counts on the assumption
 # that traffic grows with the interactions.
-TRAFFIC = {"pp": {"PP_D": 4.6e-3}, "nodes": {"CC_E": 2.6, "CP_E": 2.6}, "leaf": {"PP_E": 0.127, "PC_E": 0.127}}
+TRAFFIC = {"pp": {"PP_D": 4.3e-3}, "nodes": {"CC_E": 2.6, "CP_E": 2.6}, "leaf": {"PP_E": 0.86, "PC_E": 0.86}}
 TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum per interaction of a small capture, "
                   "scaled by this run's interaction counts")
 
