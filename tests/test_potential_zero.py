@@ -2,7 +2,7 @@
 pair or nearly so: the mean over the particles of the FP32 path's phi stays
 within 4e-7 of the oracle's in the reference's arithmetic.  Both lie below the FP64
 sums: the oracle by the mean error of its erfc, 5.3e-7 per pair of unit mass over the
-cube of separations, the FP32 path by a constant, 4.8e-7.
+cube of separations, the FP32 path by a constant, 5.2e-7.
 The bound tells that the constant is there, not that the potentials are exact."""
 import numpy as np
 import pytest

@@ -33,10 +33,11 @@ constexpr float EWALD_PHI0 = 2.8372975f; /* r -> 0 limit (tigergrav/green.hpp:27
 /* The FP32 pair's potential keeps the mean by which the FP32 sums of the reference's
  * split (alpha = 2, Abramowitz & Stegun 7.1.26 for erfc) lie below FP64: -4.7e-7 to
  * -5.3e-7 per pair of unit mass over the cube of separations (-6.9e-7 for |x_d| < 1/4,
- * -9e-7 below 1/20).
- * Without it the potentials of small boxes, which cancel to a few 1e-2, differ from
- * the reference's FP32 ones by 2e-5 of their size. */
-constexpr double SEP_OFFSET = -4.8e-7;
+ * -9e-7 below 1/20); one number for all of them, which keeps the potentials where they
+ * were with 7.1.26 in the mirror images (-4.8e-7 and -4e-8 from it).  Without it the
+ * potentials of small boxes, which cancel to a few 1e-2, differ from the reference's
+ * FP32 ones by 2e-5 of their size. */
+constexpr double SEP_OFFSET = -5.2e-7;
 template <class T> struct Sep;
 template <> struct Sep<float> {
     static constexpr double ALPHA = 4.5;
